@@ -38,11 +38,11 @@ UNIT = "steps/s"
 # SpMV inputs at the 6 neighbours come from cache).
 BYTES_PER_CELL = {
     "assemble": 8 + 8 + 24 + 56 + 8 + 8,   # phi, phi_old, 3 face velocities; 7 diagonals, rhs, x0
-    "step1": 88,    # r, u, 6 off-diagonals, r_hat; u', v
-    "step2": 88,    # r, v, 6 off-diagonals, r_hat; r', s
-    "step3": 88,    # s, v, 6 off-diagonals, r_hat; v', w
-    "step4": 104,   # s, w, 6 off-diagonals, r', v'; r'', s', t
-    "step5": 96,    # x, r'', s', t, u', r', v', w, r_hat; x, r, u
+    "step1": 80,    # r, u, 6 off-diagonals, r_hat; v
+    "step2": 80,    # r, v, 6 off-diagonals, r_hat; s
+    "step3": 80,    # s, v, 6 off-diagonals, r_hat; w
+    "step4": 88,    # s, w, 6 off-diagonals, r, v; t
+    "step5": 88,    # x, r, u, v, s, w, t, r_hat; x, r, u
 }
 
 
@@ -690,8 +690,8 @@ def measure_hetero(D, ctx, n=512, seed=0, warmup=1, steps=2):
     p32.solve(system)
     ctx.synchronize()
     fp32_kernels = {}
-    for name, bpc in (("fp32_step1", 44), ("fp32_step2", 44), ("fp32_step3", 44), ("fp32_step4", 52),
-                      ("fp32_step5", 48)):
+    for name, bpc in (("fp32_step1", 40), ("fp32_step2", 40), ("fp32_step3", 40), ("fp32_step4", 44),
+                      ("fp32_step5", 44)):
         tot, cnt = ctx.kernel_stats(name)
         if cnt:
             fp32_kernels[name] = {"launches": cnt, "ms_avg": tot / cnt, "bytes_per_cell": bpc,

@@ -13,10 +13,8 @@
 //     keeping the fused input of planes i-1, i, i+1 in registers and plane i
 //     (with its j/k halo) in shared memory, so each operand is read from HBM
 //     once and each fused value is evaluated once per cell (plus the halo).
-//     Each of r, u, v and s has a second buffer for the value of the middle
-//     of an iteration: step (10), x += alpha u, and step (15),
-//     u = r - beta u, wait for the last kernel, which reads both buffers.
-//     A graph holds two iterations.
+//     They store only the products; the fifth kernel does every vector update
+//     of the iteration.  A graph holds two iterations.
 //   * Scalars (alpha, beta, rho, omega, ...) never leave the device: the last
 //     block of each kernel reduces the per-block partials in a fixed order
 //     (deterministic, no floating-point atomics), evaluates the reference's
@@ -104,7 +102,7 @@ int ensure_solver_ws(dare_system* s) {
     ws->n = n;
     cudaError_t e = cudaMalloc(&ws->ahat, (size_t)n * 6 * sizeof(double));
     if (e == cudaSuccess) e = cudaMalloc(&ws->invd, (size_t)n * sizeof(double));
-    if (e == cudaSuccess) e = cudaMalloc(&ws->vec, (size_t)n * 11 * sizeof(double));
+    if (e == cudaSuccess) e = cudaMalloc(&ws->vec, (size_t)n * kNumSolverVecs * sizeof(double));
     if (e == cudaSuccess) e = cudaMalloc(&ws->partials, (size_t)kMaxQ * kMaxBlocks * sizeof(double) + 64);
     if (e == cudaSuccess) e = cudaMalloc(&ws->st, sizeof(SolverState));
     if (e == cudaSuccess) e = cudaMemsetAsync(ws->st, 0, sizeof(SolverState), ctx->stream);
@@ -125,16 +123,12 @@ VecsT<T> carve_vecs(T* base, int64_t n, T* x, const T* b) {
     v.x = x;
     v.b = b;
     v.rh = base;
-    v.r[0] = base + 1 * n;
-    v.r[1] = base + 2 * n;
-    v.u[0] = base + 3 * n;
-    v.u[1] = base + 4 * n;
-    v.v[0] = base + 5 * n;
-    v.v[1] = base + 6 * n;
-    v.s[0] = base + 7 * n;
-    v.s[1] = base + 8 * n;
-    v.w = base + 9 * n;
-    v.t = base + 10 * n;
+    v.r = base + 1 * n;
+    v.u = base + 2 * n;
+    v.v = base + 3 * n;
+    v.s = base + 4 * n;
+    v.w = base + 5 * n;
+    v.t = base + 6 * n;
     return v;
 }
 template VecsT<double> carve_vecs<double>(double*, int64_t, double*, const double*);
@@ -172,13 +166,13 @@ int launch_iteration(dare_ctx* ctx, const GridDev& g, const MarchCfg& m, int sbl
     if (ev) DARE_CUDA(ctx, cudaEventRecord(ev[4], sm));
     int vec4 = 0;
     if constexpr (sizeof(T) == 4) {
-        const void* arrs[10] = {vs.x, vs.r[0], vs.s[1], vs.t, vs.u[0], vs.u[1], vs.r[1], vs.v[1], vs.w, vs.rh};
+        const void* arrs[8] = {vs.x, vs.r, vs.u, vs.v, vs.s, vs.w, vs.t, vs.rh};
         vec4 = g.ncell % 4 == 0;
         for (const void* a : arrs)
             if (a && reinterpret_cast<uintptr_t>(a) % 16 != 0) vec4 = 0;
     }
-    k_step5<T><<<sblocks, 256, 0, sm>>>(g.ncell, vs.x, vs.r[0], vs.s[1], vs.t, vs.u[0], vs.u[1], vs.r[1], vs.v[1],
-                                        vs.w, vs.rh, st, partials, 0, 0, vec4);
+    k_step5<T><<<sblocks, 256, 0, sm>>>(g.ncell, vs.x, vs.r, vs.u, vs.v, vs.s, vs.w, vs.t, vs.rh, st, partials, 0, 0,
+                                        vec4);
     DARE_LAUNCHED(ctx);
     if (ev) DARE_CUDA(ctx, cudaEventRecord(ev[5], sm));
     return DARE_OK;
@@ -215,9 +209,9 @@ int launch_fold_init(dare_ctx* ctx, const GridDev& g, const MarchCfg& m, const d
     for (int q = 0; q < 6; q++) f.ps[q] = diag + (q + 1) * n;
     f.ps[6] = vs.b;
     f.ahat = ahat;
-    f.r = vs.r[0];
+    f.r = vs.r;
     f.rh = vs.rh;
-    f.u = vs.u[0];
+    f.u = vs.u;
     f.n = n;
     return launch_march(ctx, g, m, f, st, partials);
 }
@@ -238,7 +232,7 @@ int launch_fold32(dare_ctx* ctx, const GridDev& g, const MarchCfg& m, const doub
 template <typename T>
 int finish_step10(dare_ctx* ctx, int64_t n, const SolverState& st_host, const SolverState* st, const VecsT<T>& vs) {
     if (!step10_pending(st_host)) return DARE_OK;
-    k_step10<T><<<grid_blocks(ctx, n, 256, 8), 256, 0, ctx->stream>>>(n, st, vs.u[1], vs.x);
+    k_step10<T><<<grid_blocks(ctx, n, 256, 8), 256, 0, ctx->stream>>>(n, st, vs.r, vs.u, vs.x);
     DARE_LAUNCHED(ctx);
     return DARE_OK;
 }
@@ -410,7 +404,7 @@ int dare_bicgstab2_fp64_to(dare_system* s, const dare_solver_params* p, dare_sol
     // the state in one round trip: step (10) when the solve stopped after it
     // (decided on the device), x = M^-1 y, and the true residual of that x
     // (the report's, and the tau = 0 exit's check).
-    k_step10<double><<<grid_blocks(ctx, n, 256, 8), 256, 0, ctx->stream>>>(n, ws->st, vs.u[1], vs.x);
+    k_step10<double><<<grid_blocks(ctx, n, 256, 8), 256, 0, ctx->stream>>>(n, ws->st, vs.r, vs.u, vs.x);
     DARE_LAUNCHED(ctx);
     const GridDev& gf = s->grid->dev;   // one field component
     const bool to_field = f && field_written && f->grid == s->grid && f->ncomp == s->ncomp && solution_to_field_ok(gf);

@@ -14,7 +14,8 @@ enum : int { ST_RUNNING = 0, ST_CONVERGED = 1, ST_MAXIT = 2, ST_BREAKDOWN = 3, S
 struct SolverState {
     double alpha, beta, rho0, rho1, gamma, omega1, omega2, mu, nu, tau;
     double rnorm, rnorm0, bnorm2, tol;
-    double alpha1, beta1;  // learned solve: alpha of step 7 and beta of step 11 (its flexible update)
+    double alpha1, beta1;  // alpha of step 7; beta of step 11 (the learned solve's flexible update)
+    double beta5;          // beta of step 5 (beta is step 11's by the last kernel)
     int k, max_it, done, status, step, tol_relative;
     unsigned int count;   // reduction arrivals (reset by the last arrival)
     unsigned int queue;   // next work item of a marching kernel
@@ -34,13 +35,14 @@ struct VecsT {
     T* x;        // y in the preconditioned variable, x at the end
     const T* b;
     T* rh;       // r_hat_0
-    T* r[2];     // r[0] the iterate's r, r[1] step (8)'s r until K5 has used it
-    T* u[2];     // u[0] the iterate's u, u[1] step (5)'s u until K5 has used it
-    T* v[2];
-    T* s[2];
+    T* r;        // the iterate's r and u, replaced by the last kernel of an iteration
+    T* u;
+    T* v;        // the products of steps (6), (9), (13), (18)
+    T* s;
     T* w;
     T* t;
 };
+constexpr int kNumSolverVecs = 7;   // rh, r, u, v, s, w, t
 
 // Work decomposition of the marching kernels: (j,k) tiles of block.x by
 // block.y cells, runs of `planes` i-planes; item = chunk * tiles + tile.
@@ -179,7 +181,7 @@ struct dare_solver_ws {
     int64_t n = 0;
     double* ahat = nullptr;      // 6 * n, Jacobi-folded off-diagonals
     double* invd = nullptr;      // n
-    double* vec = nullptr;       // 11 * n work vectors
+    double* vec = nullptr;       // kNumSolverVecs * n work vectors
     double* partials = nullptr;  // kMaxQ * kMaxBlocks (+ scratch)
     dare_gpu::SolverState* st = nullptr;
     dare_gpu::SolverState* st_host = nullptr;  // pinned
@@ -188,8 +190,7 @@ struct dare_solver_ws {
     int stream_blocks = 0;
     // FP32 inner solver of the refinement driver (dare_mixed.cu)
     float* ahat32 = nullptr;     // 6 * n
-    float* vec32 = nullptr;      // 12 * n (11 work vectors + the correction)
-    double* r64 = nullptr;       // unused slot kept for layout stability
+    float* vec32 = nullptr;      // (kNumSolverVecs + 2) * n: work vectors, the correction, the right-hand side
     dare_gpu::MarchCfg march32;
     // learned-preconditioner solver (dare_learned.cu)
     struct dare_learned_ws* learned = nullptr;

@@ -43,6 +43,7 @@ __device__ inline void begin_iteration(SolverState* st, double rho1) {
     }
     st->rho1 = rho1;                                         // (4)
     st->beta = st->alpha * st->rho1 / st->rho0;
+    st->beta5 = st->beta;                                    // step (5)'s, used again in the last kernel
     st->rho0 = st->rho1;
     if (st->rho0 == 0.0) finish(st, ST_BREAKDOWN, 4);
 }
@@ -180,6 +181,15 @@ struct FInit {
     __device__ void done(SolverState* st, const double* tot) const { finish_init(st, tot); }
 };
 
+// The four SpMV kernels store only their products v, s, w and t.  The vectors
+// of the middle of an iteration -- u of step (5), r of (8), v of (12), r and s
+// of (16)-(17) -- are operands formed while staging, and a later kernel that
+// needs one again forms it again from the r, u, v, s and w it comes from, with
+// the same expression (so the same bits): none of those five is overwritten
+// before the last kernel.  That takes five stores and one load of n values
+// out of an iteration (464 -> 416 bytes per cell in FP64): the 256^3 TVD step
+// went from 12.05 to 11.33 ms, the 384^3 FP32-refine step from 24.4 to 22.7.
+
 // K1: (5) u = r - beta u; (6) v = Op u; (7) gamma = <v, r_hat_0>
 template <typename T, bool UNIT>
 struct FStep1 {
@@ -189,12 +199,11 @@ struct FStep1 {
     static constexpr bool kPairs = sizeof(T) == 4;   // two cells per thread (see launch_march)
     const T* zs[2];   // r, u
     const T* ps[NP];  // coefficients, r_hat_0
-    T *u_out, *v;
+    T* v;
     T beta;
     __device__ void load(const SolverState* st) { beta = (T)st->beta; }
     __device__ T zc(T r, T u) const { return r - beta * u; }
     __device__ void center(int64_t c, const T (&zz)[7], const T* p, double* acc) const {
-        u_out[c] = zz[0];
         const T vc = apply_pre<T, UNIT>(p, zz);
         v[c] = vc;
         acc[0] += (double)vc * (double)p[NC];
@@ -203,8 +212,8 @@ struct FStep1 {
 };
 
 // K2: (8) r = r - alpha v; (9) s = Op r; (11) rho1 = <r_hat_0, s>.  Step
-// (10), x = x + alpha u, waits for K5 (x is read by nothing in between and
-// step (15) leaves this u in place), which saves x's read and write here.
+// (10), x = x + alpha u, waits for K5 (x is read by nothing in between),
+// which saves x's read and write here.
 template <typename T, bool UNIT>
 struct FStep2 {
     using type = T;
@@ -213,12 +222,11 @@ struct FStep2 {
     static constexpr bool kPairs = sizeof(T) == 4;   // two cells per thread (see launch_march)
     const T* zs[2];   // v, r
     const T* ps[NP];  // coefficients, r_hat_0
-    T *r_out, *s;
+    T* s;
     T alpha;
     __device__ void load(const SolverState* st) { alpha = (T)st->alpha; }
     __device__ T zc(T v, T r) const { return -alpha * v + r; }
     __device__ void center(int64_t c, const T (&zz)[7], const T* p, double* acc) const {
-        r_out[c] = zz[0];
         const T sc = apply_pre<T, UNIT>(p, zz);
         s[c] = sc;
         acc[0] += (double)p[NC] * (double)sc;
@@ -235,12 +243,11 @@ struct FStep3 {
     static constexpr bool kPairs = sizeof(T) == 4;   // two cells per thread (see launch_march)
     const T* zs[2];   // s, v
     const T* ps[NP];  // coefficients, r_hat_0
-    T *v_out, *w;
+    T* w;
     T beta;
     __device__ void load(const SolverState* st) { beta = (T)st->beta; }
     __device__ T zc(T s, T v) const { return s - beta * v; }
     __device__ void center(int64_t c, const T (&zz)[7], const T* p, double* acc) const {
-        v_out[c] = zz[0];
         const T wc = apply_pre<T, UNIT>(p, zz);
         w[c] = wc;
         acc[0] += (double)wc * (double)p[NC];
@@ -248,26 +255,38 @@ struct FStep3 {
     __device__ void done(SolverState* st, const double* tot) const { finish_gamma(st, tot, 14); }
 };
 
+// r after steps (8) and (16), from the iterate's r, the v of step (6) and the
+// s of step (9): v' = s - beta v (12), r' = r - alpha1 v (8), r'' = r' - alpha v'
+template <typename T>
+__device__ __forceinline__ T r_of_16(T r, T v, T s, T alpha1, T alpha, T beta) {
+    const T v12 = s - beta * v;
+    const T r8 = -alpha1 * v + r;
+    return -alpha * v12 + r8;
+}
+
 // K4: (16) r = r - alpha v; (17) s = s - alpha w; (18) t = Op s;
-//     (19)-(20) <r,s>, <s,s>, <s,t>, <t,t>, <r,t>; (21)-(23).  The new r
-//     goes to the other r buffer, so K5 can still form step (15)'s
-//     u = r - beta u from this kernel's input r.
+//     (19)-(20) <r,s>, <s,s>, <s,t>, <t,t>, <r,t>; (21)-(23).  Step (16)'s
+//     terms come from the r, v and s staged here (kRaw: center3 also gets the
+//     second staged operand's own value, the s of step (9)).
 template <typename T, bool UNIT>
 struct FStep4 {
     using type = T;
     static constexpr int Q = 5, NZ = 2, NC = NCoef<UNIT>::value, NP = NC + 2;
     static constexpr bool kCheckDone = true;
     static constexpr bool kPairs = sizeof(T) == 4;   // two cells per thread (see launch_march)
+    static constexpr bool kRaw = true;
     const T* zs[2];   // w, s
-    const T* ps[NP];  // coefficients, r (of step (8)), v
-    T *r_out, *s_out, *t;
-    T alpha;
-    __device__ void load(const SolverState* st) { alpha = (T)st->alpha; }
+    const T* ps[NP];  // coefficients, r, v
+    T* t;
+    T alpha, alpha1, beta;
+    __device__ void load(const SolverState* st) {
+        alpha = (T)st->alpha;
+        alpha1 = (T)st->alpha1;
+        beta = (T)st->beta;
+    }
     __device__ T zc(T w, T s) const { return -alpha * w + s; }
-    __device__ void center(int64_t c, const T (&zz)[7], const T* p, double* acc) const {
-        const T rn = -alpha * p[NC + 1] + p[NC];
-        r_out[c] = rn;
-        s_out[c] = zz[0];
+    __device__ void center3(int64_t c, const T (&zz)[7], T s9, const T* p, double* acc) const {
+        const T rn = r_of_16(p[NC], p[NC + 1], s9, alpha1, alpha, beta);
         const T tc = apply_pre<T, UNIT>(p, zz);
         t[c] = tc;
         const double dr = rn, ds = zz[0], dt = tc;
@@ -391,10 +410,19 @@ struct SplitOperands<K, std::void_t<decltype(K::kSplit)>> {
     static constexpr bool value = K::kSplit;
 };
 
+// functors whose center step also takes the second staged operand's own value
+template <class K, class = void>
+struct RawOperand {
+    static constexpr bool value = false;
+};
+template <class K>
+struct RawOperand<K, std::void_t<decltype(K::kRaw)>> {
+    static constexpr bool value = K::kRaw;
+};
+
 // ---------------------------------------------------------------------------
-// the functors of the init kernel and of one iteration over the vectors vs
-// (halves a of r / u current, b = 1 - a written), shared by the single-grid
-// and the slab drivers
+// the functors of the init kernel and of one iteration over the vectors vs,
+// shared by the single-grid and the slab drivers
 // ---------------------------------------------------------------------------
 template <typename T, bool UNIT>
 FInit<T, UNIT> make_init(const OpT<T>& op, const VecsT<T>& vs) {
@@ -403,42 +431,39 @@ FInit<T, UNIT> make_init(const OpT<T>& op, const VecsT<T>& vs) {
     f.zs[0] = vs.x;
     set_coef_streams<T, UNIT, F::NP>(op, f.ps);
     f.ps[F::NC] = vs.b;
-    f.r = vs.r[0];
+    f.r = vs.r;
     f.rh = vs.rh;
-    f.u = vs.u[0];
+    f.u = vs.u;
     return f;
 }
 template <typename T, bool UNIT>
 FStep1<T, UNIT> make_step1(const OpT<T>& op, const VecsT<T>& vs) {
     FStep1<T, UNIT> f{};
-    f.zs[0] = vs.r[0];
-    f.zs[1] = vs.u[0];
+    f.zs[0] = vs.r;
+    f.zs[1] = vs.u;
     set_coef_streams<T, UNIT, FStep1<T, UNIT>::NP>(op, f.ps);
     f.ps[NCoef<UNIT>::value] = vs.rh;
-    f.u_out = vs.u[1];
-    f.v = vs.v[0];
+    f.v = vs.v;
     return f;
 }
 template <typename T, bool UNIT>
 FStep2<T, UNIT> make_step2(const OpT<T>& op, const VecsT<T>& vs) {
     constexpr int NC = NCoef<UNIT>::value;
     FStep2<T, UNIT> f{};
-    f.zs[0] = vs.v[0];
-    f.zs[1] = vs.r[0];
+    f.zs[0] = vs.v;
+    f.zs[1] = vs.r;
     set_coef_streams<T, UNIT, FStep2<T, UNIT>::NP>(op, f.ps);
     f.ps[NC] = vs.rh;
-    f.r_out = vs.r[1];
-    f.s = vs.s[0];
+    f.s = vs.s;
     return f;
 }
 template <typename T, bool UNIT>
 FStep3<T, UNIT> make_step3(const OpT<T>& op, const VecsT<T>& vs) {
     FStep3<T, UNIT> f{};
-    f.zs[0] = vs.s[0];
-    f.zs[1] = vs.v[0];
+    f.zs[0] = vs.s;
+    f.zs[1] = vs.v;
     set_coef_streams<T, UNIT, FStep3<T, UNIT>::NP>(op, f.ps);
     f.ps[NCoef<UNIT>::value] = vs.rh;
-    f.v_out = vs.v[1];
     f.w = vs.w;
     return f;
 }
@@ -447,12 +472,10 @@ FStep4<T, UNIT> make_step4(const OpT<T>& op, const VecsT<T>& vs) {
     constexpr int NC = NCoef<UNIT>::value;
     FStep4<T, UNIT> f{};
     f.zs[0] = vs.w;
-    f.zs[1] = vs.s[0];
+    f.zs[1] = vs.s;
     set_coef_streams<T, UNIT, FStep4<T, UNIT>::NP>(op, f.ps);
-    f.ps[NC] = vs.r[1];
-    f.ps[NC + 1] = vs.v[1];
-    f.r_out = vs.r[0];
-    f.s_out = vs.s[1];
+    f.ps[NC] = vs.r;
+    f.ps[NC + 1] = vs.v;
     f.t = vs.t;
     return f;
 }
@@ -854,7 +877,10 @@ __global__ void __launch_bounds__(256, MarchMinBlocks<K, CPT>::value) k_march(Gr
                     T pv[NP];
 #pragma unroll
                     for (int q = 0; q < NP; q++) pv[q] = sb[NZ * ZT + q * NCT + tid];
-                    k.center((int64_t)i * plane + G.o_own, z7, pv, acc);
+                    if constexpr (RawOperand<K>::value)
+                        k.center3((int64_t)i * plane + G.o_own, z7, sb[ZT + (ty + 1) * W + col], pv, acc);
+                    else
+                        k.center((int64_t)i * plane + G.o_own, z7, pv, acc);
                     zprev[0] = zcur;
                 } else if constexpr (CPT == 2) {
                     // the thread's two cells as one 16-byte (8-byte for FP32)
@@ -882,9 +908,15 @@ __global__ void __launch_bounds__(256, MarchMinBlocks<K, CPT>::value) k_march(Gr
                         pv1[q] = pq.y;
                     }
                     const T z70[7] = {zc0, zprev[0], zn0, zs0, zt0, zw, zc1};
-                    k.center((int64_t)i * plane + G.o_own, z70, pv0, acc);
                     const T z71[7] = {zc1, zprev[1], zn1, zs1, zt1, zc0, ze};
-                    k.center((int64_t)i * plane + G.o_own + 1, z71, pv1, acc);
+                    if constexpr (RawOperand<K>::value) {
+                        const Pair<T> raw = ld_pair(sb + ZT + (ty + 1) * W + col);
+                        k.center3((int64_t)i * plane + G.o_own, z70, raw.x, pv0, acc);
+                        k.center3((int64_t)i * plane + G.o_own + 1, z71, raw.y, pv1, acc);
+                    } else {
+                        k.center((int64_t)i * plane + G.o_own, z70, pv0, acc);
+                        k.center((int64_t)i * plane + G.o_own + 1, z71, pv1, acc);
+                    }
                     zprev[0] = zc0;
                     zprev[1] = zc1;
                 } else {
@@ -920,7 +952,10 @@ __global__ void __launch_bounds__(256, MarchMinBlocks<K, CPT>::value) k_march(Gr
                     for (int c = 0; c < 4; c++) {
                         const T z7[7] = {zc[c], zprev[c], zn[c], zs[c], zt[c], c == 0 ? zw : zc[c - 1],
                                          c == 3 ? ze : zc[c + 1]};
-                        k.center((int64_t)i * plane + G.o_own + c, z7, pv[c], acc);
+                        if constexpr (RawOperand<K>::value)
+                            k.center3((int64_t)i * plane + G.o_own + c, z7, sb[ZT + (ty + 1) * W + col + c], pv[c], acc);
+                        else
+                            k.center((int64_t)i * plane + G.o_own + c, z7, pv[c], acc);
                     }
 #pragma unroll
                     for (int c = 0; c < 4; c++) zprev[c] = zc[c];
@@ -1050,74 +1085,88 @@ inline int launch_march(dare_ctx* ctx, const GridDev& g, const MarchCfg& m, cons
     return launch_march_t<K, 1, HALO>(ctx, g, m1, kern, st, partials);
 }
 
-// K5: the deferred steps (10) x = x + alpha1 u1 and (15) u = r1 - beta u1
-//     (u1 the u of step (5), r1 the r of step (8)), then (24)
-//     x = x + w1 r + w2 s + alpha u; (25) r = r - w1 s - w2 t; ||r||;
-//     u = u - w1 v - w2 w; then the next iteration's (3), (4).
+// The scalars of an iteration that the last kernel applies, and one cell of it:
+// from the iterate's x, r, u and the products v, s, w, t of steps (6), (9),
+// (13), (18)
+//   u5 = r - beta5 u (5), r8 = r - alpha1 v (8), x10 = x + alpha1 u5 (10),
+//   v12 = s - beta v (12), u15 = r8 - beta u5 (15), r16 = r8 - alpha v12 (16),
+//   s17 = s - alpha w (17), then
+//   x = x10 + w1 r16 + w2 s17 + alpha u15 (24), r = r16 - w1 s17 - w2 t (25),
+//   u = u15 - w1 v12 - w2 w
+template <typename T>
+struct Step5 {
+    T w1, w2, alpha, alpha1, beta, beta5;
+    __device__ __forceinline__ explicit Step5(const SolverState* st)
+        : w1((T)st->omega1), w2((T)st->omega2), alpha((T)st->alpha), alpha1((T)st->alpha1), beta((T)st->beta),
+          beta5((T)st->beta5) {}
+    __device__ __forceinline__ void cell(T& x, T& r, T& u, T v, T s, T w, T t) const {
+        const T u5 = r - beta5 * u;
+        const T r8 = -alpha1 * v + r;
+        const T x10 = alpha1 * u5 + x;
+        const T v12 = s - beta * v;
+        const T u15 = r8 - beta * u5;
+        const T r16 = -alpha * v12 + r8;
+        const T s17 = -alpha * w + s;
+        const T xc = w1 * r16 + w2 * s17 + x10;
+        x = alpha * u15 + xc;
+        r = -w1 * s17 + -w2 * t + r16;
+        u = -w1 * v12 + -w2 * w + u15;
+    }
+};
+
+// K5: the rest of the iteration (Step5), ||r||, <r_hat_0, r>, then the next
+//     iteration's (3), (4).  Eight arrays read, three written.
 //     `base` / `total`: partial-sum slots shared with other launches (slabs;
 //     0, 0: this launch alone).  `vec4` (FP32 only; n % 4 == 0 and every
 //     array 16-byte aligned): four cells per thread and 16-byte accesses
 //     (512^3: 0.92 ms; with 4-byte accesses the FP32 kernel took 1.22 ms,
-//     81 % of copy bandwidth).
+//     81 % of copy bandwidth, both with nine arrays read).
 template <typename T>
-__global__ void __launch_bounds__(256) k_step5(int64_t n, T* __restrict__ x, T* __restrict__ r,
-                                               const T* __restrict__ s, const T* __restrict__ t,
-                                               T* __restrict__ u, const T* __restrict__ u1,
-                                               const T* __restrict__ r1, const T* __restrict__ v,
-                                               const T* __restrict__ w, const T* __restrict__ rh, SolverState* st,
-                                               double* partials, int base, int total, int vec4) {
+__global__ void __launch_bounds__(256) k_step5(int64_t n, T* __restrict__ x, T* __restrict__ r, T* __restrict__ u,
+                                               const T* __restrict__ v, const T* __restrict__ s,
+                                               const T* __restrict__ w, const T* __restrict__ t,
+                                               const T* __restrict__ rh, SolverState* st, double* partials, int base,
+                                               int total, int vec4) {
     if (st->done) return;
-    const T w1 = (T)st->omega1, w2 = (T)st->omega2, alpha = (T)st->alpha, alpha1 = (T)st->alpha1;
-    const T beta = (T)st->beta;
+    const Step5<T> f(st);
     double acc[2] = {0., 0.};
     if constexpr (sizeof(T) == 4) {
         if (vec4) {
-            // the scalar loop's expressions, cell by cell within each float4
-            auto cell = [&](float rc, float sc, float u1c, float xc0, float r1c, float tc, float vc, float wc,
-                            float rhc, float& xo, float& ro, float& uo) {
-                const float x10 = alpha1 * u1c + xc0;
-                const float u15 = r1c - beta * u1c;
-                float xc = w1 * rc + w2 * sc + x10;
-                xc = alpha * u15 + xc;
-                xo = xc;
-                const float rn = -w1 * sc + -w2 * tc + rc;
-                ro = rn;
-                uo = -w1 * vc + -w2 * wc + u15;
-                acc[0] += (double)rn * (double)rn;
-                acc[1] += (double)rhc * (double)rn;
-            };
             const int64_t n4 = n >> 2;
             for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < n4;
                  q += (int64_t)gridDim.x * blockDim.x) {
-                const float4 rq = reinterpret_cast<const float4*>(r)[q], sq = reinterpret_cast<const float4*>(s)[q];
-                const float4 u1q = reinterpret_cast<const float4*>(u1)[q], xq = reinterpret_cast<const float4*>(x)[q];
-                const float4 r1q = reinterpret_cast<const float4*>(r1)[q], tq = reinterpret_cast<const float4*>(t)[q];
-                const float4 vq = reinterpret_cast<const float4*>(v)[q], wq = reinterpret_cast<const float4*>(w)[q];
-                const float4 rhq = reinterpret_cast<const float4*>(rh)[q];
-                float4 xo, ro, uo;
-                cell(rq.x, sq.x, u1q.x, xq.x, r1q.x, tq.x, vq.x, wq.x, rhq.x, xo.x, ro.x, uo.x);
-                cell(rq.y, sq.y, u1q.y, xq.y, r1q.y, tq.y, vq.y, wq.y, rhq.y, xo.y, ro.y, uo.y);
-                cell(rq.z, sq.z, u1q.z, xq.z, r1q.z, tq.z, vq.z, wq.z, rhq.z, xo.z, ro.z, uo.z);
-                cell(rq.w, sq.w, u1q.w, xq.w, r1q.w, tq.w, vq.w, wq.w, rhq.w, xo.w, ro.w, uo.w);
-                reinterpret_cast<float4*>(x)[q] = xo;
-                reinterpret_cast<float4*>(r)[q] = ro;
-                reinterpret_cast<float4*>(u)[q] = uo;
+                float4 xq = reinterpret_cast<const float4*>(x)[q], rq = reinterpret_cast<const float4*>(r)[q];
+                float4 uq = reinterpret_cast<const float4*>(u)[q];
+                const float4 vq = reinterpret_cast<const float4*>(v)[q], sq = reinterpret_cast<const float4*>(s)[q];
+                const float4 wq = reinterpret_cast<const float4*>(w)[q], tq = reinterpret_cast<const float4*>(t)[q];
+                const float4 hq = reinterpret_cast<const float4*>(rh)[q];
+                f.cell(xq.x, rq.x, uq.x, vq.x, sq.x, wq.x, tq.x);
+                f.cell(xq.y, rq.y, uq.y, vq.y, sq.y, wq.y, tq.y);
+                f.cell(xq.z, rq.z, uq.z, vq.z, sq.z, wq.z, tq.z);
+                f.cell(xq.w, rq.w, uq.w, vq.w, sq.w, wq.w, tq.w);
+                reinterpret_cast<float4*>(x)[q] = xq;
+                reinterpret_cast<float4*>(r)[q] = rq;
+                reinterpret_cast<float4*>(u)[q] = uq;
+                acc[0] += (double)rq.x * (double)rq.x;
+                acc[1] += (double)hq.x * (double)rq.x;
+                acc[0] += (double)rq.y * (double)rq.y;
+                acc[1] += (double)hq.y * (double)rq.y;
+                acc[0] += (double)rq.z * (double)rq.z;
+                acc[1] += (double)hq.z * (double)rq.z;
+                acc[0] += (double)rq.w * (double)rq.w;
+                acc[1] += (double)hq.w * (double)rq.w;
             }
             n = 0;   // the scalar loop below has nothing left to do
         }
     }
     for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n; c += (int64_t)gridDim.x * blockDim.x) {
-        const T rc = r[c], sc = s[c], u1c = u1[c];
-        const T x10 = alpha1 * u1c + x[c];
-        const T u15 = r1[c] - beta * u1c;
-        T xc = w1 * rc + w2 * sc + x10;
-        xc = alpha * u15 + xc;
+        T xc = x[c], rc = r[c], uc = u[c];
+        f.cell(xc, rc, uc, v[c], s[c], w[c], t[c]);
         x[c] = xc;
-        const T rn = -w1 * sc + -w2 * t[c] + rc;
-        r[c] = rn;
-        u[c] = -w1 * v[c] + -w2 * w[c] + u15;
-        acc[0] += (double)rn * (double)rn;
-        acc[1] += (double)rh[c] * (double)rn;
+        r[c] = rc;
+        u[c] = uc;
+        acc[0] += (double)rc * (double)rc;
+        acc[1] += (double)rh[c] * (double)rc;
     }
     double tot[2];
     if (!grid_reduce<2>(acc, partials, &st->count, tot, base, total)) return;
@@ -1125,16 +1174,20 @@ __global__ void __launch_bounds__(256) k_step5(int64_t n, T* __restrict__ x, T* 
 }
 
 // Step (10) of an iteration that stopped after it and before K5 (a
-// breakdown in steps (14), (20) or (21)): x = x + alpha1 u1.
+// breakdown in steps (14), (20) or (21)): x = x + alpha1 u of step (5), formed
+// from the r and u that K5 has not replaced.
 inline __host__ __device__ bool step10_pending_state(int status, int step) {
     return status == ST_TAU0 || (status == ST_BREAKDOWN && (step == 14 || step == 20));
 }
 template <typename T>
-__global__ void k_step10(int64_t n, const SolverState* st, const T* __restrict__ u1, T* __restrict__ x) {
+__global__ void k_step10(int64_t n, const SolverState* st, const T* __restrict__ r, const T* __restrict__ u,
+                         T* __restrict__ x) {
     if (!step10_pending_state(st->status, st->step)) return;   // read on the device: no host round trip
-    const T alpha1 = (T)st->alpha1;
-    for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n; c += (int64_t)gridDim.x * blockDim.x)
-        x[c] = alpha1 * u1[c] + x[c];
+    const T alpha1 = (T)st->alpha1, beta5 = (T)st->beta5;
+    for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n; c += (int64_t)gridDim.x * blockDim.x) {
+        const T u5 = r[c] - beta5 * u[c];
+        x[c] = alpha1 * u5 + x[c];
+    }
 }
 inline bool step10_pending(const SolverState& st) { return step10_pending_state(st.status, st.step); }
 

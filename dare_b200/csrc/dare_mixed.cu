@@ -21,10 +21,8 @@ void dare_mixed_ws_free(dare_solver_ws* ws) {
     if (!ws) return;
     cudaFree(ws->ahat32);
     cudaFree(ws->vec32);
-    cudaFree(ws->r64);
     ws->ahat32 = nullptr;
     ws->vec32 = nullptr;
-    ws->r64 = nullptr;
 }
 
 namespace dare_gpu {
@@ -96,7 +94,7 @@ int dare_bicgstab2_refine(dare_system* s, const dare_solver_params* p, dare_solv
     const int64_t n = g.ncell;
     if (!ws->ahat32) {
         cudaError_t e = cudaMalloc(&ws->ahat32, (size_t)n * 6 * sizeof(float));
-        if (e == cudaSuccess) e = cudaMalloc(&ws->vec32, (size_t)n * 13 * sizeof(float));
+        if (e == cudaSuccess) e = cudaMalloc(&ws->vec32, (size_t)n * (kNumSolverVecs + 2) * sizeof(float));
         if (e != cudaSuccess) {
             dare_mixed_ws_free(ws);
             return check_cuda(ctx, e, "refinement workspace");
@@ -111,8 +109,8 @@ int dare_bicgstab2_refine(dare_system* s, const dare_solver_params* p, dare_solv
     // Ahat = A D^-1, folded straight to FP32
     if ((rc = launch_fold32(ctx, g, m, s->diag, ws->invd, ws->ahat32, ws->st, ws->partials))) return rc;
     OpT<float> op32{nullptr, ws->ahat32, n};
-    float* dy = ws->vec32 + 11 * n;
-    float* r32 = ws->vec32 + 12 * n;
+    float* dy = ws->vec32 + kNumSolverVecs * n;
+    float* r32 = ws->vec32 + (kNumSolverVecs + 1) * n;
     VecsT<float> vs32 = carve_vecs<float>(ws->vec32, n, dy, r32);
 
     double* scratch = ws->partials + (size_t)kMaxQ * kMaxBlocks;
