@@ -36,6 +36,7 @@ SOURCES = {
     "dare_assembly3.cu": [],
     "dare_slabs.cu": [],
     "dare_bicgstab2.cu": [],
+    "dare_resident.cu": [],
     "dare_mixed.cu": [],
     "dare_step.cu": [],
     "dare_noalloc.cu": [],

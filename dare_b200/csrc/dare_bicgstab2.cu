@@ -26,7 +26,7 @@
 #include <cstring>
 #include <new>
 
-#include "dare_march.cuh"
+#include "dare_team.cuh"
 
 using namespace dare_gpu;
 
@@ -39,6 +39,7 @@ void dare_solver_ws_free(dare_solver_ws* ws) {
     cudaFree(ws->invd);
     cudaFree(ws->vec);
     cudaFree(ws->partials);
+    cudaFree(ws->packets);
     cudaFree(ws->st);
     if (ws->st_host) cudaFreeHost(ws->st_host);
     dare_mixed_ws_free(ws);
@@ -104,6 +105,8 @@ int ensure_solver_ws(dare_system* s) {
     if (e == cudaSuccess) e = cudaMalloc(&ws->invd, (size_t)n * sizeof(double));
     if (e == cudaSuccess) e = cudaMalloc(&ws->vec, (size_t)n * kNumSolverVecs * sizeof(double));
     if (e == cudaSuccess) e = cudaMalloc(&ws->partials, (size_t)kMaxQ * kMaxBlocks * sizeof(double) + 64);
+    if (e == cudaSuccess) e = cudaMalloc(&ws->packets, kTeamBytes);
+    if (e == cudaSuccess) e = cudaMemsetAsync(ws->packets, 0, kTeamBytes, ctx->stream);
     if (e == cudaSuccess) e = cudaMalloc(&ws->st, sizeof(SolverState));
     if (e == cudaSuccess) e = cudaMemsetAsync(ws->st, 0, sizeof(SolverState), ctx->stream);
     if (e == cudaSuccess) e = cudaMallocHost(&ws->st_host, sizeof(SolverState));
@@ -384,44 +387,64 @@ int dare_bicgstab2_fp64_to(dare_system* s, const dare_solver_params* p, dare_sol
 
     OpT<double> full{s->diag, s->diag + n, n};
     OpT<double> folded{nullptr, ws->ahat, n};
-    SolverState init{};   // also zeroes the reduction and queue counters
-    init.tol = p->tol;
-    init.max_it = p->max_it;
-    init.tol_relative = p->tol_relative;
-    DARE_CUDA(ctx, cudaMemcpyAsync(ws->st, &init, sizeof(init), cudaMemcpyHostToDevice, ctx->stream));
     VecsT<double> vs = carve_vecs<double>(ws->vec, n, s->x, s->rhs);
-    rc = jacobi ? launch_fold_init(ctx, g, m, s->diag, ws->invd, ws->ahat, vs, ws->st, ws->partials)
-                : launch_init<double, false>(ctx, g, m, full, vs, ws->st, ws->partials);
-    if (rc) return rc;
-    rc = jacobi ? run_iterations<double, true>(ctx, g, m, ws->stream_blocks, folded, vs, ws->st, ws->st_host,
-                                               ws->partials, &ws->graph[1][0], p->max_it, p->check_every, KID_STEP1,
-                                               false)
-                : run_iterations<double, false>(ctx, g, m, ws->stream_blocks, full, vs, ws->st, ws->st_host,
-                                                ws->partials, &ws->graph[0][0], p->max_it, p->check_every, KID_STEP1,
-                                                false);
-    if (rc) return rc;
-    // The exit's device work, queued behind the iterations and read back with
-    // the state in one round trip: step (10) when the solve stopped after it
-    // (decided on the device), x = M^-1 y, and the true residual of that x
-    // (the report's, and the tau = 0 exit's check).
-    k_step10<double><<<grid_blocks(ctx, n, 256, 8), 256, 0, ctx->stream>>>(n, ws->st, vs.r, vs.u, vs.x);
-    DARE_LAUNCHED(ctx);
     const GridDev& gf = s->grid->dev;   // one field component
     const bool to_field = f && field_written && f->grid == s->grid && f->ncomp == s->ncomp && solution_to_field_ok(gf);
-    if (to_field) {
-        for (int c = 0; c < s->ncomp; c++)
-            if ((rc = launch_solution_to_field(ctx, gf, jacobi ? ws->invd + (size_t)c * gf.ncell : nullptr,
-                                               s->x + (size_t)c * gf.ncell, f->level[0] + (size_t)c * gf.ncell_ghosted)))
-                return rc;
-    } else if (jacobi && (rc = launch_scale(ctx, n, ws->invd, s->x))) {
-        return rc;
-    }
     bool field_current = to_field;
     double* tres = &ws->st->tres;
-    if (p->compute_true_residual &&
-        (rc = launch_true_residual(ctx, g, m, full, s->x, s->rhs, ws->st, ws->partials, tres)))
-        return rc;
-    if ((rc = finish_iterations(ctx, ws->st, ws->st_host))) return rc;
+    // Small systems run in one launch (timed as one kernel when profiling)
+    int blocks = 0, chunk = 0;
+    if (resident_shape(ctx, n, jacobi, &blocks, &chunk)) {
+        const bool prof = ctx->profiling != 0;
+        if (prof) DARE_CUDA(ctx, cudaEventRecord(ctx->ev[0], ctx->stream));
+        if ((rc = launch_resident(s, p, vs, blocks, chunk, to_field ? f->level[0] : nullptr))) return rc;
+        if (prof) DARE_CUDA(ctx, cudaEventRecord(ctx->ev[1], ctx->stream));
+        DARE_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+        float ms = 0.f;
+        if (prof && cudaEventElapsedTime(&ms, ctx->ev[0], ctx->ev[1]) == cudaSuccess) {
+            ctx->stat_ms[KID_SOLVE] += ms;
+            ctx->stat_n[KID_SOLVE] += 1;
+        }
+        if (!ws->st_host->done) {   // a wait between its blocks ran out: start the exchanges over
+            DARE_CUDA(ctx, cudaMemsetAsync(ws->packets, 0, kTeamBytes, ctx->stream));
+            return set_error(ctx, DARE_ERR_TIMEOUT, "bicgstab2: a wait between blocks ran out");
+        }
+    } else {
+        SolverState init{};   // also zeroes the reduction and queue counters
+        init.tol = p->tol;
+        init.max_it = p->max_it;
+        init.tol_relative = p->tol_relative;
+        DARE_CUDA(ctx, cudaMemcpyAsync(ws->st, &init, sizeof(init), cudaMemcpyHostToDevice, ctx->stream));
+        rc = jacobi ? launch_fold_init(ctx, g, m, s->diag, ws->invd, ws->ahat, vs, ws->st, ws->partials)
+                    : launch_init<double, false>(ctx, g, m, full, vs, ws->st, ws->partials);
+        if (rc) return rc;
+        rc = jacobi ? run_iterations<double, true>(ctx, g, m, ws->stream_blocks, folded, vs, ws->st, ws->st_host,
+                                                   ws->partials, &ws->graph[1][0], p->max_it, p->check_every,
+                                                   KID_STEP1, false)
+                    : run_iterations<double, false>(ctx, g, m, ws->stream_blocks, full, vs, ws->st, ws->st_host,
+                                                    ws->partials, &ws->graph[0][0], p->max_it, p->check_every,
+                                                    KID_STEP1, false);
+        if (rc) return rc;
+        // The exit's device work, queued behind the iterations and read back
+        // with the state in one round trip: step (10) when the solve stopped
+        // after it (decided on the device), x = M^-1 y, and the true residual
+        // of that x (the report's, and the tau = 0 exit's check).
+        k_step10<double><<<grid_blocks(ctx, n, 256, 8), 256, 0, ctx->stream>>>(n, ws->st, vs.r, vs.u, vs.x);
+        DARE_LAUNCHED(ctx);
+        if (to_field) {
+            for (int c = 0; c < s->ncomp; c++)
+                if ((rc = launch_solution_to_field(ctx, gf, jacobi ? ws->invd + (size_t)c * gf.ncell : nullptr,
+                                                   s->x + (size_t)c * gf.ncell,
+                                                   f->level[0] + (size_t)c * gf.ncell_ghosted)))
+                    return rc;
+        } else if (jacobi && (rc = launch_scale(ctx, n, ws->invd, s->x))) {
+            return rc;
+        }
+        if (p->compute_true_residual &&
+            (rc = launch_true_residual(ctx, g, m, full, s->x, s->rhs, ws->st, ws->partials, tres)))
+            return rc;
+        if ((rc = finish_iterations(ctx, ws->st, ws->st_host))) return rc;
+    }
     SolverState st = *ws->st_host;
 
     std::memset(rep, 0, sizeof(*rep));

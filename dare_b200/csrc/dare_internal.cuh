@@ -58,7 +58,7 @@ enum KernelId : int {
     KID_STEP3 = 5,
     KID_STEP4 = 6,
     KID_STEP5 = 7,
-    KID_FINAL = 8,
+    KID_SOLVE = 8,   // the whole solve of a small system (dare_resident.cu)
     KID_COUNT = 16
 };
 }  // namespace dare_gpu

@@ -531,6 +531,17 @@ int dare_slabs_solve(dare_slabs* sl, const dare_solver_params* p, dare_solve_rep
     const bool jacobi = p->precond == DARE_PREC_JACOBI;
     const int S = sl->S;
     int rc;
+    if (S == 1) {   // one slab is the whole grid: its x halo is its own wrap
+        dare_system view = *sl->systems[0];
+        dare_grid whole = *sl->grids[0];
+        whole.dev.periodic[0] = view.sdev.periodic[0] = sl->global.periodic[0];
+        view.grid = &whole;
+        dare_solver_params q = *p;
+        q.compute_true_residual = 0;   // a slab solve reports none
+        rc = dare_bicgstab2_fp64(&view, &q, rep);
+        sl->systems[0]->ws = view.ws;
+        return rc;
+    }
     SolverState init{};
     init.tol = p->tol;
     init.max_it = p->max_it;

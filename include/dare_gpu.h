@@ -198,7 +198,8 @@ DARE_API const char* dare_ctx_last_error(const dare_ctx* ctx);
 DARE_API int64_t dare_ctx_launch_count(const dare_ctx* ctx);
 /* Optional per-kernel CUDA-event timing on the context's stream (no reference
  * counterpart: the reference has no timers).  Kernel ids: 0 assembly,
- * 3..7 the five fused BiCGStab(2) kernels (steps 5-7, 8-11, 12-14, 15-23, 24-25). */
+ * 3..7 the five fused BiCGStab(2) kernels (steps 5-7, 8-11, 12-14, 15-23, 24-25),
+ * 8 the whole solve of a small system, which runs as one kernel. */
 DARE_API int dare_ctx_set_profiling(dare_ctx* ctx, int on);
 DARE_API int dare_ctx_reset_kernel_stats(dare_ctx* ctx);
 DARE_API int dare_ctx_kernel_stats(const dare_ctx* ctx, int kernel_id, double* total_ms, int64_t* count);
