@@ -35,12 +35,7 @@ void dare_solver_ws_free(dare_solver_ws* ws) {
     for (auto& row : ws->graph)
         for (auto& g : row)
             if (g) cudaGraphExecDestroy(g);
-    cudaFree(ws->ahat);
-    cudaFree(ws->invd);
-    cudaFree(ws->vec);
-    cudaFree(ws->partials);
-    cudaFree(ws->packets);
-    cudaFree(ws->st);
+    cudaFree(ws->ahat);   // invd .. st are parts of it
     if (ws->st_host) cudaFreeHost(ws->st_host);
     dare_mixed_ws_free(ws);
     dare_learned_ws_free(ws->learned);
@@ -101,14 +96,28 @@ int ensure_solver_ws(dare_system* s) {
     dare_solver_ws* ws = new (std::nothrow) dare_solver_ws();
     if (!ws) return DARE_ERR_OOM;
     ws->n = n;
-    cudaError_t e = cudaMalloc(&ws->ahat, (size_t)n * 6 * sizeof(double));
-    if (e == cudaSuccess) e = cudaMalloc(&ws->invd, (size_t)n * sizeof(double));
-    if (e == cudaSuccess) e = cudaMalloc(&ws->vec, (size_t)n * kNumSolverVecs * sizeof(double));
-    if (e == cudaSuccess) e = cudaMalloc(&ws->partials, (size_t)kMaxQ * kMaxBlocks * sizeof(double) + 64);
-    if (e == cudaSuccess) e = cudaMalloc(&ws->packets, kTeamBytes);
-    if (e == cudaSuccess) e = cudaMemsetAsync(ws->packets, 0, kTeamBytes, ctx->stream);
-    if (e == cudaSuccess) e = cudaMalloc(&ws->st, sizeof(SolverState));
-    if (e == cudaSuccess) e = cudaMemsetAsync(ws->st, 0, sizeof(SolverState), ctx->stream);
+    // one allocation, its parts on 256-byte lines
+    size_t total = 0;
+    const auto part = [&](size_t bytes) {
+        const size_t at = total;
+        total += (bytes + 255) / 256 * 256;
+        return at;
+    };
+    const size_t at_ahat = part((size_t)n * 6 * sizeof(double)), at_invd = part((size_t)n * sizeof(double));
+    const size_t at_vec = part((size_t)n * kNumSolverVecs * sizeof(double));
+    const size_t at_part = part((size_t)kMaxQ * kMaxBlocks * sizeof(double) + 64);
+    const size_t at_team = part(sizeof(TeamBuffer)), at_st = part(sizeof(SolverState));
+    char* base = nullptr;
+    cudaError_t e = cudaMalloc(&base, total);
+    if (e == cudaSuccess) {
+        ws->ahat = reinterpret_cast<double*>(base + at_ahat);
+        ws->invd = reinterpret_cast<double*>(base + at_invd);
+        ws->vec = reinterpret_cast<double*>(base + at_vec);
+        ws->partials = reinterpret_cast<double*>(base + at_part);
+        ws->team_buf = base + at_team;
+        ws->st = reinterpret_cast<SolverState*>(base + at_st);
+        e = cudaMemsetAsync(ws->team_buf, 0, total - at_team, ctx->stream);
+    }
     if (e == cudaSuccess) e = cudaMallocHost(&ws->st_host, sizeof(SolverState));
     if (e != cudaSuccess) {
         dare_solver_ws_free(ws);
@@ -394,7 +403,7 @@ int dare_bicgstab2_fp64_to(dare_system* s, const dare_solver_params* p, dare_sol
     double* tres = &ws->st->tres;
     // Small systems run in one launch (timed as one kernel when profiling)
     int blocks = 0, chunk = 0;
-    if (resident_shape(ctx, n, jacobi, &blocks, &chunk)) {
+    if (resident_shape(ctx, g, jacobi, &blocks, &chunk)) {
         const bool prof = ctx->profiling != 0;
         if (prof) DARE_CUDA(ctx, cudaEventRecord(ctx->ev[0], ctx->stream));
         if ((rc = launch_resident(s, p, vs, blocks, chunk, to_field ? f->level[0] : nullptr))) return rc;
@@ -406,7 +415,7 @@ int dare_bicgstab2_fp64_to(dare_system* s, const dare_solver_params* p, dare_sol
             ctx->stat_n[KID_SOLVE] += 1;
         }
         if (!ws->st_host->done) {   // a wait between its blocks ran out: start the exchanges over
-            DARE_CUDA(ctx, cudaMemsetAsync(ws->packets, 0, kTeamBytes, ctx->stream));
+            DARE_CUDA(ctx, cudaMemsetAsync(ws->team_buf, 0, sizeof(TeamBuffer), ctx->stream));
             return set_error(ctx, DARE_ERR_TIMEOUT, "bicgstab2: a wait between blocks ran out");
         }
     } else {

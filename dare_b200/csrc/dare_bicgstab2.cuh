@@ -170,7 +170,7 @@ int launch_fold32(dare_ctx* ctx, const GridDev& g, const MarchCfg& m, const doub
                   SolverState* st, double* partials);
 int launch_scale(dare_ctx* ctx, int64_t n, const double* invd, double* x);
 // The one-launch solve of small systems (dare_resident.cu)
-bool resident_shape(const dare_ctx* ctx, int64_t n, bool unit, int* blocks, int* chunk);
+bool resident_shape(const dare_ctx* ctx, const GridDev& g, bool unit, int* blocks, int* chunk);
 int launch_resident(dare_system* s, const dare_solver_params* p, const VecsT<double>& vs, int blocks, int chunk,
                     double* field);
 // Apply step (10) when the solve stopped between it and the last kernel of
@@ -192,7 +192,7 @@ struct dare_solver_ws {
     cudaGraphExec_t graph[3][2] = {{nullptr, nullptr}, {nullptr, nullptr}, {nullptr, nullptr}};
     dare_gpu::MarchCfg march;
     int stream_blocks = 0;
-    unsigned long long* packets = nullptr;   // exchanges of the one-launch solve (dare_team.cuh)
+    void* team_buf = nullptr;   // exchanges of the one-launch solve (dare_team.cuh)
     // FP32 inner solver of the refinement driver (dare_mixed.cu)
     float* ahat32 = nullptr;     // 6 * n
     float* vec32 = nullptr;      // (kNumSolverVecs + 2) * n: work vectors, the correction, the right-hand side

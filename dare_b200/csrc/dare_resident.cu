@@ -27,94 +27,153 @@ struct ResidentArgs {
     TeamVecs v;
     double tol;
     int max_it, tol_relative, want_residual;
-    unsigned long long* packets;   // exchange packets, then the number of the last exchange (kTeamEpoch)
+    TeamBuffer* buf;
     SolverState *st, *st_host;     // results (device copy, pinned host copy)
 };
 
-// Rows of this block in shared memory: NC coefficients of m cells (stride
-// `chunk`), and the faces each cell touches.
-template <bool UNIT>
+// 1024 threads and one block per SM: 64 registers each, and 32 warps to hide
+// the L2 latency of one another.
+constexpr int kResidentThreads = 1024;
+
+// The rows of this block in shared memory: NC coefficients of m cells (stride
+// `stride`), the faces each cell touches, and a tile for the operand on the
+// block's cells and the rows before and after them, where the j and k
+// neighbours are.  A block's cells are a run in memory, usually shorter than a
+// plane, so the i neighbours have no second reader here: each thread forms
+// its own cells' from global memory.  CPT cells a thread, all their loads in
+// flight before the barrier: a 64^3 pass takes 2.6 us (operand formed at all 7
+// points from L1 3.1 us), an 82^3 pass 4.8 us (6.6).
+template <bool UNIT, int CPT>
 struct ResidentOp {
-    TeamGeo geo;
-    const double* coef;
-    const unsigned char* faces;
-    int stride, m, c0;
-    template <class F>
-    __device__ __forceinline__ double row(int lc, int c, F zf, double& z0) const {
-        double z[7];
-        team_points(geo, c, faces[lc], zf, z);
-        z0 = z[0];
-        double y = UNIT ? z[0] : coef[6 * stride + lc] * z[0];
+    const TeamGeo& geo;
+    double *coef, *tile;
+    unsigned char* faces;
+    int ncell, stride, m, c0;
+
+    // the thread's first cell, opaque to the compiler: otherwise it keeps the
+    // addresses of every cell from one pass to the next, in spilled registers
+    __device__ __forceinline__ int first() const {
+        int t = threadIdx.x;
+        asm volatile("" : "+r"(t));
+        return t;
+    }
+    __device__ __forceinline__ bool gone(unsigned f, int q) const { return (f & geo.gone) >> q & 1u; }
+    template <class ZF, class Pre, class Body>
+    __device__ __forceinline__ void pass(ZF zf, Pre pre, Body body) {
+        constexpr int nt = kResidentThreads;
+        const int tid = first(), sy = geo.sy;
+        double zw[CPT], ze[CPT], p[CPT];
 #pragma unroll
-        for (int q = 0; q < 6; q++) y += coef[q * stride + lc] * z[q + 1];
-        return y;
+        for (int q = 0; q < CPT; q++) {
+            const int lc = tid + q * nt, c = c0 + lc;
+            if (lc < m) {
+                const unsigned f = faces[lc];
+                const double z = zf(c);
+                const double w = zf(c + (f & 1u ? geo.off[0] : -geo.sx)), e = zf(c + (f & 2u ? geo.off[1] : geo.sx));
+                p[q] = pre(c);
+                zw[q] = gone(f, 0) ? 0. : w;
+                ze[q] = gone(f, 1) ? 0. : e;
+                tile[sy + lc] = z;
+            }
+        }
+        for (int h = tid; h < 2 * sy; h += nt) {
+            const int lc = h < sy ? h - sy : m + h - sy, c = c0 + lc;
+            tile[sy + lc] = c >= 0 && c < ncell ? zf(c) : 0.;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < CPT; q++) {
+            const int lc = tid + q * nt, c = c0 + lc;
+            if (lc < m) {
+                const unsigned f = faces[lc];
+                const double *t = tile + sy + lc, *a = coef + lc;
+                // past a periodic j face the neighbour is n1 - 1 rows away,
+                // past a k face n2 - 1 cells: inside the tile
+                const double s = gone(f, 2) ? 0. : f & 4u ? zf(c + geo.off[2]) : t[-sy];
+                const double n = gone(f, 3) ? 0. : f & 8u ? zf(c + geo.off[3]) : t[sy];
+                const double b = gone(f, 4) ? 0. : t[f & 16u ? geo.off[4] : -1];
+                const double u = gone(f, 5) ? 0. : t[f & 32u ? geo.off[5] : 1];
+                double y = UNIT ? t[0] : a[6 * stride] * t[0];
+                y += a[0] * zw[q];
+                y += a[stride] * ze[q];
+                y += a[2 * stride] * s;
+                y += a[3 * stride] * n;
+                y += a[4 * stride] * b;
+                y += a[5 * stride] * u;
+                body(c, y, t[0], p[q]);
+            }
+        }
+    }
+    template <int U, class Body>
+    __device__ __forceinline__ void each(Body body) {
+#pragma unroll U
+        for (int lc = first(); lc < m; lc += kResidentThreads) body(c0 + lc);
+    }
+    // f at the six neighbours of own cell c, zero where there is none
+    template <class F>
+    __device__ __forceinline__ void neighbours(int c, F f, double (&z)[6]) const {
+        const int step[6] = {-geo.sx, geo.sx, -geo.sy, geo.sy, -1, 1};
+        const unsigned at = faces[c - c0];
+#pragma unroll
+        for (int q = 0; q < 6; q++) z[q] = gone(at, q) ? 0. : f(c + (at >> q & 1u ? geo.off[q] : step[q]));
     }
 };
 
-// 1024 threads and one block per SM: 64 registers each, enough for one cell's
-// loads in flight, and 32 warps hide the L2 latency of the others.
-constexpr int kResidentThreads = 1024;
-
-template <bool UNIT>
+template <bool UNIT, int CPT>
 __global__ void __launch_bounds__(kResidentThreads, 1) k_resident(ResidentArgs A) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ TeamShared sh;
     __shared__ SolverState st_s;
     SolverState* st = &st_s;
-    const int tid = threadIdx.x, nt = blockDim.x;
+    const int tid = threadIdx.x;
     constexpr int NC = NCoef<UNIT>::value;
-    double* coef = reinterpret_cast<double*>(smem_raw);
-    unsigned char* faces = smem_raw + (size_t)NC * A.chunk * sizeof(double);
-    const int c0 = blockIdx.x * A.chunk;
-    const int m = max(0, min(A.chunk, A.ncell - c0));
     const int64_t n = A.ncell;
-    GridTeam team{A.packets, &sh, (int)blockIdx.x, (int)gridDim.x, (unsigned)A.packets[kTeamEpoch]};
+    const int ch = A.chunk, c0 = blockIdx.x * ch, m = max(0, min(ch, A.ncell - c0));
+    double* smem = reinterpret_cast<double*>(smem_raw);
+    ResidentOp<UNIT, CPT> op{A.geo, smem,      smem + (size_t)NC * ch,
+                             reinterpret_cast<unsigned char*>(smem + (size_t)(NC + 1) * ch + 2 * A.geo.sy),
+                             A.ncell, ch, m, c0};
+    GridTeam team{A.buf, &sh, (int)blockIdx.x, (int)gridDim.x, 0u};
+    team.start();
     if (tid == 0) {
-        sh.timeout = 0;
         SolverState z{};
         z.tol = A.tol;
         z.max_it = A.max_it;
         z.tol_relative = A.tol_relative;
         *st = z;
     }
-    for (int lc = tid; lc < m; lc += nt) {
-        faces[lc] = (unsigned char)team_faces(A.geo, c0 + lc);
-        if (UNIT) A.invd[c0 + lc] = 1. / A.diag[c0 + lc];
-    }
+    op.template each<1>([&](int c) {
+        op.faces[c - c0] = (unsigned char)team_faces(A.geo, c);
+        if (UNIT) A.invd[c] = 1. / A.diag[c];
+    });
     bool ok = true;
-    double none[1] = {0.}, dummy[1];
-    if (UNIT) ok = team.sum<1>(none, dummy);   // invd of every block
-    else __syncthreads();
+    const double none[1] = {0.};
+    __syncthreads();
+    if (UNIT) ok = team.sum<1>(none, [](const double*) {});   // invd of every block
     // Ahat = A D^-1 (columns scaled) into shared memory; r = b - Ahat y,
     // r_hat_0 = r, u = 0
-    double a2[2] = {0., 0.}, t2[2] = {0., 0.};
     if (ok) {
-        const ResidentOp<UNIT> op{A.geo, coef, faces, A.chunk, m, c0};
-        for (int lc = tid; lc < m; lc += nt) {
-            const int c = c0 + lc;
-            if constexpr (UNIT) {
-                double iv[7];
-                team_points(A.geo, c, faces[lc], [&](int e) { return A.invd[e]; }, iv);
+        op.template each<1>([&](int c) {
+            double iv[6];
+            if (UNIT) op.neighbours(c, [&](int e) { return A.invd[e]; }, iv);
 #pragma unroll
-                for (int q = 0; q < 6; q++) coef[q * A.chunk + lc] = A.diag[(q + 1) * n + c] * iv[q + 1];
-            } else {
-#pragma unroll
-                for (int q = 0; q < 6; q++) coef[q * A.chunk + lc] = A.diag[(q + 1) * n + c];
-                coef[6 * A.chunk + lc] = A.diag[c];
+            for (int q = 0; q < 6; q++) {
+                const double a = A.diag[(q + 1) * n + c];
+                op.coef[q * ch + c - c0] = UNIT ? a * iv[q] : a;
             }
-            double y0;
-            const double yy = op.row(lc, c, [&](int e) { return A.v.x[e]; }, y0);
-            const double bc = A.b[c], rr = bc - yy;
-            A.v.r[c] = rr;
-            A.v.rh[c] = rr;
-            A.v.u[c] = 0.;
-            a2[0] += rr * rr;
-            a2[1] += bc * bc;
-        }
-        ok = team.sum<2>(a2, t2);
-        if (ok && tid == 0) finish_init(st, t2);
-        __syncthreads();
-        ok = ok && team_iterations(team, op, A.v, st);
+            if (!UNIT) op.coef[6 * ch + c - c0] = A.diag[c];
+        });
+        double a2[2] = {0., 0.};
+        op.pass([&](int e) { return A.v.x[e]; }, [&](int c) { return A.b[c]; },
+                [&](int c, double y, double, double bc) {
+                    const double rr = bc - y;
+                    A.v.r[c] = rr;
+                    A.v.rh[c] = rr;
+                    A.v.u[c] = 0.;
+                    a2[0] += rr * rr;
+                    a2[1] += bc * bc;
+                });
+        ok = team.sum<2>(a2, [&](const double* t) { finish_init(st, t); }) && team_iterations(team, op, A.v, st);
     }
     if (ok) {
         // the exit: step (10) when the solve stopped between it and the last
@@ -123,8 +182,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1) k_resident(ResidentArgs A
         const bool pend = step10_pending_state(st->status, st->step);
         const double alpha1 = st->alpha1, beta5 = st->beta5;
         const GridDev& g = A.grid;
-        for (int lc = tid; lc < m; lc += nt) {
-            const int c = c0 + lc;
+        op.template each<1>([&](int c) {
             double xc = A.v.x[c];
             if (pend) {
                 const double u5 = A.v.r[c] - beta5 * A.v.u[c];
@@ -132,7 +190,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1) k_resident(ResidentArgs A
             }
             if (UNIT) xc = A.invd[c] * xc;
             if (UNIT || pend) A.v.x[c] = xc;
-            if (!A.field) continue;
+            if (!A.field) return;
             const int ia = c / A.geo.sx, rem = c - ia * A.geo.sx, j = rem / A.geo.sy, k = rem - j * A.geo.sy;
             const int comp = ia / A.geo.n0;
             double* phi = A.field + (size_t)comp * g.ncell_ghosted;
@@ -151,30 +209,32 @@ __global__ void __launch_bounds__(kResidentThreads, 1) k_resident(ResidentArgs A
                     phi[((int64_t)p[0] * g.gn[1] + p[1]) * g.gn[2] + p[2]] = xc;
                 }
             }
-        }
+        });
         if (A.want_residual) {   // ||b - A x||_2 with the assembled rows
-            ok = team.sum<1>(none, dummy);
-            double a1[1] = {0.}, t1[1] = {0.};
+            ok = team.sum<1>(none, [](const double*) {});
+            double a1[1] = {0.};
             if (ok) {
-                for (int lc = tid; lc < m; lc += nt) {
-                    const int c = c0 + lc;
-                    double z[7];
-                    team_points(A.geo, c, faces[lc], [&](int e) { return A.v.x[e]; }, z);
-                    double y = A.diag[c] * z[0];
+                op.template each<1>([&](int c) {
+                    double z[7], p[7], zn[6];
+                    op.neighbours(c, [&](int e) { return A.v.x[e]; }, zn);
+                    z[0] = A.v.x[c];
+                    p[6] = A.diag[c];
 #pragma unroll
-                    for (int q = 0; q < 6; q++) y += A.diag[(q + 1) * n + c] * z[q + 1];
-                    const double r = A.b[c] - y;
+                    for (int q = 0; q < 6; q++) {
+                        z[q + 1] = zn[q];
+                        p[q] = A.diag[(q + 1) * n + c];
+                    }
+                    const double r = A.b[c] - apply_pre<double, false>(p, z);
                     a1[0] += r * r;
-                }
-                ok = team.sum<1>(a1, t1);
+                });
+                ok = team.sum<1>(a1, [&](const double* t) { st->tres = sqrt(t[0]); });
             }
-            if (tid == 0) st->tres = sqrt(t1[0]);
         }
     }
     // a block that gave up leaves `done` 0 in its copy; block 0 reports
+    team.stop();
     if (blockIdx.x == 0 && tid == 0) {
         if (!ok) st->done = 0;
-        A.packets[kTeamEpoch] = team.epoch;   // every block read it before the first exchange
         *A.st = *st;
         *A.st_host = *st;
     }
@@ -183,34 +243,47 @@ __global__ void __launch_bounds__(kResidentThreads, 1) k_resident(ResidentArgs A
 // The team's shape for a system, or false when a block's rows do not fit its
 // shared memory: beyond that the marching kernels are the faster path (their
 // vectors no longer stay in L2 either).
-static size_t resident_smem(bool unit, int chunk) {
-    return (size_t)chunk * ((unit ? 6 : 7) * sizeof(double) + 1);
+constexpr int kResidentCells = 4;   // most cells a thread
+static size_t resident_smem(bool unit, int chunk, int sy) {
+    return ((size_t)chunk * (unit ? 7 : 8) + 2 * (size_t)sy) * sizeof(double) + chunk;
 }
-bool resident_shape(const dare_ctx* ctx, int64_t n, bool unit, int* blocks, int* chunk) {
+bool resident_shape(const dare_ctx* ctx, const GridDev& g, bool unit, int* blocks, int* chunk) {
     constexpr size_t kMost = 227 * 1024 - sizeof(TeamShared) - sizeof(SolverState) - 1024;
+    const int64_t n = g.ncell;
     const int nb = ctx->num_sms < kTeamMaxBlocks ? ctx->num_sms : kTeamMaxBlocks;
-    if (n > (int64_t)nb * 8192) return false;
+    if (n > (int64_t)nb * kResidentThreads * kResidentCells) return false;
     // as many blocks as have a cell for each of half their threads: below
     // that an SM more does not shorten a pass
     int64_t want = (n + kResidentThreads / 2 - 1) / (kResidentThreads / 2);
     if (want > nb) want = nb;
     int64_t ch = (n + want - 1) / want;
     ch = (ch + 31) / 32 * 32;
-    if (resident_smem(unit, (int)ch) > kMost) return false;
+    if (ch > kResidentThreads * kResidentCells || g.n[2] > (1 << 15) || resident_smem(unit, (int)ch, g.n[2]) > kMost)
+        return false;
     *chunk = (int)ch;
     *blocks = (int)((n + ch - 1) / ch);
     return true;
 }
 
-template <bool UNIT>
+template <bool UNIT, int CPT>
 static int launch_resident_t(dare_ctx* ctx, ResidentArgs& a, int blocks) {
-    const size_t smem = resident_smem(UNIT, a.chunk);
-    DARE_CUDA(ctx, cudaFuncSetAttribute(k_resident<UNIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const size_t smem = resident_smem(UNIT, a.chunk, a.geo.sy);
+    const auto k = k_resident<UNIT, CPT>;
+    DARE_CUDA(ctx, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     void* args[] = {&a};
-    DARE_CUDA(ctx, cudaLaunchCooperativeKernel((const void*)k_resident<UNIT>, dim3(blocks), dim3(kResidentThreads), args,
-                                               smem, ctx->stream));
+    DARE_CUDA(ctx, cudaLaunchCooperativeKernel((const void*)k, dim3(blocks), dim3(kResidentThreads), args, smem,
+                                               ctx->stream));
     DARE_LAUNCHED(ctx);
     return DARE_OK;
+}
+template <bool UNIT>
+static int launch_resident_u(dare_ctx* ctx, ResidentArgs& a, int blocks) {
+    switch ((a.chunk + kResidentThreads - 1) / kResidentThreads) {
+    case 1: return launch_resident_t<UNIT, 1>(ctx, a, blocks);
+    case 2: return launch_resident_t<UNIT, 2>(ctx, a, blocks);
+    case 3: return launch_resident_t<UNIT, 3>(ctx, a, blocks);
+    default: return launch_resident_t<UNIT, kResidentCells>(ctx, a, blocks);
+    }
 }
 
 // The whole solve of system s in one launch: x (and field level 0 when given)
@@ -234,11 +307,11 @@ int launch_resident(dare_system* s, const dare_solver_params* p, const VecsT<dou
     a.max_it = p->max_it;
     a.tol_relative = p->tol_relative;
     a.want_residual = p->compute_true_residual;
-    a.packets = ws->packets;
+    a.buf = static_cast<TeamBuffer*>(ws->team_buf);
     a.st = ws->st;
     a.st_host = ws->st_host;
-    return p->precond == DARE_PREC_JACOBI ? launch_resident_t<true>(ctx, a, blocks)
-                                          : launch_resident_t<false>(ctx, a, blocks);
+    return p->precond == DARE_PREC_JACOBI ? launch_resident_u<true>(ctx, a, blocks)
+                                          : launch_resident_u<false>(ctx, a, blocks);
 }
 
 }  // namespace dare_gpu

@@ -21,98 +21,173 @@
 
 namespace dare_gpu {
 
-constexpr int kTeamMaxBlocks = 160;   // blocks of a grid team (packets of one exchange)
-constexpr int kTeamEpoch = 2 * kMaxQ * kTeamMaxBlocks * 2;   // word of a grid team's buffer: its last exchange
-constexpr size_t kTeamBytes = (kTeamEpoch + 1) * sizeof(unsigned long long);
+constexpr int kTeamMaxBlocks = 160;   // blocks of a grid team
+constexpr int kTeamPolls = 1 << 22;   // polls of a wait before the block gives up
+
+__device__ __forceinline__ double team_xor(double v, int o) { return __shfl_xor_sync(0xffffffffu, v, o); }
+
+// Sums of Q values over a warp, red[q * 32 + warp] written by one lane each.
+// Several values share the shuffles: at each step a lane hands over the half
+// of its values that the other lane will sum (5 values: 8 shuffles, not 25;
+// a double costs two of the SM's 32 lanes a clock, and 32 warps wait for it).
+template <int Q>
+__device__ __forceinline__ void team_warp_sums(const double (&v)[Q], double* red) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    if constexpr (Q == 1) {
+        double a = v[0];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) a += team_xor(a, o);
+        if (lane == 0) red[wid] = a;
+    } else if constexpr (Q == 2) {
+        const bool h = lane & 16;
+        double a = h ? v[1] : v[0];
+        a += team_xor(h ? v[0] : v[1], 16);
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) a += team_xor(a, o);
+        if ((lane & 15) == 0) red[(h ? 32 : 0) + wid] = a;
+    } else {
+        static_assert(Q == 5, "one, two or five values");
+        // lanes 0-15 keep values 0, 1, 2 and lanes 16-31 values 3, 4; then by
+        // bit 3 the pair (0, 1) or 2, the pair (3, 4) or none; then by bit 2
+        const bool h = lane & 16, h8 = lane & 8, h4 = lane & 4;
+        double k0 = h ? v[3] : v[0], k1 = h ? v[4] : v[1], k2 = h ? 0. : v[2];
+        k0 += team_xor(h ? v[0] : v[3], 16);
+        k1 += team_xor(h ? v[1] : v[4], 16);
+        k2 += team_xor(h ? v[2] : 0., 16);
+        double m0 = h8 ? k2 : k0, m1 = h8 ? 0. : k1;
+        m0 += team_xor(h8 ? k0 : k2, 8);
+        m1 += team_xor(h8 ? k1 : 0., 8);
+        double a = h4 ? m1 : m0;
+        a += team_xor(h4 ? m0 : m1, 4);
+        a += team_xor(a, 2);
+        a += team_xor(a, 1);
+        const int q = (h ? 3 : 0) + (h8 ? 2 : 0) + (h4 ? 1 : 0);
+        if ((lane & 3) == 0 && !(h8 && (h4 || h))) red[q * 32 + wid] = a;
+    }
+}
 
 // Block part of a sum: afterwards warp q (q < Q) holds the block's sum of
 // value q in every lane.  The barrier inside also orders every store of the
 // block before what those warps do next.
 template <int Q>
-__device__ __forceinline__ double team_block_sum(double (&v)[Q], double* red /* [32 * kMaxQ] */) {
-#pragma unroll
-    for (int q = 0; q < Q; q++) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v[q] += __shfl_xor_sync(0xffffffffu, v[q], o);
-    }
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    if (lane == 0) {
-#pragma unroll
-        for (int q = 0; q < Q; q++) red[q * 32 + wid] = v[q];
-    }
+__device__ __forceinline__ double team_block_sum(const double (&v)[Q], double* red /* [32 * kMaxQ] */) {
+    team_warp_sums<Q>(v, red);
     __syncthreads();
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     double a = 0.;
     if (wid < Q) {
         a = lane < ((int)blockDim.x >> 5) ? red[wid * 32 + lane] : 0.;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+        for (int o = 16; o > 0; o >>= 1) a += team_xor(a, o);
     }
     return a;
 }
 
+// A grid team's buffer in global memory: per value a counter of arrivals on a
+// line of its own, the arrivals at the end of the last launch, and two sets
+// (a block can be one exchange ahead of another at most, which still reads
+// the other set) of partial sums and of totals.  A total is stored as its two
+// halves, each beside the low word of the counter's value it belongs to:
+// 8-byte accesses are single, so a reader that finds that word in both has it.
+struct TeamBuffer {
+    struct {
+        unsigned n, pad[31];
+    } arrived[kMaxQ];
+    unsigned base[kMaxQ], set;
+    struct {
+        unsigned long long half[2], pad[14];
+    } total[2][kMaxQ];
+    double parts[2][kMaxQ][kTeamMaxBlocks];
+};
+
 // Shared-memory scratch of a team's exchanges.
 struct TeamShared {
     double red[32 * kMaxQ];
-    double parts[kMaxQ * kTeamMaxBlocks];   // cluster teams: [2][kMaxQ][16], written by the peers
+    double tot[kMaxQ];
+    unsigned target[kMaxQ];
     int timeout;
 };
 
-// The blocks of a cooperative launch.  Each exchange, a block publishes one
-// 16-byte packet per value: the double's two halves, each beside the
-// exchange's number, so that a reader that sees the number in both words has
-// the value (8-byte stores are single) and needs no separate flag.  Every
-// block polls the packets of all blocks: one store and one load latency,
-// without atomics.  Packets alternate between two sets: a block can be one
-// exchange ahead of another at most, which still reads the other set.
+// The blocks of a cooperative launch.  Value q is handled by warp q of every
+// block: it stores the block's sum and counts itself in; the last one adds the
+// sums in block order and publishes the total the others wait for.  148
+// blocks that all read all 148 partial sums queue at the few L2 slices that
+// hold them (4000 cycles on top of 1200, every other exchange), which is why
+// one does.
 // Every wait ends: after kTeamPolls polls the block gives up, and so do the
 // blocks that wait for it.
-constexpr int kTeamPolls = 1 << 22;
 struct GridTeam {
-    unsigned long long* packets;   // [2][kMaxQ][size][2]
+    TeamBuffer* buf;
     TeamShared* sh;
     int rank, size;
-    unsigned epoch;                // number of the last exchange
+    unsigned set;   // partial-sum set of the last exchange
 
-    // Totals of Q values in thread 0 (tot), after a barrier of the team.
-    // False when a wait ran out.
-    template <int Q>
-    __device__ bool sum(double (&v)[Q], double (&tot)[Q]) {
-        epoch++;
+    __device__ void start() {   // before the block's first barrier
+        if (threadIdx.x < kMaxQ) sh->target[threadIdx.x] = buf->base[threadIdx.x];
+        if (threadIdx.x == 0) sh->timeout = 0;
+        set = buf->set;
+    }
+    __device__ void stop() {    // after the last exchange
+        if (rank == 0 && threadIdx.x < kMaxQ) buf->base[threadIdx.x] = sh->target[threadIdx.x];
+        if (rank == 0 && threadIdx.x == 0) buf->set = set;
+    }
+    // The totals of Q values to fin(tot) in thread 0, then a barrier of the
+    // block: what any block stored before its call is visible to all.  False
+    // (in every thread) when a wait ran out; fin is not run then.
+    template <int Q, class F>
+    __device__ bool sum(const double (&v)[Q], F fin) {
+        set ^= 1u;
         const double a = team_block_sum<Q>(v, sh->red);
         const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-        unsigned long long* set = packets + (size_t)(epoch & 1u) * kMaxQ * size * 2;
-        const unsigned long long tag = (unsigned long long)epoch << 32;
-        if (wid < Q && lane == 0) {
-            const unsigned long long bits = (unsigned long long)__double_as_longlong(a);
-            asm volatile("fence.acq_rel.gpu;" ::: "memory");
-            asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(set + 2 * ((size_t)wid * size + rank)),
-                         "l"(tag | (bits & 0xffffffffull)), "l"(tag | (bits >> 32))
-                         : "memory");
-        }
-        bool mine = false;
-        for (int p = threadIdx.x; p < Q * size; p += blockDim.x) {
-            unsigned long long lo, hi;
-            int polls = 0;
-            do {
-                asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(lo), "=l"(hi) : "l"(set + 2 * (size_t)p)
-                             : "memory");
-            } while (((lo ^ tag) >> 32 || (hi ^ tag) >> 32) && ++polls < kTeamPolls);
-            if (polls >= kTeamPolls) sh->timeout = 1;
-            sh->parts[p] = __longlong_as_double((long long)((lo & 0xffffffffull) | (hi << 32)));
-            mine = true;
-        }
-        if (mine) asm volatile("fence.acq_rel.gpu;" ::: "memory");
-        __syncthreads();
-        if (wid == 0) {
-#pragma unroll
-            for (int q = 0; q < Q; q++) {
+        if (wid < Q) {
+            double* parts = buf->parts[set][wid];
+            unsigned long long* total = buf->total[set][wid].half;
+            unsigned* n = &buf->arrived[wid].n;
+            unsigned target = 0, old = 0;
+            if (lane == 0) {
+                target = sh->target[wid] + (unsigned)size;
+                sh->target[wid] = target;
+                asm volatile("st.relaxed.gpu.global.f64 [%0], %1;" ::"l"(parts + rank), "d"(a) : "memory");
+                asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(old) : "l"(n) : "memory");
+            }
+            if (__shfl_sync(0xffffffffu, old + 1u == target, 0)) {
                 double s = 0.;
-                for (int b = lane; b < size; b += 32) s += sh->parts[q * size + b];
+                for (int b = lane; b < size; b += 32) {
+                    double p;
+                    asm volatile("ld.relaxed.gpu.global.f64 %0, [%1];" : "=d"(p) : "l"(parts + b) : "memory");
+                    s += p;
+                }
 #pragma unroll
-                for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-                tot[q] = s;
+                for (int o = 16; o > 0; o >>= 1) s += team_xor(s, o);
+                if (lane == 0) {
+                    const unsigned long long bits = (unsigned long long)__double_as_longlong(s);
+                    const unsigned long long tag = (unsigned long long)target << 32;
+                    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(total), "l"(tag | (bits & 0xffffffffull))
+                                 : "memory");
+                    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(total + 1), "l"(tag | (bits >> 32))
+                                 : "memory");
+                    sh->tot[wid] = s;
+                }
+            } else if (lane == 0) {
+                // the total, and with the counter's value (acquired) every
+                // store that any block made before it counted itself in
+                unsigned long long lo, hi;
+                unsigned have;
+                int polls = 0;
+                bool wait;
+                do {
+                    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(lo) : "l"(total) : "memory");
+                    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(hi) : "l"(total + 1) : "memory");
+                    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(have) : "l"(n) : "memory");
+                    wait = (unsigned)(lo >> 32) != target || (unsigned)(hi >> 32) != target || (int)(have - target) < 0;
+                } while (wait && ++polls < kTeamPolls);
+                if (wait) sh->timeout = 1;
+                sh->tot[wid] = __longlong_as_double((long long)((lo & 0xffffffffull) | (hi << 32)));
             }
         }
+        if (Q > 1) __syncthreads();   // (one value: thread 0's own warp)
+        if (threadIdx.x == 0 && !sh->timeout) fin(sh->tot);
+        __syncthreads();
         return sh->timeout == 0;
     }
 };
@@ -146,19 +221,6 @@ __device__ __forceinline__ unsigned team_faces(const TeamGeo& g, int c) {
     return (i == 0) | (i == g.n0 - 1) << 1 | (j == 0) << 2 | (j == g.n1 - 1) << 3 | (k == 0) << 4 |
            (k == g.n2 - 1) << 5;
 }
-// the operand zf at the 7 points of cell c, a removed neighbour's value zero
-template <class F>
-__device__ __forceinline__ void team_points(const TeamGeo& g, int c, unsigned f, F zf, double (&z)[7]) {
-    const int step[6] = {-g.sx, g.sx, -g.sy, g.sy, -1, 1};
-    z[0] = zf(c);
-#pragma unroll
-    for (int q = 0; q < 6; q++) {
-        const bool at = f >> q & 1u;
-        const double a = zf(c + (at ? g.off[q] : step[q]));
-        z[q + 1] = at && (g.gone >> q & 1u) ? 0. : a;
-    }
-}
-
 // Vectors of a team solve (global memory, the iterate's values in r and u)
 struct TeamVecs {
     double *x, *rh, *r, *u, *v, *s, *w, *t;
@@ -166,73 +228,60 @@ struct TeamVecs {
 
 // The iterations, from a state that finish_init has set, until it is done:
 // the passes K1 .. K5 of dare_march.cuh over this block's cells.  Op gives
-// m (cells of the block), c0 (the first) and
-//   row(lc, c, zf, z0): the operator's row for operand zf, its own value in z0.
+//   pass(zf, pre, body): for each of the block's cells, body(c, y, z0, pre(c))
+//     with y the operator's row for the operand zf and z0 its own value (pre
+//     is called early, so that its loads run beside the operand's);
+//   each<U>(body): body(c) for each cell, U of them at a time.
 // Returns false when a wait of the team ran out.
+// The four SpMV passes are one loop over (a, b, out, coefficient): every
+// operand has the form b + coefficient a, and the code of one pass keeps the
+// registers of one pass (four copies of it spilled 360 bytes a thread).
 template <class Team, class Op>
-__device__ bool team_iterations(Team& team, const Op& op, const TeamVecs& V, SolverState* st) {
-    const int tid = threadIdx.x, nt = blockDim.x;
+__device__ bool team_iterations(Team& team, Op& op, const TeamVecs& V, SolverState* st) {
     while (!st->done) {
-        double a1[1] = {0.}, t1[1] = {0.};
-        const double beta5 = st->beta;
-        for (int lc = tid; lc < op.m; lc += nt) {                       // (5)-(7)
-            const int c = op.c0 + lc;
-            double z0;
-            const double vc = op.row(lc, c, [&](int e) { return V.r[e] - beta5 * V.u[e]; }, z0);
-            V.v[c] = vc;
-            a1[0] += vc * V.rh[c];
+#pragma unroll 1
+        for (int stage = 0; stage < 4; stage++) {
+            // (5)-(7): v = Op(r - beta5 u); (8), (9), (11): s = Op(r - alpha1 v);
+            // (12)-(14): w = Op(s - beta v); (16)-(20): t = Op(s - alpha w)
+            const double* a = stage == 0 ? V.u : stage == 3 ? V.w : V.v;
+            const double* b = stage < 2 ? V.r : V.s;
+            double* out = stage == 0 ? V.v : stage == 1 ? V.s : stage == 2 ? V.w : V.t;
+            const double alpha = st->alpha, alpha1 = st->alpha1, beta = st->beta;
+            const double coef = stage & 1 ? -alpha : -beta;
+            double dot[5] = {0., 0., 0., 0., 0.};
+            op.pass([&](int e) { return coef * a[e] + b[e]; },
+                    [&](int c) {
+                        return stage < 3 ? V.rh[c] : r_of_16(V.r[c], V.v[c], V.s[c], alpha1, alpha, beta);
+                    },
+                    [&](int c, double y, double z, double p) {
+                        out[c] = y;
+                        if (stage < 3) {
+                            dot[0] += y * p;
+                        } else {
+                            dot[0] += p * z;
+                            dot[1] += z * z;
+                            dot[2] += z * y;
+                            dot[3] += y * y;
+                            dot[4] += p * y;
+                        }
+                    });
+            if (stage < 3) {
+                const double d1[1] = {dot[0]};
+                if (!team.template sum<1>(d1, [&](const double* t) {
+                        if (stage == 1)
+                            finish_rho(st, t);
+                        else
+                            finish_gamma(st, t, stage == 0 ? 7 : 14);
+                    }))
+                    return false;
+            } else if (!team.template sum<5>(dot, [&](const double* t) { finish_omega(st, t); })) {
+                return false;
+            }
+            if (st->done) return true;
         }
-        if (!team.template sum<1>(a1, t1)) return false;
-        if (tid == 0) finish_gamma(st, t1, 7);
-        __syncthreads();
-        if (st->done) break;
-        const double alpha1 = st->alpha;
-        a1[0] = 0.;
-        for (int lc = tid; lc < op.m; lc += nt) {                       // (8), (9), (11)
-            const int c = op.c0 + lc;
-            double z0;
-            const double sc = op.row(lc, c, [&](int e) { return -alpha1 * V.v[e] + V.r[e]; }, z0);
-            V.s[c] = sc;
-            a1[0] += V.rh[c] * sc;
-        }
-        if (!team.template sum<1>(a1, t1)) return false;
-        if (tid == 0) finish_rho(st, t1);
-        __syncthreads();
-        const double beta = st->beta;
-        a1[0] = 0.;
-        for (int lc = tid; lc < op.m; lc += nt) {                       // (12)-(14)
-            const int c = op.c0 + lc;
-            double z0;
-            const double wc = op.row(lc, c, [&](int e) { return V.s[e] - beta * V.v[e]; }, z0);
-            V.w[c] = wc;
-            a1[0] += wc * V.rh[c];
-        }
-        if (!team.template sum<1>(a1, t1)) return false;
-        if (tid == 0) finish_gamma(st, t1, 14);
-        __syncthreads();
-        if (st->done) break;
-        const double alpha = st->alpha;
-        double a5[5] = {0., 0., 0., 0., 0.}, t5[5] = {0., 0., 0., 0., 0.};
-        for (int lc = tid; lc < op.m; lc += nt) {                       // (16)-(20)
-            const int c = op.c0 + lc;
-            double ds;
-            const double dt = op.row(lc, c, [&](int e) { return -alpha * V.w[e] + V.s[e]; }, ds);
-            V.t[c] = dt;
-            const double dr = r_of_16(V.r[c], V.v[c], V.s[c], alpha1, alpha, beta);
-            a5[0] += dr * ds;
-            a5[1] += ds * ds;
-            a5[2] += ds * dt;
-            a5[3] += dt * dt;
-            a5[4] += dr * dt;
-        }
-        if (!team.template sum<5>(a5, t5)) return false;
-        if (tid == 0) finish_omega(st, t5);
-        __syncthreads();
-        if (st->done) break;
         const Step5<double> f(st);
-        double a2[2] = {0., 0.}, t2[2] = {0., 0.};
-        for (int lc = tid; lc < op.m; lc += nt) {                       // (10), (15), (24), (25)
-            const int c = op.c0 + lc;
+        double a2[2] = {0., 0.};
+        op.template each<2>([&](int c) {                                // (10), (15), (24), (25)
             double xc = V.x[c], rc = V.r[c], uc = V.u[c];
             f.cell(xc, rc, uc, V.v[c], V.s[c], V.w[c], V.t[c]);
             V.x[c] = xc;
@@ -240,10 +289,8 @@ __device__ bool team_iterations(Team& team, const Op& op, const TeamVecs& V, Sol
             V.u[c] = uc;
             a2[0] += rc * rc;
             a2[1] += V.rh[c] * rc;
-        }
-        if (!team.template sum<2>(a2, t2)) return false;
-        if (tid == 0) finish_update(st, t2);
-        __syncthreads();
+        });
+        if (!team.template sum<2>(a2, [&](const double* t) { finish_update(st, t); })) return false;
     }
     return true;
 }
