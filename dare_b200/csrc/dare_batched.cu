@@ -1,5 +1,5 @@
 // dare_batched.cu -- thousands of independent implicit diffusion steps of
-// uneven sizes, each solved by Jacobi-BiCGStab(2), in one persistent launch.
+// uneven sizes, each solved by Jacobi-BiCGStab(2) inside one kernel.
 //
 // Every instance is a 3D box with constant D, one implicit-Euler step (DDT +
 // div(D grad), DDT.inl:39-81, Divergence_Cartesian.inl:139-207) and
@@ -10,12 +10,14 @@
 // assembled centre coefficient and its inverse, computed on the host with the
 // same operation order as the assembly kernel.
 //
-// A persistent grid pulls instances from a device queue (heaviest first).
-// One block solves one instance completely -- its reductions are block
-// reductions, so there is no inter-block wait anywhere and results are
-// deterministic -- and records the instance's own convergence status (the
-// per-instance mask of the batch).  The block size and the cells each thread
-// handles per sweep are tuned by dare_batch_autotune.
+// A box is solved to its end by one team of thread blocks, a cluster of 1 to 16
+// of them by its size (k_boxes, dare_team.cuh), so thousands of boxes need no
+// exchange between clusters and results are deterministic.  One persistent
+// launch per cluster size in use pulls its boxes from a device queue, heaviest
+// first, all of them at the same time.  Boxes whose blocks' cells do not fit
+// shared memory (beyond ~65^3) are solved by one block each (k_batched).  Every
+// box records its own convergence status (the per-instance mask of the batch).
+// The block size and the cells a block takes are tuned by dare_batch_autotune.
 #include <algorithm>
 #include <chrono>
 #include <cmath>
@@ -23,14 +25,17 @@
 #include <new>
 #include <vector>
 
-#include "dare_march.cuh"
+#include "dare_team.cuh"
 
 using namespace dare_gpu;
 
 namespace dare_gpu {
 
+constexpr int kBoxClasses = 5;   // cluster sizes 1, 2, 4, 8, 16
+
 struct BInst {
     int n0, n1, n2, vec;
+    int chunk;            // cells of each block of the box's cluster
     int64_t off;          // first cell in the arena
     double tt;            // (V * 1) / dt
     double offd[3];       // off-diagonal per dimension: -(A_d * (dn_d * D))
@@ -63,13 +68,21 @@ struct dare_batch {
     int64_t total = 0;
     std::vector<dare_gpu::BInst> host;
     std::vector<int> order;          // solve order, heaviest first
+    // The boxes by cluster size (1 << class; kBoxClasses: k_batched), each in
+    // solve order, one after the other in d_order; shared memory of a block
+    int class_at[dare_gpu::kBoxClasses + 2] = {0};
+    size_t class_smem[dare_gpu::kBoxClasses] = {0};
+    int class_clusters[dare_gpu::kBoxClasses] = {0};        // resident at a time (0: not asked yet) ...
+    int clusters_block = 0;                                  // ... with this block size
     dare_gpu::BInst* d_inst = nullptr;
     int* d_order = nullptr;
     dare_gpu::BOut* d_out = nullptr;
-    unsigned* d_queue = nullptr;
+    unsigned* d_queue = nullptr;     // one per class
+    cudaStream_t side[dare_gpu::kBoxClasses] = {nullptr};   // the classes run side by side
+    cudaEvent_t fork = nullptr, join[dare_gpu::kBoxClasses] = {nullptr};
     double* arena = nullptr;         // 9 vectors of `total` cells
     int block = 512;
-    int vec_by_size[8] = {1, 1, 1, 1, 1, 1, 1, 1};
+    int vec_by_size[8] = {2, 2, 2, 2, 2, 2, 2, 2};
 };
 
 namespace dare_gpu {
@@ -396,6 +409,181 @@ __global__ void __launch_bounds__(1024) k_batched(const BInst* __restrict__ inst
 
 #undef DARE_SWEEP
 
+// ---------------------------------------------------------------------------
+// k_boxes: a cluster solves a box
+// ---------------------------------------------------------------------------
+// The rows of one block's cells of a box.  A pass forms the operand, already
+// scaled by D^-1, on the block's cells and the plane before and after them, a
+// run of memory that the block loads once into a shared-memory tile; the rows
+// of A are then applied to the tile.  (The one-block kernel below read all
+// seven points of a row from L1 or L2, with a table look-up for each, and one
+// SM had to move a whole box: 64^3 boxes took 12 ms a step on it.)
+struct BoxOp {
+    int sx, sy;
+    double off0, off1, off2;
+    const double *C, *invd;           // centre coefficient and its inverse by boundary mask
+    double* tile;
+    const unsigned char* faces;       // boundary mask of each tile cell
+    int t0, tn, c0, m;                // first cell and cells of the tile, of the block
+
+    template <class ZF, class Pre, class Body>
+    __device__ __forceinline__ void pass(ZF zf, Pre pre, Body body) const {
+        const int tid = threadIdx.x, nt = blockDim.x;
+#pragma unroll 4
+        for (int e = tid; e < tn; e += nt) tile[e] = invd[faces[e]] * zf(t0 + e);
+        __syncthreads();
+#pragma unroll 2
+        for (int lc = tid; lc < m; lc += nt) {
+            const int c = c0 + lc, e = c - t0;
+            const unsigned f = faces[e];
+            const double* t = tile + e;
+            const double w = f & 1u ? 0. : t[-sx], ea = f & 2u ? 0. : t[sx];
+            const double so = f & 4u ? 0. : t[-sy], no = f & 8u ? 0. : t[sy];
+            const double bo = f & 16u ? 0. : t[-1], to = f & 32u ? 0. : t[1];
+            const double z0 = C[f] * t[0];
+            double y = z0 + off0 * (w + ea);
+            y += off1 * (so + no);
+            y += off2 * (bo + to);
+            body(c, y, z0, pre(c));
+        }
+    }
+    template <int U, class Body>
+    __device__ __forceinline__ void each(Body body) const {
+#pragma unroll U
+        for (int lc = threadIdx.x; lc < m; lc += blockDim.x) body(c0 + lc);
+    }
+};
+
+__global__ void __launch_bounds__(1024, 1) k_boxes(const BInst* __restrict__ insts, const int* __restrict__ order,
+                                                   int count, BVecs vs, BParams prm, BOut* __restrict__ out,
+                                                   unsigned* queue, int tile_cells) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ TeamShared sh;
+    __shared__ SolverState st_s;
+    __shared__ double sC[64], sinvd[64], tfold[6];
+    __shared__ int s_item;
+    SolverState* st = &st_s;
+    const int tid = threadIdx.x;
+    double* tile = reinterpret_cast<double*>(smem_raw);
+    unsigned char* faces = smem_raw + (size_t)tile_cells * sizeof(double);
+    ClusterTeam team = ClusterTeam::here(&sh);
+    for (;;) {
+        if (team.rank == 0 && tid == 0) {
+            const int next = (int)atomicAdd(queue, 1u);
+            for (int b = 0; b < team.size; b++)
+                asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(ClusterTeam::remote(&s_item, b)), "r"(next)
+                             : "memory");
+        }
+        team.barrier();
+        const int item = s_item;
+        if (item >= count) break;
+        const int id = order[item];
+        const BInst* __restrict__ Ip = insts + id;
+        const int n0 = Ip->n0, n1 = Ip->n1, n2 = Ip->n2;
+        BoxOp op;
+        op.sy = n2;
+        op.sx = n1 * n2;
+        const int N = n0 * op.sx;
+        op.off0 = Ip->offd[0];
+        op.off1 = Ip->offd[1];
+        op.off2 = Ip->offd[2];
+        op.C = sC;
+        op.invd = sinvd;
+        op.tile = tile;
+        op.faces = faces;
+        op.c0 = min(N, team.rank * Ip->chunk);
+        op.m = min(Ip->chunk, N - op.c0);
+        op.t0 = max(0, op.c0 - op.sx);
+        op.tn = op.m > 0 ? min(N, op.c0 + op.m + op.sx) - op.t0 : 0;
+        if (tid < 64) {
+            sC[tid] = Ip->C[tid];
+            sinvd[tid] = Ip->invd[tid];
+        }
+        if (tid < 6) tfold[tid] = Ip->tfold[tid];
+        if (tid == 0) {
+            SolverState z{};
+            z.tol = prm.tol;
+            z.max_it = prm.max_it;
+            z.tol_relative = prm.tol_relative;
+            *st = z;
+        }
+        for (int e = tid; e < op.tn; e += blockDim.x) {
+            const int g = op.t0 + e, i = g / op.sx, rem = g - i * op.sx, j = rem / n2, k = rem - j * n2;
+            faces[e] = (unsigned char)((i == 0) | (i == n0 - 1) << 1 | (j == 0) << 2 | (j == n1 - 1) << 3 |
+                                       (k == 0) << 4 | (k == n2 - 1) << 5);
+        }
+        __syncthreads();
+        const int64_t off = Ip->off;
+        const TeamVecs V{vs.x + off, vs.rh + off, vs.r + off, vs.u + off, vs.v + off, vs.s + off, vs.w + off, vs.t + off};
+        double* b = vs.b + off;
+        const double tt = Ip->tt;
+        // Build (b = tt phi_old, then the Dirichlet folds; phi_old = x is the
+        // initial guess, as the reference's Build copies the field into x),
+        // (0)-(2): r = b - Ahat y, r_hat_0 = r, u = 0
+        double a2[2] = {0., 0.};
+        op.pass([&](int e) { return V.x[e]; }, [&](int c) { return V.x[c]; },
+                [&](int c, double y, double, double xc) {
+                    const unsigned f = faces[c - op.t0];
+                    double bc = tt * xc;
+#pragma unroll
+                    for (int q = 0; q < 6; q++)
+                        if (f >> q & 1u) bc -= tfold[q];
+                    b[c] = bc;
+                    const double rr = bc - y;
+                    V.r[c] = rr;
+                    V.rh[c] = rr;
+                    V.u[c] = 0.;
+                    a2[0] += rr * rr;
+                    a2[1] += bc * bc;
+                });
+        team.sum<2>(a2, [&](const double* t) { finish_init(st, t); });
+        team_iterations(team, op, V, st);
+        // the exit: step (10) when the solve stopped between it and the last
+        // pass, x = M^-1 y
+        const bool pend = step10_pending_state(st->status, st->step);
+        const double alpha1 = st->alpha1, beta5 = st->beta5;
+        op.each<1>([&](int c) {
+            double xc = V.x[c];
+            if (pend) {
+                const double u5 = V.r[c] - beta5 * V.u[c];
+                xc = alpha1 * u5 + xc;
+            }
+            V.x[c] = sinvd[faces[c - op.t0]] * xc;
+        });
+        if (st->status == ST_TAU0) {
+            // BiCGStab2.inl:407-424: true residual; on failure M^-1 once more
+            team.barrier();
+            double a1[1] = {0.};
+            // (the tile holds x / C here: its rows are those of A x after the
+            // scaling is undone by the operand C x)
+            op.pass([&](int e) { return sC[faces[e - op.t0]] * V.x[e]; }, [&](int c) { return b[c]; },
+                    [&](int, double y, double, double bc) {
+                        const double rr = bc - y;
+                        a1[0] += rr * rr;
+                    });
+            team.sum<1>(a1, [&](const double* t) {
+                st->rnorm = sqrt(t[0]);
+                st->status = st->rnorm <= st->tol ? ST_CONVERGED : ST_BREAKDOWN;
+                if (st->status == ST_CONVERGED) st->step = 0;
+            });
+            if (st->status == ST_BREAKDOWN)
+                op.each<1>([&](int c) { V.x[c] = sinvd[faces[c - op.t0]] * V.x[c]; });
+        }
+        if (team.rank == 0 && tid == 0) {
+            BOut o{};
+            o.iters = st->k;
+            o.converged = st->rnorm <= st->tol;
+            o.status = st->status;
+            o.step = st->step;
+            o.res_abs = st->rnorm;
+            o.b_norm = sqrt(st->bnorm2);
+            o.tol_abs = st->tol;
+            out[id] = o;
+        }
+        __syncthreads();   // the next box's state, masks and tile replace these
+    }
+}
+
 // size classes of the cells-per-thread table: <=16, <=24, <=32, <=48, <=64, <=96, <=128, larger
 int size_class(int n) {
     static const int edges[7] = {16, 24, 32, 48, 64, 96, 128};
@@ -468,6 +656,106 @@ static int fill_instance(const dare_batch_instance& in, BInst& I) {
     return DARE_OK;
 }
 
+// A block's cells and tile (with the plane before and after) in a cluster of
+// `blocks` blocks
+static int64_t box_chunk(int64_t cells, int blocks) { return ((cells + blocks - 1) / blocks + 31) / 32 * 32; }
+static int64_t box_tile(int64_t cells, int64_t plane, int64_t chunk) { return std::min(cells, chunk + 2 * plane); }
+constexpr size_t kBoxSmem = 220 * 1024;   // beside the kernel's static shared memory
+static size_t box_smem(int64_t tile) { return (size_t)(tile + 15) / 16 * 16 * (sizeof(double) + 1); }
+
+// The cluster size of every box: as few blocks as leave each at most 4096 x
+// vec cells (vec = 1, 2 or 4 by size class, tuned): fewer cells and the
+// exchanges show, more and the box's eight vectors times the boxes in flight
+// leave L2.  Batches too small to fill the device take larger clusters, down
+// to a block of 512 cells.
+static int upload_instances(dare_batch* bt) {
+    dare_ctx* ctx = bt->ctx;
+    std::vector<int> cls(bt->count);
+    for (int grow = 0;; grow++) {
+        int64_t blocks = 0;
+        bool more = false;
+        for (int q = 0; q < bt->count; q++) {
+            BInst& I = bt->host[q];
+            const int64_t cells = (int64_t)I.n0 * I.n1 * I.n2, plane = (int64_t)I.n1 * I.n2;
+            I.vec = bt->vec_by_size[size_class(std::max(I.n0, std::max(I.n1, I.n2)))];
+            int c = 0;
+            while (c < kBoxClasses - 1 && cells > ((int64_t)4096 * I.vec << c)) c++;
+            while (c < kBoxClasses && box_smem(box_tile(cells, plane, box_chunk(cells, 1 << c))) > kBoxSmem) c++;
+            if (c < kBoxClasses)
+                for (int k = 0; k < grow && c < kBoxClasses - 1 && cells >= (int64_t)1024 << c; k++) c++;
+            if (c < kBoxClasses - 1 && cells >= (int64_t)1024 << c) more = true;
+            cls[q] = c;
+            I.chunk = c < kBoxClasses ? (int)box_chunk(cells, 1 << c) : 0;
+            blocks += c < kBoxClasses ? 1 << c : 1;
+        }
+        if (!more || blocks > ctx->num_sms / 2) break;
+    }
+    std::vector<int> order;
+    order.reserve(bt->count);
+    for (int c = 0; c <= kBoxClasses; c++) {
+        bt->class_at[c] = (int)order.size();
+        size_t smem = 0;
+        for (int id : bt->order)
+            if (cls[id] == c) {
+                const BInst& I = bt->host[id];
+                order.push_back(id);
+                if (c < kBoxClasses)
+                    smem = std::max(smem, box_smem(box_tile((int64_t)I.n0 * I.n1 * I.n2, (int64_t)I.n1 * I.n2, I.chunk)));
+            }
+        if (c < kBoxClasses) bt->class_smem[c] = smem;
+    }
+    bt->class_at[kBoxClasses + 1] = (int)order.size();
+    bt->clusters_block = 0;
+    DARE_CUDA(ctx, cudaMemcpyAsync(bt->d_order, order.data(), sizeof(int) * bt->count, cudaMemcpyHostToDevice,
+                                   ctx->stream));
+    DARE_CUDA(ctx, cudaMemcpyAsync(bt->d_inst, bt->host.data(), sizeof(BInst) * bt->count, cudaMemcpyHostToDevice,
+                                   ctx->stream));
+    DARE_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    return DARE_OK;
+}
+
+static int launch_class(dare_batch* bt, int c, const BVecs& vs, const BParams& prm, int block, cudaStream_t sm) {
+    dare_ctx* ctx = bt->ctx;
+    const int first = bt->class_at[c], count = bt->class_at[c + 1] - first;
+    if (c == kBoxClasses) {
+        int per_sm = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batched, block, 0);
+        const int blocks = std::min(std::max(per_sm, 1) * ctx->num_sms, count);
+        k_batched<<<blocks, block, 0, sm>>>(bt->d_inst, bt->d_order + first, count, vs, prm, bt->d_out,
+                                            bt->d_queue + c);
+        DARE_LAUNCHED(ctx);
+        return DARE_OK;
+    }
+    const size_t smem = bt->class_smem[c];
+    DARE_CUDA(ctx, cudaFuncSetAttribute(k_boxes, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBoxSmem));
+    DARE_CUDA(ctx, cudaFuncSetAttribute(k_boxes, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = 1u << c;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = sm;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cfg.gridDim = dim3(ctx->num_sms / (1 << c) * (1 << c));
+    if (bt->clusters_block != block) {
+        std::fill(bt->class_clusters, bt->class_clusters + kBoxClasses, 0);
+        bt->clusters_block = block;
+    }
+    int& clusters = bt->class_clusters[c];
+    if (!clusters) DARE_CUDA(ctx, cudaOccupancyMaxActiveClusters(&clusters, k_boxes, &cfg));
+    if (clusters < 1) return set_error(ctx, DARE_ERR_UNSUPPORTED, "dare_batch: a cluster does not fit the device");
+    cfg.gridDim = dim3((unsigned)std::min(clusters, count) << c);
+    DARE_CUDA(ctx, cudaLaunchKernelEx(&cfg, k_boxes, (const BInst*)bt->d_inst, (const int*)(bt->d_order + first), count,
+                                      vs, prm, bt->d_out, bt->d_queue + c, (int)(smem / (sizeof(double) + 1))));
+    DARE_LAUNCHED(ctx);
+    return DARE_OK;
+}
+
+// All classes at the same time: the largest clusters on the context's stream,
+// the others on the batch's own between two events.
 static int launch_batch(dare_batch* bt, const dare_solver_params* p, int block) {
     dare_ctx* ctx = bt->ctx;
     BVecs vs;
@@ -483,28 +771,24 @@ static int launch_batch(dare_batch* bt, const dare_solver_params* p, int block) 
     vs.w = base + 7 * T;
     vs.t = base + 8 * T;
     BParams prm{p->tol, p->max_it, p->tol_relative};
-    DARE_CUDA(ctx, cudaMemsetAsync(bt->d_queue, 0, sizeof(unsigned), ctx->stream));
-    int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batched, block, 0);
-    if (per_sm < 1) per_sm = 1;
-    int blocks = per_sm * ctx->num_sms;
-    if (blocks > bt->count) blocks = bt->count;
-    k_batched<<<blocks, block, 0, ctx->stream>>>(bt->d_inst, bt->d_order, bt->count, vs, prm, bt->d_out,
-                                                 bt->d_queue);
-    DARE_LAUNCHED(ctx);
-    return DARE_OK;
-}
-
-static int upload_instances(dare_batch* bt) {
-    dare_ctx* ctx = bt->ctx;
-    for (auto& I : bt->host) {
-        const int cls = size_class(std::max(I.n0, std::max(I.n1, I.n2)));
-        I.vec = bt->vec_by_size[cls];
+    DARE_CUDA(ctx, cudaMemsetAsync(bt->d_queue, 0, (kBoxClasses + 1) * sizeof(unsigned), ctx->stream));
+    bool used[kBoxClasses + 1];
+    int main_class = -1, nused = 0;
+    for (int c = kBoxClasses; c >= 0; c--) {
+        used[c] = bt->class_at[c + 1] > bt->class_at[c];
+        if (used[c] && main_class < 0) main_class = c;
+        nused += used[c];
     }
-    DARE_CUDA(ctx, cudaMemcpyAsync(bt->d_inst, bt->host.data(), sizeof(BInst) * bt->count, cudaMemcpyHostToDevice,
-                                   ctx->stream));
-    DARE_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    return DARE_OK;
+    if (nused > 1) DARE_CUDA(ctx, cudaEventRecord(bt->fork, ctx->stream));
+    int rc = launch_class(bt, main_class, vs, prm, block, ctx->stream);
+    for (int c = main_class - 1; c >= 0 && rc == DARE_OK; c--) {
+        if (!used[c]) continue;
+        DARE_CUDA(ctx, cudaStreamWaitEvent(bt->side[c], bt->fork, 0));
+        rc = launch_class(bt, c, vs, prm, block, bt->side[c]);
+        DARE_CUDA(ctx, cudaEventRecord(bt->join[c], bt->side[c]));
+        DARE_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, bt->join[c], 0));
+    }
+    return rc;
 }
 
 }  // namespace dare_gpu
@@ -546,11 +830,14 @@ int dare_batch_create(dare_ctx* ctx, int count, const dare_batch_instance* inst,
     cudaError_t e = cudaMalloc(&bt->d_inst, sizeof(BInst) * count);
     if (e == cudaSuccess) e = cudaMalloc(&bt->d_order, sizeof(int) * count);
     if (e == cudaSuccess) e = cudaMalloc(&bt->d_out, sizeof(BOut) * count);
-    if (e == cudaSuccess) e = cudaMalloc(&bt->d_queue, sizeof(unsigned));
+    if (e == cudaSuccess) e = cudaMalloc(&bt->d_queue, (kBoxClasses + 1) * sizeof(unsigned));
+    for (int c = 0; c < kBoxClasses; c++) {
+        if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&bt->side[c], cudaStreamNonBlocking);
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&bt->join[c], cudaEventDisableTiming);
+    }
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&bt->fork, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaMalloc(&bt->arena, sizeof(double) * 9 * (size_t)bt->total);
     if (e == cudaSuccess) e = cudaMemsetAsync(bt->arena, 0, sizeof(double) * (size_t)bt->total, ctx->stream);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(bt->d_order, bt->order.data(), sizeof(int) * count, cudaMemcpyHostToDevice, ctx->stream);
     if (e != cudaSuccess) {
         dare_batch_destroy(bt);
         return check_cuda(ctx, e, "dare_batch_create");
@@ -572,6 +859,11 @@ int dare_batch_destroy(dare_batch* bt) {
     cudaFree(bt->d_out);
     cudaFree(bt->d_queue);
     cudaFree(bt->arena);
+    for (auto& q : bt->side)
+        if (q) cudaStreamDestroy(q);
+    for (auto& q : bt->join)
+        if (q) cudaEventDestroy(q);
+    if (bt->fork) cudaEventDestroy(bt->fork);
     delete bt;
     return DARE_OK;
 }
