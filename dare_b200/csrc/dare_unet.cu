@@ -50,108 +50,18 @@ constexpr size_t kMaxSmem = 232448;  // 227 KB of opt-in shared memory per CTA
 // flattened position Q0, as C/8 planes of 16-byte chunks with row pitch RP
 // (chunk (kc, q) at byte (kc * RP + q) * 16).  Positions outside the array
 // and rows q >= valid_rows read zero.
-// IN_EMBED (C == 16) takes an FP32 vector over the internal cells as channel
-// 0 (rounded to bf16) and zero elsewhere: the slot's other channels are
-// zeroed once per kernel (stage_zero), the FP32 values land asynchronously
-// in a raw 4-byte-per-row buffer, and stage_finish (run by the issuing
-// thread after its cp.async wait) writes the bf16 channel-0 values.
-// FP32 channel-0 rows q = first, first + stride, ... of a plane segment into
-// the raw buffer.  The padded coordinates of a row are stepped from the
-// previous one (one division per call, not per row).
-__device__ __forceinline__ void embed_rows(float* raw, const float* __restrict__ in32, const Geom& g, int64_t Q0,
-                                           int rows, int valid_rows, int first, int stride) {
-    const int Jn = g.n1 + 2;
-    int64_t Q = Q0 + first;
-    int I = 0, J = 0, K = 0;
-    bool have = false;
-    for (int q = first; q < rows; q += stride, Q += stride) {
-        if (!have && Q >= 0) {
-            I = (int)(Q / g.plane);
-            const int rem = (int)(Q - (int64_t)I * g.plane);
-            J = rem / g.W;
-            K = rem - J * g.W;
-            have = true;
-        }
-        const bool ok = have && Q < g.total && q < valid_rows && I >= 1 && I <= g.n0 && J >= 1 && J <= g.n1 &&
-                        K >= 1 && K <= g.n2;
-        if (ok)
-            cp4(raw + q, in32 + ((int64_t)(I - 1) * g.n1 + (J - 1)) * g.n2 + (K - 1));
-        else
-            raw[q] = 0.f;
-        if (have) {
-            K += stride;
-            while (K >= g.W) {
-                K -= g.W;
-                if (++J == Jn) {
-                    J = 0;
-                    ++I;
-                }
-            }
-        }
+template <int C>
+__device__ __forceinline__ void stage(uint8_t* slot, const bf16* __restrict__ in, const Geom& g, int64_t Q0, int rows,
+                                      int RP, int valid_rows) {
+    constexpr int KC = C / 8;
+    const int nent = rows * KC;
+    for (int idx = threadIdx.x; idx < nent; idx += kThreads) {
+        const int q = idx / KC, kc = idx - q * KC;
+        const int64_t Q = Q0 + q;
+        const bool v = Q >= 0 && Q < g.total && q < valid_rows;
+        cp16(slot + ((size_t)kc * RP + q) * 16, in + act_off(g.total, v ? Q : 0, kc), v);
     }
 }
-
-template <int C, int MODE>
-__device__ __forceinline__ void stage(uint8_t* slot, float* raw, const bf16* __restrict__ in,
-                                      const float* __restrict__ in32, const Geom& g, int64_t Q0, int rows, int RP,
-                                      int valid_rows) {
-    if (MODE == IN_BF16) {
-        constexpr int KC = C / 8;
-        const int nent = rows * KC;
-        for (int idx = threadIdx.x; idx < nent; idx += kThreads) {
-            const int q = idx / KC, kc = idx - q * KC;
-            const int64_t Q = Q0 + q;
-            const bool v = Q >= 0 && Q < g.total && q < valid_rows;
-            cp16(slot + ((size_t)kc * RP + q) * 16, in + act_off(g.total, v ? Q : 0, kc), v);
-        }
-    } else {
-        embed_rows(raw, in32, g, Q0, rows, valid_rows, threadIdx.x, kThreads);
-    }
-}
-
-template <int MODE>
-__device__ __forceinline__ void stage_finish(uint8_t* slot, const float* raw, int rows) {
-    if (MODE == IN_EMBED) {
-        for (int q = threadIdx.x; q < rows; q += kThreads)
-            *reinterpret_cast<bf16*>(slot + (size_t)q * 16) = __float2bfloat16_rn(raw[q]);
-    }
-}
-
-__device__ __forceinline__ void stage_zero(uint8_t* p, uint32_t bytes, int nthreads = kThreads) {
-    for (uint32_t o = threadIdx.x * 16; o < bytes; o += nthreads * 16)
-        *reinterpret_cast<uint4*>(p + o) = make_uint4(0u, 0u, 0u, 0u);
-}
-
-// The same staging done by one warp (lane-strided), for the producer warp of
-// the warp-specialised forward kernel.
-template <int C, int MODE>
-__device__ __forceinline__ void stage_lanes(uint8_t* slot, float* raw, const bf16* __restrict__ in,
-                                            const float* __restrict__ in32, const Geom& g, int64_t Q0, int rows,
-                                            int RP, int lane) {
-    if (MODE == IN_BF16) {
-        constexpr int KC = C / 8;
-        const int nent = rows * KC;
-        for (int idx = lane; idx < nent; idx += 32) {
-            const int q = idx / KC, kc = idx - q * KC;
-            const int64_t Q = Q0 + q;
-            const bool v = Q >= 0 && Q < g.total;
-            cp16(slot + ((size_t)kc * RP + q) * 16, in + act_off(g.total, v ? Q : 0, kc), v);
-        }
-    } else {
-        embed_rows(raw, in32, g, Q0, rows, rows, lane, 32);
-    }
-}
-
-template <int MODE>
-__device__ __forceinline__ void stage_finish_lanes(uint8_t* slot, const float* raw, int rows, int lane) {
-    if (MODE == IN_EMBED) {
-        for (int q = lane; q < rows; q += 32)
-            *reinterpret_cast<bf16*>(slot + (size_t)q * 16) = __float2bfloat16_rn(raw[q]);
-    }
-}
-
-// raw FP32 staging bytes of one slot (IN_EMBED), 16-byte aligned
-__host__ __device__ inline uint32_t raw_bytes(int rows) { return (uint32_t)(((rows + 3) / 4) * 16); }
 
 // ---------------------------------------------------------------------------
 // forward convolution
@@ -1040,10 +950,8 @@ __global__ void __launch_bounds__(out_threads(MT)) k_conv_out(OutArgs a) {
 // weight gradient
 struct WgrArgs {
     Geom g;
-    const bf16* x;     // input activations (IN_BF16) ...
-    const float* x32;  // ... or the FP32 vector (IN_EMBED)
-    const bf16* dy;    // output gradient (IN_BF16) ...
-    const float* dy32; // ... or the FP32 vector (IN_EMBED)
+    const bf16* x;     // input activations
+    const bf16* dy;    // output gradient
     float* part;       // [cta][tpg][COUT][CIN]
     int ppc, tpg;
     uint32_t cols;
@@ -1056,7 +964,7 @@ __host__ __device__ constexpr int dy_pitch() {
     return kTileM + (C == 16 ? 4 : (C == 32 ? 2 : 1));
 }
 
-template <int CIN, int COUT, int XM, int YM>
+template <int CIN, int COUT>
 __global__ void __launch_bounds__(kThreads) k_conv_wgrad(WgrArgs a) {
     extern __shared__ __align__(1024) uint8_t smem[];
     constexpr int KCX = CIN / 8, KCY = COUT / 8;
@@ -1067,13 +975,9 @@ __global__ void __launch_bounds__(kThreads) k_conv_wgrad(WgrArgs a) {
     const int rows = stage_rows(g);
     const int RP = row_pitch(rows, CIN);
     const uint32_t SB = (uint32_t)KCX * RP * 16;
-    const uint32_t RBX = XM == IN_EMBED ? raw_bytes(rows) : 0u;
-    const uint32_t RBY = YM == IN_EMBED ? raw_bytes(kTileM) : 0u;
     uint8_t* dys = smem;
     uint8_t* xs = smem + 2 * DB;
-    float* xraw = reinterpret_cast<float*>(xs + 4 * SB);
-    float* yraw = reinterpret_cast<float*>(xs + 4 * SB + 4 * RBX);
-    uint64_t* mbar = reinterpret_cast<uint64_t*>(xs + 4 * SB + 4 * RBX + 2 * RBY);
+    uint64_t* mbar = reinterpret_cast<uint64_t*>(xs + 4 * SB);
     uint32_t* tslot = reinterpret_cast<uint32_t*>(mbar + 2);
 
     const int P0 = blockIdx.x * kTileM;
@@ -1087,8 +991,6 @@ __global__ void __launch_bounds__(kThreads) k_conv_wgrad(WgrArgs a) {
         mbar_init(&mbar[1], 1);
         mbar_fence_init();
     }
-    if (XM == IN_EMBED) stage_zero(xs, 4 * SB);
-    if (YM == IN_EMBED) stage_zero(dys, 2 * DB);
     if (tid < 32) tmem_alloc(tslot, a.cols);
     fence_before_sync();
     __syncthreads();
@@ -1097,14 +999,12 @@ __global__ void __launch_bounds__(kThreads) k_conv_wgrad(WgrArgs a) {
 
     const int64_t pbase = (int64_t)P0 - g.W - 1;
     for (int I = I0 - 1; I <= I0 + 1; I++)
-        stage<CIN, XM>(xs + (I & 3) * SB, xraw + (I & 3) * (RBX / 4), a.x, a.x32, g, (int64_t)I * g.plane + pbase,
-                       rows, RP, rows);
+        stage<CIN>(xs + (I & 3) * SB, a.x, g, (int64_t)I * g.plane + pbase, rows, RP, rows);
     // dY only at the tile's positions inside this plane: on coarse levels a
     // 128-position tile runs past the plane's end into the next plane's rows,
     // which that plane's own pass counts
     const int yrows = min(kTileM, g.plane - P0);
-    stage<COUT, YM>(dys + (I0 & 1) * DB, yraw + (I0 & 1) * (RBY / 4), a.dy, a.dy32, g, (int64_t)I0 * g.plane + P0,
-                    kTileM, RPD, yrows);
+    stage<COUT>(dys + (I0 & 1) * DB, a.dy, g, (int64_t)I0 * g.plane + P0, kTileM, RPD, yrows);
     cp_commit();
 
     constexpr uint32_t idesc = idesc_bf16(kTileM, CIN, 1, 1);
@@ -1113,9 +1013,6 @@ __global__ void __launch_bounds__(kThreads) k_conv_wgrad(WgrArgs a) {
     for (int I = I0; I <= I1; I++) {
         const int buf = (I - I0) & 1;
         cp_wait_all();
-        for (int p = (I == I0 ? I0 - 1 : I + 1); p <= I + 1; p++)
-            stage_finish<XM>(xs + (p & 3) * SB, xraw + (p & 3) * (RBX / 4), rows);
-        stage_finish<YM>(dys + (I & 1) * DB, yraw + (I & 1) * (RBY / 4), kTileM);
         fence_proxy_async();
         __syncthreads();
         if (tid == 0) {
@@ -1143,11 +1040,9 @@ __global__ void __launch_bounds__(kThreads) k_conv_wgrad(WgrArgs a) {
             }
         }
         if (I + 2 <= I1 + 1)
-            stage<CIN, XM>(xs + ((I + 2) & 3) * SB, xraw + ((I + 2) & 3) * (RBX / 4), a.x, a.x32, g,
-                           (int64_t)(I + 2) * g.plane + pbase, rows, RP, rows);
+            stage<CIN>(xs + ((I + 2) & 3) * SB, a.x, g, (int64_t)(I + 2) * g.plane + pbase, rows, RP, rows);
         if (I + 1 <= I1)
-            stage<COUT, YM>(dys + ((I + 1) & 1) * DB, yraw + ((I + 1) & 1) * (RBY / 4), a.dy, a.dy32, g,
-                            (int64_t)(I + 1) * g.plane + P0, kTileM, RPD, yrows);
+            stage<COUT>(dys + ((I + 1) & 1) * DB, a.dy, g, (int64_t)(I + 1) * g.plane + P0, kTileM, RPD, yrows);
         cp_commit();
     }
     if (!aborted) {
@@ -1189,18 +1084,140 @@ __global__ void __launch_bounds__(kThreads) k_conv_wgrad(WgrArgs a) {
     }
 }
 
-// grad[t][co][ci] += scale * sum over the CTAs of tap group t / tpg (fixed order)
-__global__ void k_wgrad_reduce(const float* __restrict__ part, int nxy, int tpg, int CINK, int COUTK, int cin,
-                               int cout, float scale, float* __restrict__ grad) {
-    const int total = kTaps * cout * cin;
-    const size_t ps = (size_t)tpg * COUTK * CINK;
-    for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += gridDim.x * blockDim.x) {
+// grad[t][co][ci] += scale * sum over the CTAs of tap group t / tpg (fixed
+// order).  Threads x take consecutive values, threads y parts of the CTAs, about
+// eight each: one thread a value left the 432-value layers with two blocks
+// that each read 560 partials in turn (47 us; 4 now).
+constexpr int kRedThreads = 256;
+__global__ void __launch_bounds__(kRedThreads) k_wgrad_reduce(const float* __restrict__ part, int nxy, int tpg,
+                                                             int CINK, int COUTK, int cin, int cout, float scale,
+                                                             float* __restrict__ grad) {
+    __shared__ double sh[kRedThreads];
+    const int nx = blockDim.x, ny = blockDim.y;
+    const int idx = blockIdx.x * nx + threadIdx.x;
+    const bool inside = idx < kTaps * cout * cin;
+    double s = 0.;
+    if (inside) {
+        const size_t ps = (size_t)tpg * COUTK * CINK;
         const int ci = idx % cin, co = (idx / cin) % cout, t = idx / (cin * cout);
         const int z = t / tpg, tl = t - z * tpg;
         const float* p = part + (size_t)z * nxy * ps + ((size_t)tl * COUTK + co) * CINK + ci;
-        double s = 0.;
-        for (int b = 0; b < nxy; b++) s += (double)p[(size_t)b * ps];
-        grad[idx] += scale * (float)s;
+#pragma unroll 4
+        for (int b = threadIdx.y; b < nxy; b += ny) s += (double)p[(size_t)b * ps];
+    }
+    if (ny > 1) {
+        sh[threadIdx.y * nx + threadIdx.x] = s;
+        __syncthreads();
+        if (threadIdx.y > 0) return;
+        for (int y = 1; y < ny; y++) s += sh[y * nx + threadIdx.x];
+    }
+    if (inside) grad[idx] += scale * (float)s;
+}
+
+// Weight gradient of the two layers with one channel on a side (enc0, dec0):
+// D[c][t] = sum_q A[q][c] v[q + sign d_t], A the 16-channel side (dY of enc0, the
+// input of dec0) and v the FP32 vector (the input, dz), rounded to bf16.
+// 432 numbers: as an MMA with M = 128 and one N = 16 block a tap (k_conv_wgrad)
+// 7/8 of the rows and 15/16 of the channels were padding, 100-110 us at 64^3.
+// Here the channels are M = 16 and the taps N = 27 of 32 of warp-level MMAs
+// over K = 16 positions, which leaves reading A (8.4 MB at 64^3) as the bound:
+// 8 us.  A position is a flattened padded position of one plane: A is zero at
+// ghosts, so no position needs a mask.
+struct Wgr1Args {
+    Geom g;
+    const bf16* a;
+    const float* v;
+    float* part;   // [cta][tap][16]
+    int sign, ppc;
+};
+constexpr int kWgr1Seg = 1024;     // positions of a plane a CTA stages at a time
+constexpr int kWgr1Warps = 8;
+__host__ __device__ inline int wgr1_vlen(const Geom& g) { return (kWgr1Seg + 2 * g.W + 2 + 7) / 8 * 8; }
+inline size_t wgr1_smem(const Geom& g) { return (size_t)2 * kWgr1Seg * 16 + (size_t)2 * 3 * wgr1_vlen(g) * sizeof(bf16); }
+
+__global__ void __launch_bounds__(kWgr1Warps * 32) k_wgrad_1ch(Wgr1Args a) {
+    extern __shared__ __align__(1024) uint8_t smem[];
+    const Geom g = a.g;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int VL = wgr1_vlen(g);
+    uint8_t* as = smem;                                              // [chunk][position][8 channels]
+    bf16* ve = reinterpret_cast<bf16*>(smem + 2 * kWgr1Seg * 16);    // [plane][VL] ...
+    bf16* vo = ve + 3 * VL;                                          // ... and the same one position on: odd
+                                                                     // offsets are 4-byte aligned there
+    const int P0 = blockIdx.x * kWgr1Seg, L = min(kWgr1Seg, g.plane - P0);
+    const int I0 = 1 + blockIdx.y * a.ppc, I1 = min(g.n0, I0 + a.ppc - 1);
+    // this thread's columns of B: tap 8 nb + lane / 4 (taps past 26 repeat the last; they are not stored)
+    const uint32_t* bsrc[4];
+#pragma unroll
+    for (int nb = 0; nb < 4; nb++) {
+        const int t = min(kTaps - 1, 8 * nb + (lane >> 2));
+        const int di = a.sign * (t / 9 - 1), dj = a.sign * ((t / 3) % 3 - 1), dk = a.sign * (t % 3 - 1);
+        const int off = (dj + 1) * g.W + dk + 1;
+        const bf16* base = off & 1 ? vo + (di + 1) * VL + off - 1 : ve + (di + 1) * VL + off;
+        bsrc[nb] = reinterpret_cast<const uint32_t*>(base + 2 * (lane & 3));
+    }
+    float d[4][4];
+#pragma unroll
+    for (int nb = 0; nb < 4; nb++)
+#pragma unroll
+        for (int r = 0; r < 4; r++) d[nb][r] = 0.f;
+    // ldmatrix rows: matrix lane / 8 is (chunk lane / 8 & 1, positions 8 (lane / 16) ..)
+    const uint32_t arow = smem_u32(as) + (uint32_t)(((lane >> 3) & 1) * kWgr1Seg + (lane >> 4) * 8 + (lane & 7)) * 16;
+
+    for (int I = I0; I <= I1; I++) {
+        __syncthreads();   // the last plane's tiles are read
+        for (int e = tid; e < 2 * kWgr1Seg; e += blockDim.x) {
+            const int kc = e / kWgr1Seg, q = e - kc * kWgr1Seg;
+            cp16(as + (size_t)e * 16, a.a + act_off(g.total, (int64_t)I * g.plane + P0 + (q < L ? q : 0), kc), q < L);
+        }
+        cp_commit();
+        for (int e = tid; e < 3 * VL; e += blockDim.x) {
+            const int pl = e / VL, x = e - pl * VL, Q = P0 - g.W - 1 + x, i = I - 1 + pl;
+            float v = 0.f;
+            if (Q >= 0 && Q < g.plane) {
+                const int J = Q / g.W, K = Q - J * g.W;
+                if (i >= 1 && i <= g.n0 && J >= 1 && J <= g.n1 && K >= 1 && K <= g.n2)
+                    v = a.v[((int64_t)(i - 1) * g.n1 + (J - 1)) * g.n2 + (K - 1)];
+            }
+            const bf16 b = __float2bfloat16_rn(v);
+            ve[e] = b;
+            if (x > 0) vo[e - 1] = b;
+            if (x == VL - 1) vo[e] = __float2bfloat16_rn(0.f);
+        }
+        cp_wait_all();
+        __syncthreads();
+        for (int k0 = warp * 16; k0 < L; k0 += kWgr1Warps * 16) {
+            uint32_t af[4];
+            asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                         : "=r"(af[0]), "=r"(af[1]), "=r"(af[2]), "=r"(af[3])
+                         : "r"(arow + (uint32_t)k0 * 16));
+#pragma unroll
+            for (int nb = 0; nb < 4; nb++) {
+                const uint32_t b0 = bsrc[nb][k0 / 2], b1 = bsrc[nb][k0 / 2 + 4];
+                asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, "
+                             "{%8, %9}, {%0, %1, %2, %3};"
+                             : "+f"(d[nb][0]), "+f"(d[nb][1]), "+f"(d[nb][2]), "+f"(d[nb][3])
+                             : "r"(af[0]), "r"(af[1]), "r"(af[2]), "r"(af[3]), "r"(b0), "r"(b1));
+            }
+        }
+    }
+    // the warps' sums, in warp order
+    __syncthreads();
+    float* sums = reinterpret_cast<float*>(smem);   // [warp][tap][16]
+#pragma unroll
+    for (int nb = 0; nb < 4; nb++)
+#pragma unroll
+        for (int r = 0; r < 4; r++) {
+            const int t = 8 * nb + 2 * (lane & 3) + (r & 1), c = (lane >> 2) + 8 * (r >> 1);
+            if (t < kTaps) sums[(warp * kTaps + t) * 16 + c] = d[nb][r];
+        }
+    __syncthreads();
+    float* out = a.part + ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * kTaps * 16;
+    for (int e = tid; e < kTaps * 16; e += blockDim.x) {
+        float s = sums[e];
+#pragma unroll
+        for (int w = 1; w < kWgr1Warps; w++) s += sums[w * kTaps * 16 + e];
+        out[e] = s;
     }
 }
 
@@ -1416,11 +1433,14 @@ __global__ void __launch_bounds__(256) k_make_pair(GridDev g, const double* __re
     }
 }
 
-__global__ void k_store_norm(const double* acc, float* out) { *out = (float)*acc; }
+__global__ void k_store_norm(const double* acc, float* out) { out[threadIdx.x] = (float)acc[threadIdx.x]; }
 
+// acc[y] += ||e[y]||^2 of the vectors y, n apart
 __global__ void __launch_bounds__(256) k_sqnorm(int64_t n, const float* __restrict__ e, double* __restrict__ acc) {
     __shared__ double sh[8];
     double s = 0.;
+    e += (int64_t)blockIdx.y * n;
+    acc += blockIdx.y;
     for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n; c += (int64_t)gridDim.x * blockDim.x)
         s += (double)e[c] * e[c];
     for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
@@ -1537,12 +1557,11 @@ static int pick_ppc(int n0, int64_t units, int64_t resident) {
 
 static int dy_pitch_rt(int c) { return kTileM + (c == 16 ? 4 : (c == 32 ? 2 : 1)); }
 
-static size_t wgr_smem(int cin, int cout, const Geom& g, bool xembed, bool yembed) {
+static size_t wgr_smem(int cin, int cout, const Geom& g) {
     const int rows = stage_rows(g);
     const int RP = row_pitch(rows, cin);
     const size_t DB = (size_t)(cout / 8) * dy_pitch_rt(cout) * 16;
-    const size_t body = 2 * DB + 4 * (size_t)(cin / 8) * RP * 16 + (xembed ? 4 * (size_t)raw_bytes(rows) : 0) +
-                        (yembed ? 2 * (size_t)raw_bytes(kTileM) : 0) + 32;
+    const size_t body = 2 * DB + 4 * (size_t)(cin / 8) * RP * 16 + 32;
     // the A operand (dY^T, 128 rows of which Cout are real) of the second dY
     // slot reaches 16 row groups past its start: keep that inside the CTA
     const size_t reach = DB + (size_t)(kTileM / 16) * 256 + 15 * (size_t)dy_pitch_rt(cout) * 16 + 256;
@@ -1627,11 +1646,11 @@ static int launch_fwd(dare_ctx* ctx, LaunchCfg& lc, int cin, int nt, int nz, int
     return set_error(ctx, DARE_ERR_UNSUPPORTED, "unet: no forward convolution kernel for this shape");
 }
 
-template <int CIN, int COUT, int XM, int YM>
+template <int CIN, int COUT>
 static int launch_wgr_t(dare_ctx* ctx, LaunchCfg& lc, WgrArgs a, size_t* part_need) {
-    auto kern = k_conv_wgrad<CIN, COUT, XM, YM>;
+    auto kern = k_conv_wgrad<CIN, COUT>;
     if (!lc.ready) {
-        size_t smem = wgr_smem(CIN, COUT, a.g, XM == IN_EMBED, YM == IN_EMBED);
+        size_t smem = wgr_smem(CIN, COUT, a.g);
         if (smem > kMaxSmem) return set_error(ctx, DARE_ERR_UNSUPPORTED, "unet: level too wide for the staged conv");
         const int tpg = std::min(kTaps, 256 / CIN);
         uint32_t cols = 32;
@@ -1662,19 +1681,37 @@ static int launch_wgr_t(dare_ctx* ctx, LaunchCfg& lc, WgrArgs a, size_t* part_ne
     return DARE_OK;
 }
 
-static int launch_wgr(dare_ctx* ctx, LaunchCfg& lc, int cin, int cout, int xm, int ym, const WgrArgs& a,
-                      size_t* part_need) {
-#define DARE_WGR(CI, CO, XM, YM) \
-    if (cin == CI && cout == CO && xm == XM && ym == YM) return launch_wgr_t<CI, CO, XM, YM>(ctx, lc, a, part_need);
-    DARE_WGR(16, 16, IN_EMBED, IN_BF16)
-    DARE_WGR(16, 32, IN_BF16, IN_BF16)
-    DARE_WGR(32, 64, IN_BF16, IN_BF16)
-    DARE_WGR(64, 64, IN_BF16, IN_BF16)
-    DARE_WGR(64, 32, IN_BF16, IN_BF16)
-    DARE_WGR(32, 16, IN_BF16, IN_BF16)
-    DARE_WGR(16, 16, IN_BF16, IN_EMBED)
+static int launch_wgr(dare_ctx* ctx, LaunchCfg& lc, int cin, int cout, const WgrArgs& a, size_t* part_need) {
+#define DARE_WGR(CI, CO) \
+    if (cin == CI && cout == CO) return launch_wgr_t<CI, CO>(ctx, lc, a, part_need);
+    DARE_WGR(16, 32)
+    DARE_WGR(32, 64)
+    DARE_WGR(64, 64)
+    DARE_WGR(64, 32)
+    DARE_WGR(32, 16)
 #undef DARE_WGR
     return set_error(ctx, DARE_ERR_UNSUPPORTED, "unet: no weight-gradient kernel for this shape");
+}
+
+// the one-channel layers: runs of planes for about four CTAs an SM
+static int launch_wgr1(dare_ctx* ctx, LaunchCfg& lc, Wgr1Args a, size_t* part_need) {
+    if (!lc.ready) {
+        const size_t smem = wgr1_smem(a.g);
+        DARE_CUDA(ctx, cudaFuncSetAttribute(k_wgrad_1ch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        const int segs = (a.g.plane + kWgr1Seg - 1) / kWgr1Seg;
+        lc.ppc = std::max(1, (int)((int64_t)a.g.n0 * segs / ((int64_t)ctx->num_sms * 4)));
+        lc.tpg = kTaps;
+        lc.occ = 4;
+        lc.grid = dim3(segs, (a.g.n0 + lc.ppc - 1) / lc.ppc, 1);
+        lc.smem = smem;
+        lc.ready = true;
+    }
+    *part_need = (size_t)lc.grid.x * lc.grid.y * kTaps * 16;
+    if (!a.part) return DARE_OK;  // sizing pass
+    a.ppc = lc.ppc;
+    k_wgrad_1ch<<<lc.grid, kWgr1Warps * 32, lc.smem, ctx->stream>>>(a);
+    DARE_LAUNCHED(ctx);
+    return DARE_OK;
 }
 
 // Ring depth (4..8 staged planes) of a plane-marching kernel: the deepest ring
@@ -1909,33 +1946,38 @@ static int conv_dgrad(dare_unet* net, int l, const bf16* dy, const float* dy32, 
     return launch_fwd(net->ctx, L.bwd, L.coutk, L.ntb, L.cink / L.ntb, OUT_STORE, a);
 }
 
+// (with `sizing` set: no launch, *sizing the floats its partial sums need)
 static int conv_wgrad(dare_unet* net, int l, const bf16* x, const float* x32, const bf16* dy, const float* dy32,
-                      float scale) {
+                      float scale, size_t* sizing = nullptr) {
     Layer& L = net->layer[l];
     dare_ctx* ctx = net->ctx;
+    const bool one = x32 || dy32;   // enc0, dec0
+    Wgr1Args a1{};
+    a1.g = net->geo[L.level];
+    a1.a = x32 ? dy : x;
+    a1.v = x32 ? x32 : dy32;
+    a1.sign = x32 ? 1 : -1;
     WgrArgs a{};
     a.g = net->geo[L.level];
     a.x = x;
-    a.x32 = x32;
     a.dy = dy;
-    a.dy32 = dy32;
     a.err = net->err;
+    const auto launch = [&](size_t* need) {
+        return one ? launch_wgr1(ctx, L.wgr, a1, need) : launch_wgr(ctx, L.wgr, L.cink, L.coutk, a, need);
+    };
+    if (sizing) return launch(sizing);   // the partial sums' room alone
     size_t need = 0;
-    int rc = launch_wgr(ctx, L.wgr, L.cink, L.coutk, x32 ? IN_EMBED : IN_BF16, dy32 ? IN_EMBED : IN_BF16, a, &need);
-    if (rc) return rc;
-    if (need > net->part_floats) {
-        cudaFree(net->part);
-        net->part = nullptr;
-        net->part_floats = 0;
-        DARE_CUDA(ctx, cudaMalloc(&net->part, need * sizeof(float)));
-        net->part_floats = need;
-    }
-    a.part = net->part;
-    if ((rc = launch_wgr(ctx, L.wgr, L.cink, L.coutk, x32 ? IN_EMBED : IN_BF16, dy32 ? IN_EMBED : IN_BF16, a, &need)))
-        return rc;
+    int rc;
+    a.part = a1.part = net->part;
+    if ((rc = launch(&need))) return rc;
+    // (the one-channel layers' partials are [tap][channel], as their gradient)
     const int nxy = (int)(L.wgr.grid.x * L.wgr.grid.y);
-    k_wgrad_reduce<<<eblocks(ctx, kTaps * L.cin * L.cout), 256, 0, ctx->stream>>>(
-        net->part, nxy, L.wgr.tpg, L.cink, L.coutk, L.cin, L.cout, scale, net->grad + L.woff);
+    int ny = 1;
+    while (ny < 32 && ny * 8 < nxy) ny *= 2;
+    const int nx = kRedThreads / ny;
+    k_wgrad_reduce<<<(kTaps * L.cin * L.cout + nx - 1) / nx, dim3(nx, ny), 0, ctx->stream>>>(
+        net->part, nxy, L.wgr.tpg, one ? L.cin : L.cink, one ? L.cout : L.coutk, L.cin, L.cout, scale,
+        net->grad + L.woff);
     DARE_LAUNCHED(ctx);
     return DARE_OK;
 }
@@ -2076,20 +2118,288 @@ static int check_err(dare_unet* net) {
     return DARE_OK;
 }
 
-// Mean loss and gradient over `count` pairs; grad is zeroed first.
+// The room for the weight gradients' partial sums, once for every layer
+static int ensure_part(dare_unet* net) {
+    if (net->part) return DARE_OK;
+    static const float one = 0.f;   // (marks an FP32 side; never read)
+    size_t most = 0;
+    for (int l = 0; l < kLayers; l++) {
+        size_t need = 0;
+        const int rc = conv_wgrad(net, l, nullptr, l == ENC0 ? &one : nullptr, nullptr, l == DEC0 ? &one : nullptr, 1.f,
+                                  &need);
+        if (rc) return rc;
+        most = std::max(most, need);
+    }
+    DARE_CUDA(net->ctx, cudaMalloc(&net->part, most * sizeof(float)));
+    net->part_floats = most;
+    return DARE_OK;
+}
+
+// The activations of a network in one zeroed allocation with room for
+// `extra` bytes after them (at *extra_at), every buffer 256-byte aligned
+static cudaError_t alloc_acts(dare_unet* net, size_t extra, uint8_t** extra_at, cudaStream_t stream) {
+    const int64_t T[4] = {net->geo[0].total, net->geo[1].total, net->geo[2].total, net->geo[3].total};
+    struct Slot {
+        bf16** p;
+        int level, c, extra;
+    } slots[] = {{&net->S0, 0, 16}, {&net->P1, 1, 16}, {&net->S1, 1, 32}, {&net->P2, 2, 32}, {&net->S2, 2, 64},
+                 {&net->P3, 3, 64}, {&net->E3, 3, 64}, {&net->dS0, 0, 16}, {&net->dD1, 1, 16}, {&net->dS1, 1, 32},
+                 {&net->dD2, 2, 32}, {&net->dS2, 2, 64}, {&net->dD3, 3, 64}, {&net->dE3, 3, 64}, {&net->dP3, 3, 64},
+                 {&net->dP2, 2, 32}, {&net->dP1, 1, 16}};
+    // a staged plane segment reaches up to W + 8 rows before the start of an
+    // array (the unused halo of the ghost plane 0) and kActSlackRows bounds W
+    size_t bytes = (size_t)kActSlackRows * 16;
+    std::vector<size_t> offs;
+    for (auto& s : slots) {
+        offs.push_back(bytes);
+        bytes += (((size_t)T[s.level] * s.c + s.extra) * sizeof(bf16) + 255) / 256 * 256;
+    }
+    bytes += (size_t)kActSlackRows * 16;  // rows a staged segment may read past the last array
+    net->act_block = nullptr;
+    cudaError_t e = cudaMalloc(&net->act_block, bytes + extra);
+    if (e == cudaSuccess) e = cudaMemsetAsync(net->act_block, 0, bytes, stream);
+    uint8_t* base = static_cast<uint8_t*>(net->act_block);
+    for (size_t i = 0; i < sizeof(slots) / sizeof(slots[0]) && e == cudaSuccess; i++)
+        *slots[i].p = reinterpret_cast<bf16*>(base + offs[i]);
+    if (extra_at) *extra_at = base + bytes;
+    return e;
+}
+
+}  // namespace unet
+}  // namespace dare_gpu
+
+// A lane: the network with buffers and a stream of its own (weights, error
+// word and everything else shared)
+struct dare_unet_lane {
+    dare_unet net;
+    dare_ctx ctx;
+    cudaEvent_t done = nullptr;
+};
+
+namespace dare_gpu {
+namespace unet {
+
+constexpr int kLanes = 4;
+// Lanes of a minibatch of `count` pairs.  A pair is a chain of ~42 kernels of
+// ~10 us that fill a fraction of the device on the coarse levels; above 128^3
+// they fill it.
+static int lanes_for(const dare_unet* net, int count) {
+    return net->ncell <= (int64_t)1 << 21 ? std::min(count, kLanes) : 1;
+}
+
+static void free_lane(dare_unet_lane* ln) {
+    if (!ln) return;
+    if (ln->done) cudaEventDestroy(ln->done);
+    if (ln->ctx.stream) cudaStreamDestroy(ln->ctx.stream);
+    cudaFree(ln->net.act_block);
+    cudaFree(ln->net.part);
+    delete ln;
+}
+
+static int ensure_lane(dare_unet* net, int l) {
+    dare_ctx* ctx = net->ctx;
+    if (!net->fork) DARE_CUDA(ctx, cudaEventCreateWithFlags(&net->fork, cudaEventDisableTiming));
+    if (net->lane[l]) return DARE_OK;
+    dare_unet_lane* ln = new (std::nothrow) dare_unet_lane();
+    if (!ln) return DARE_ERR_OOM;
+    ln->net = *net;
+    ln->ctx.device = ctx->device;
+    ln->ctx.num_sms = ctx->num_sms;
+    ln->net.ctx = &ln->ctx;
+    ln->net.part = nullptr;
+    ln->net.act_block = nullptr;
+    for (auto& o : ln->net.lane) o = nullptr;
+    const size_t vec = ((size_t)net->ncell * sizeof(float) + 255) / 256 * 256;
+    uint8_t* at = nullptr;
+    cudaError_t e = cudaStreamCreateWithFlags(&ln->ctx.stream, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ln->done, cudaEventDisableTiming);
+    if (e == cudaSuccess)
+        e = alloc_acts(&ln->net, 3 * vec + net->nparam * sizeof(float), &at, ln->ctx.stream);
+    if (e != cudaSuccess) {
+        free_lane(ln);
+        return check_cuda(ctx, e, "unet: training lane");
+    }
+    ln->net.z = reinterpret_cast<float*>(at);
+    ln->net.g = reinterpret_cast<float*>(at + vec);
+    ln->net.X0 = reinterpret_cast<float*>(at + 2 * vec);
+    ln->net.grad = reinterpret_cast<float*>(at + 3 * vec);
+    net->lane[l] = ln;
+    return DARE_OK;
+}
+
+// out = ((g[0] + g[1]) + ...), the lanes' gradients in the order of their first pairs
+struct LaneGrads {
+    const float* g[kLanes];
+    int n;
+};
+__global__ void __launch_bounds__(256) k_sum_grads(int64_t n, LaneGrads s, float* out) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        float a = s.g[0][i];
+        for (int l = 1; l < s.n; l++) a += s.g[l][i];
+        out[i] = a;
+    }
+}
+
+// Queues the loss (dscal[0]) and its mean gradient over `count` pairs; grad is
+// zeroed first.  Pair b runs on lane (count - 1 - b) mod lanes, so the last
+// pair's activations stay in the network's own buffers.
+static int queue_loss_grad(dare_unet* net, const float* const* r, const float* const* e, const float* const* en2,
+                           int count) {
+    dare_ctx* ctx = net->ctx;
+    int rc;
+    const int lanes = lanes_for(net, count);
+    if ((rc = ensure_part(net))) return rc;
+    DARE_CUDA(ctx, cudaMemsetAsync(net->grad, 0, net->nparam * sizeof(float), ctx->stream));
+    DARE_CUDA(ctx, cudaMemsetAsync(net->dscal, 0, sizeof(double), ctx->stream));
+    const float scale = 1.f / (float)count;
+    dare_unet* on[kLanes] = {net};
+    for (int l = 1; l < lanes; l++) {
+        if ((rc = ensure_lane(net, l))) return rc;
+        on[l] = &net->lane[l]->net;
+        on[l]->wait_limit = net->wait_limit;
+        on[l]->debug_skip = 0;
+        net->lane[l]->ctx.launches = 0;
+        if ((rc = ensure_part(on[l]))) return set_error(ctx, rc, on[l]->ctx->last_error);
+        if (l == 1) DARE_CUDA(ctx, cudaEventRecord(net->fork, ctx->stream));
+        cudaStream_t s = on[l]->ctx->stream;
+        DARE_CUDA(ctx, cudaStreamWaitEvent(s, net->fork, 0));
+        DARE_CUDA(ctx, cudaMemsetAsync(on[l]->grad, 0, net->nparam * sizeof(float), s));
+    }
+    rc = DARE_OK;
+    for (int b = 0; b < count && rc == DARE_OK; b++) {
+        dare_unet* ln = on[(count - 1 - b) % lanes];
+        dare_ctx* lc = ln->ctx;
+        if (b > 0 && b < lanes) {   // the launch configurations that the first pair's lane has found
+            const dare_unet* first = on[(count - 1) % lanes];
+            for (int l = 0; l < kLayers; l++) {
+                if (!ln->layer[l].fwd.ready) ln->layer[l].fwd = first->layer[l].fwd;
+                if (!ln->layer[l].bwd.ready) ln->layer[l].bwd = first->layer[l].bwd;
+            }
+        }
+        if ((rc = apply_grid(ln, r[b], ln->z)) == DARE_OK) {   // pairs live on the network's grid
+            k_loss_grad<<<eblocks(ctx, net->ncell), 256, 0, lc->stream>>>(net->ncell, ln->z, e[b], en2[b], scale, ln->g,
+                                                                          net->dscal);
+            lc->launches++;
+            const cudaError_t ce = cudaGetLastError();
+            rc = ce == cudaSuccess ? backward(ln, r[b], ln->g, 1.f) : check_cuda(ctx, ce, "kernel launch");
+        }
+        if (rc && lc != ctx) set_error(ctx, rc, lc->last_error);
+    }
+    // the lanes end before the context's stream goes on, after an error too
+    LaneGrads sum{};
+    for (int l = 1; l < lanes; l++) {
+        dare_unet_lane* ln = net->lane[l];
+        DARE_CUDA(ctx, cudaEventRecord(ln->done, ln->ctx.stream));
+        DARE_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, ln->done, 0));
+        ctx->launches += ln->ctx.launches;
+    }
+    if (rc) return rc;
+    if (lanes > 1) {
+        sum.n = lanes;
+        for (int b = 0; b < lanes; b++) sum.g[b] = on[(count - 1 - b) % lanes]->grad;
+        k_sum_grads<<<eblocks(ctx, net->nparam), 256, 0, ctx->stream>>>(net->nparam, sum, net->grad);
+        DARE_LAUNCHED(ctx);
+    }
+    return DARE_OK;
+}
+
+// The inputs of a minibatch into the graph's own buffers
+constexpr int kGraphPairs = 8;
+struct PairPtrs {
+    const float *r[kGraphPairs], *e[kGraphPairs], *en[kGraphPairs];
+};
+__global__ void __launch_bounds__(256) k_gather_pairs(int64_t n, int count, PairPtrs p, float* __restrict__ r,
+                                                      float* __restrict__ e, float* __restrict__ en) {
+    const float *rs = p.r[blockIdx.y], *es = p.e[blockIdx.y];
+    r += (int64_t)blockIdx.y * n;
+    e += (int64_t)blockIdx.y * n;
+    for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n; c += (int64_t)gridDim.x * blockDim.x) {
+        r[c] = rs[c];
+        e[c] = es[c];
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) en[blockIdx.y] = *p.en[blockIdx.y];
+}
+
+static void drop_loss_graph(dare_unet* net) {
+    if (net->lg_graph) cudaGraphExecDestroy(net->lg_graph);
+    net->lg_graph = nullptr;
+    net->lg_count = 0;
+}
+
+// The graph of a minibatch of `count` pairs: ~42 kernels a pair, most shorter
+// than the 4 us it takes to launch them one by one (4 pairs of 16^3: 680 us of
+// launches).  Captured on a stream of its own, so that the context's may be any.
+static int build_loss_graph(dare_unet* net, int count) {
+    dare_ctx* ctx = net->ctx;
+    const int64_t n = net->ncell;
+    drop_loss_graph(net);
+    if (net->lg_cap < count) {
+        cudaFree(net->lg_in);
+        net->lg_in = nullptr;
+        net->lg_cap = 0;
+        DARE_CUDA(ctx, cudaMalloc(&net->lg_in, ((size_t)2 * count * n + count) * sizeof(float)));
+        net->lg_cap = count;
+    }
+    float *r = net->lg_in, *e = r + (size_t)net->lg_cap * n, *en = e + (size_t)net->lg_cap * n;
+    std::vector<const float*> rp(count), ep(count), np(count);
+    for (int b = 0; b < count; b++) {
+        rp[b] = r + (size_t)b * n;
+        ep[b] = e + (size_t)b * n;
+        np[b] = en + b;
+    }
+    cudaStream_t cap, saved = ctx->stream;
+    DARE_CUDA(ctx, cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
+    const int64_t before = ctx->launches;
+    ctx->stream = cap;
+    cudaGraph_t graph = nullptr;
+    int rc = DARE_OK;
+    cudaError_t ce = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
+    if (ce == cudaSuccess) {
+        rc = queue_loss_grad(net, rp.data(), ep.data(), np.data(), count);
+        const cudaError_t c2 = cudaStreamEndCapture(cap, &graph);
+        if (ce == cudaSuccess) ce = c2;
+    }
+    ctx->stream = saved;
+    net->lg_launches = ctx->launches - before;
+    ctx->launches = before;
+    if (ce == cudaSuccess && rc == DARE_OK) ce = cudaGraphInstantiate(&net->lg_graph, graph, 0);
+    if (graph) cudaGraphDestroy(graph);
+    cudaStreamDestroy(cap);
+    if (rc) return rc;
+    if (ce != cudaSuccess) {
+        net->lg_graph = nullptr;
+        return check_cuda(ctx, ce, "unet: minibatch graph");
+    }
+    net->lg_count = count;
+    return DARE_OK;
+}
+
+// Mean loss and gradient (net->grad) over `count` pairs
 static int loss_grad(dare_unet* net, const float* const* r, const float* const* e, const float* const* en2, int count,
                      double* loss) {
     dare_ctx* ctx = net->ctx;
     int rc;
-    DARE_CUDA(ctx, cudaMemsetAsync(net->grad, 0, net->nparam * sizeof(float), ctx->stream));
-    DARE_CUDA(ctx, cudaMemsetAsync(net->dscal, 0, sizeof(double), ctx->stream));
-    const float scale = 1.f / (float)count;
-    for (int b = 0; b < count; b++) {
-        if ((rc = apply_grid(net, r[b], net->z))) return rc;   // pairs live on the network's grid
-        k_loss_grad<<<eblocks(ctx, net->ncell), 256, 0, ctx->stream>>>(net->ncell, net->z, e[b], en2[b], scale,
-                                                                       net->g, net->dscal);
+    // the graph from the second minibatch of a size on: the first sets the
+    // launch configurations and the buffers, and may be the only one
+    const bool replay = count <= kGraphPairs && net->lg_last == count && !net->debug_skip;
+    net->lg_last = count;
+    if (replay) {
+        if (net->lg_count != count && (rc = build_loss_graph(net, count))) return rc;
+        PairPtrs p{};
+        for (int b = 0; b < count; b++) {
+            p.r[b] = r[b];
+            p.e[b] = e[b];
+            p.en[b] = en2[b];
+        }
+        const int64_t n = net->ncell;
+        float *gr = net->lg_in, *ge = gr + (size_t)net->lg_cap * n;
+        k_gather_pairs<<<dim3(eblocks(ctx, n), count), 256, 0, ctx->stream>>>(n, count, p, gr, ge,
+                                                                              ge + (size_t)net->lg_cap * n);
         DARE_LAUNCHED(ctx);
-        if ((rc = backward(net, r[b], net->g, 1.f))) return rc;
+        DARE_CUDA(ctx, cudaGraphLaunch(net->lg_graph, ctx->stream));
+        ctx->launches += net->lg_launches;
+    } else if ((rc = queue_loss_grad(net, r, e, en2, count))) {
+        return rc;
     }
     if (loss) {
         DARE_CUDA(ctx, cudaMemcpyAsync(loss, net->dscal, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
@@ -2109,15 +2419,24 @@ static int adam_step(dare_unet* net, const dare_unet_train_params* p) {
     return pack_weights(net);
 }
 
-// ||e||^2 of device pairs into out[b] (for the public loss calls)
-static int pair_norms(dare_unet* net, const float* e, int count, float* out) {
+// ||e||^2 of device pairs into net->en[b] (for the public loss calls)
+static int pair_norms(dare_unet* net, const float* e, int count) {
     dare_ctx* ctx = net->ctx;
-    for (int b = 0; b < count; b++) {
-        DARE_CUDA(ctx, cudaMemsetAsync(net->dscal + 1, 0, sizeof(double), ctx->stream));
-        k_sqnorm<<<eblocks(ctx, net->ncell), 256, 0, ctx->stream>>>(net->ncell, e + (size_t)b * net->ncell,
-                                                                    net->dscal + 1);
+    if (net->en_cap < count) {   // [sums (double)][norms (float)]
+        cudaFree(net->en);
+        net->en = nullptr;
+        net->en_cap = 0;
+        DARE_CUDA(ctx, cudaMalloc(&net->en, (size_t)count * (sizeof(double) + sizeof(float))));
+        net->en_cap = count;
+    }
+    float* out = reinterpret_cast<float*>(net->en + net->en_cap);
+    DARE_CUDA(ctx, cudaMemsetAsync(net->en, 0, count * sizeof(double), ctx->stream));
+    for (int b = 0; b < count; b += 1024) {   // (grid and block limits)
+        const int m = std::min(count - b, 1024);
+        k_sqnorm<<<dim3(eblocks(ctx, net->ncell), m), 256, 0, ctx->stream>>>(net->ncell, e + (size_t)b * net->ncell,
+                                                                             net->en + b);
         DARE_LAUNCHED(ctx);
-        k_store_norm<<<1, 1, 0, ctx->stream>>>(net->dscal + 1, out + b);
+        k_store_norm<<<1, m, 0, ctx->stream>>>(net->en + b, out + b);
         DARE_LAUNCHED(ctx);
     }
     return DARE_OK;
@@ -2144,6 +2463,11 @@ void dare_unet_train_params_default(dare_unet_train_params* p) {
 }
 
 static void unet_free(dare_unet* net) {
+    drop_loss_graph(net);
+    for (auto* ln : net->lane) free_lane(ln);
+    cudaFree(net->lg_in);
+    cudaFree(net->en);
+    if (net->fork) cudaEventDestroy(net->fork);
     for (int l = 0; l < kLayers; l++) {
         cudaFree(net->layer[l].wf);
         cudaFree(net->layer[l].wb);
@@ -2199,7 +2523,9 @@ int dare_unet_create(dare_ctx* ctx, const int n[3], uint64_t seed, dare_unet** o
         const bool fits_bwd = l == ENC0   ? true
                               : l == DEC0 ? in_smem(kInMT) <= kMaxSmem
                                           : fwd_smem(L.coutk, L.ntb, g, 1, 4) <= kMaxSmem;
-        if (!fits_fwd || !fits_bwd || wgr_smem(L.cink, L.coutk, g, l == ENC0, l == DEC0) > kMaxSmem) {
+        // (a row length limit: what the first layers' weight gradients would take with their FP32 side staged too)
+        const size_t fp32 = l == ENC0 ? 4 * (size_t)((stage_rows(g) + 3) / 4 * 16) : l == DEC0 ? 2 * kTileM * 4 : 0;
+        if (!fits_fwd || !fits_bwd || wgr_smem(L.cink, L.coutk, g) + fp32 > kMaxSmem) {
             delete net;
             return set_error(ctx, DARE_ERR_UNSUPPORTED, "dare_unet_create: grid too wide for the staged convolutions");
         }
@@ -2209,28 +2535,7 @@ int dare_unet_create(dare_ctx* ctx, const int n[3], uint64_t seed, dare_unet** o
     }
     net->nparam = off;
 
-    // activations: one zeroed block, every buffer 256-byte aligned
-    const int64_t T[4] = {net->geo[0].total, net->geo[1].total, net->geo[2].total, net->geo[3].total};
-    struct Slot {
-        bf16** p;
-        int level, c, extra;
-    } slots[] = {{&net->S0, 0, 16}, {&net->P1, 1, 16}, {&net->S1, 1, 32}, {&net->P2, 2, 32}, {&net->S2, 2, 64},
-                 {&net->P3, 3, 64}, {&net->E3, 3, 64}, {&net->dS0, 0, 16}, {&net->dD1, 1, 16}, {&net->dS1, 1, 32},
-                 {&net->dD2, 2, 32}, {&net->dS2, 2, 64}, {&net->dD3, 3, 64}, {&net->dE3, 3, 64}, {&net->dP3, 3, 64},
-                 {&net->dP2, 2, 32}, {&net->dP1, 1, 16}};
-    // a staged plane segment reaches up to W + 8 rows before the start of an
-    // array (the unused halo of the ghost plane 0) and kActSlackRows bounds W
-    size_t bytes = (size_t)kActSlackRows * 16;
-    std::vector<size_t> offs;
-    for (auto& s : slots) {
-        offs.push_back(bytes);
-        bytes += (((size_t)T[s.level] * s.c + s.extra) * sizeof(bf16) + 255) / 256 * 256;
-    }
-    bytes += (size_t)kActSlackRows * 16;  // rows a staged segment may read past the last array
-    cudaError_t e = cudaMalloc(&net->act_block, bytes);
-    if (e == cudaSuccess) e = cudaMemset(net->act_block, 0, bytes);
-    for (size_t i = 0; i < sizeof(slots) / sizeof(slots[0]) && e == cudaSuccess; i++)
-        *slots[i].p = reinterpret_cast<bf16*>(static_cast<uint8_t*>(net->act_block) + offs[i]);
+    cudaError_t e = alloc_acts(net, 0, nullptr, 0);
     const size_t pb = net->nparam * sizeof(float);
     // (grid sizes are multiples of 8, so the pitched copy is only for a
     // caller's vector that does not start on a 16-byte boundary)
@@ -2312,6 +2617,7 @@ int dare_unet_system_shape(const dare_unet* net, int n[3]) {
 int dare_unet_set_wait_limit(dare_unet* net, int64_t polls) {
     if (!net || polls < 0 || polls > 0xFFFFFFFFll) return DARE_ERR_BAD_ARG;
     net->wait_limit = polls == 0 ? kWaitLimit : (uint32_t)polls;
+    drop_loss_graph(net);   // it holds the old limit
     return DARE_OK;
 }
 
@@ -2383,9 +2689,9 @@ int dare_unet_loss_grad(dare_unet* net, const float* r, const float* e, int coun
     if (!net || !r || !e || count < 1) return DARE_ERR_BAD_ARG;
     dare_ctx* ctx = net->ctx;
     cudaSetDevice(ctx->device);
-    float* en2 = nullptr;
-    DARE_CUDA(ctx, cudaMalloc(&en2, count * sizeof(float)));
-    int rc = pair_norms(net, e, count, en2);
+    int rc = pair_norms(net, e, count);
+    if (rc) return rc;
+    const float* en2 = reinterpret_cast<const float*>(net->en + net->en_cap);
     std::vector<const float*> rp(count), ep(count), np(count);
     for (int b = 0; b < count; b++) {
         rp[b] = r + (size_t)b * net->ncell;
@@ -2393,14 +2699,13 @@ int dare_unet_loss_grad(dare_unet* net, const float* r, const float* e, int coun
         np[b] = en2 + b;
     }
     double l = 0.;
-    if (!rc) rc = loss_grad(net, rp.data(), ep.data(), np.data(), count, &l);
+    rc = loss_grad(net, rp.data(), ep.data(), np.data(), count, &l);
     if (!rc && grad_host) {
         cudaError_t ce = cudaMemcpyAsync(grad_host, net->grad, net->nparam * sizeof(float), cudaMemcpyDeviceToHost,
                                          ctx->stream);
         if (ce == cudaSuccess) ce = cudaStreamSynchronize(ctx->stream);
         if (ce != cudaSuccess) rc = check_cuda(ctx, ce, "dare_unet_loss_grad");
     }
-    cudaFree(en2);
     if (loss) *loss = l;
     return rc;
 }

@@ -83,7 +83,6 @@ constexpr LayerDef kDefs[kLayers] = {{0, 1, 16},  {1, 16, 32}, {2, 32, 64}, {3, 
                                      {3, 64, 64}, {2, 64, 32}, {1, 32, 16}, {0, 16, 1}};
 enum LayerId { ENC0 = 0, ENC1, ENC2, ENC3, DEC3, DEC2, DEC1, DEC0 };
 
-enum { IN_BF16 = 0, IN_EMBED = 1 };                  // operand staging
 enum { OUT_STORE = 0, OUT_ADDUP = 1, OUT_F32 = 2 };  // forward epilogue
 
 struct LaunchCfg {
@@ -155,12 +154,24 @@ struct dare_unet {
     dare_gpu::unet::bf16* dP2 = nullptr;
     dare_gpu::unet::bf16* dP1 = nullptr;
     void* act_block = nullptr;            // one allocation for all of the above
+    // Training: the pairs of a minibatch run side by side, each lane with its
+    // own activations, gradients and stream (the network's own are lane 0)
+    struct dare_unet_lane* lane[4] = {nullptr, nullptr, nullptr, nullptr};
+    cudaEvent_t fork = nullptr;
+    // ... as one graph from the second minibatch of the same size on, its
+    // inputs copied into lg_in ([residuals][errors][norms] of lg_cap pairs)
+    cudaGraphExec_t lg_graph = nullptr;
+    int lg_count = 0, lg_last = 0, lg_cap = 0;
+    int64_t lg_launches = 0;
+    float* lg_in = nullptr;
     float* X0 = nullptr;                  // k_conv_in input with a 16-byte row pitch, when the caller's has none
     float* z = nullptr;                   // forward output during training
     float* g = nullptr;                   // dL/dz
     float* part = nullptr;                // weight-gradient partial sums
     size_t part_floats = 0;
     double* dscal = nullptr;              // [0] loss accumulator
+    double* en = nullptr;                 // ||e||^2 of en_cap pairs of a public loss call, then as floats
+    int en_cap = 0;
     int* err = nullptr;                   // device error word (bounded waits)
     uint32_t wait_limit = 1u << 22;       // polls of the role-to-role waits (= tc::kWaitLimit; dare_unet_set_wait_limit)
     int debug_skip = 0;                   // one-shot test hook (dare_unet_debug_skip_plane)
