@@ -49,7 +49,7 @@ namespace dare_gpu {
 // ---------------------------------------------------------------------------
 MarchCfg march_config(const dare_ctx* ctx, const GridDev& g, size_t elem, int max_items) {
     MarchCfg m;
-    const int n0 = g.n[0], n1 = g.n[1], n2 = g.n[2];
+    const int n1 = g.n[1], n2 = g.n[2];
     int tk = n2 > 16 ? 32 : n2 > 8 ? 16 : n2 > 4 ? 8 : n2 > 2 ? 4 : 1;
     int tj = 256 / tk;
     if (n2 % 2 == 0 && n2 >= 32) {
@@ -70,19 +70,7 @@ MarchCfg march_config(const dare_ctx* ctx, const GridDev& g, size_t elem, int ma
     m.block = dim3(tk, tj, 1);
     m.tiles_x = (n2 + tk * m.cpt - 1) / (tk * m.cpt);
     m.tiles_y = (n1 + tj - 1) / tj;
-    const int64_t tiles = (int64_t)m.tiles_x * m.tiles_y;
-    // Longest plane run that still leaves ~4 items per resident block (the
-    // dynamic queue then ends with a short tail); each run re-reads 2 planes.
-    // With several field components (stacked along i) runs stay inside one.
-    const int nc = g.ncomp, n0c = n0 / nc;
-    const int64_t want = (int64_t)ctx->num_sms * 3 * 4;
-    int planes = 32;
-    while (planes > 4 && tiles * nc * ((n0c + planes - 1) / planes) < want) planes /= 2;
-    while (tiles * nc * ((n0c + planes - 1) / planes) > max_items && planes < n0c) planes *= 2;
-    if (planes > n0c) planes = n0c;
-    m.planes = planes;
-    m.cpc = (n0c + planes - 1) / planes;
-    m.nitems = (int)(tiles * nc * m.cpc);
+    march_split(g, m, (int64_t)ctx->num_sms * 2, max_items);
     m.smem = 2 * (size_t)(tk * m.cpt + 2) * (tj + 2) * elem;
     return m;
 }

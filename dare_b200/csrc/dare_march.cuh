@@ -993,9 +993,36 @@ __global__ void __launch_bounds__(256, MarchMinBlocks<K, CPT>::value) k_march(Gr
     }
 }
 
+// The plane runs of a tile for a kernel with `slots` resident blocks: an item of
+// p planes costs a block about p + 3 plane times (filling its pipeline and its
+// reduction), and the last round of items is usually not full, so take the
+// number of runs whose rounds are the cheapest.  Runs of 4 planes, as many as
+// gave four items a block, cost 128^3 steps 2.12 ms and 192^3 steps 5.28; 15-
+// and 28-plane runs in two and four rounds 1.78 and 4.68 (1.5 or 5 in place of
+// 3 planes: within 4 % either way).  With several field components (stacked
+// along i) runs stay inside one.
+inline void march_split(const GridDev& g, MarchCfg& m, int64_t slots, int max_items) {
+    const int nc = g.ncomp, n0c = g.n[0] / nc;
+    const int64_t tiles = (int64_t)m.tiles_x * m.tiles_y * nc;
+    int64_t best = 0;
+    for (int runs = 1; runs <= n0c; runs++) {
+        const int p = (n0c + runs - 1) / runs;
+        if (runs > 1 && (p < 4 || tiles * runs > max_items)) break;
+        if ((n0c + p - 1) / p != runs) continue;   // the same runs as with fewer
+        const int64_t cost = (tiles * runs + slots - 1) / slots * (p + 3);
+        if (runs == 1 || cost < best) {
+            best = cost;
+            m.planes = p;
+            m.cpc = runs;
+        }
+    }
+    m.nitems = (int)(tiles * m.cpc);
+}
+
 template <class K, int CPT, bool HALO, bool PAIR>
-inline int launch_march_k(dare_ctx* ctx, const GridDev& g, const MarchCfg& m, const K& kern, SolverState* st,
+inline int launch_march_k(dare_ctx* ctx, const GridDev& g, const MarchCfg& m0, const K& kern, SolverState* st,
                           double* partials) {
+    MarchCfg m = m0;
     const int ic = PAIR ? 16 / (int)sizeof(typename K::type) : m.cpt;   // first interior column of an operand row
     const size_t smem = 3 * march_stage_elems<K>(m.block.x * m.cpt, m.block.y, ic) * sizeof(typename K::type);
     static int per_sm = 0;
@@ -1010,6 +1037,7 @@ inline int launch_march_k(dare_ctx* ctx, const GridDev& g, const MarchCfg& m, co
         per_sm_smem = smem;
     }
     int blocks = per_sm * ctx->num_sms;
+    if (m.nitems_total == 0) march_split(g, m, blocks, kMaxBlocks);   // (slabs share the slots of their runs)
     if (blocks > m.nitems) blocks = m.nitems;
     k_march<K, CPT, HALO, PAIR><<<blocks, m.block, smem, ctx->stream>>>(g, kern, st, partials, m);
     DARE_LAUNCHED(ctx);
