@@ -171,8 +171,8 @@ int launch_iteration(dare_ctx* ctx, const GridDev& g, const MarchCfg& m, int sbl
         for (const void* a : arrs)
             if (a && reinterpret_cast<uintptr_t>(a) % 16 != 0) vec4 = 0;
     }
-    k_step5<T><<<sblocks, 256, 0, sm>>>(g.ncell, vs.x, vs.r, vs.u, vs.v, vs.s, vs.w, vs.t, vs.rh, st, partials, 0, 0,
-                                        vec4);
+    launch_pdl(k_step5<T>, dim3(sblocks), dim3(256), 0, sm, true, g.ncell, vs.x, vs.r, vs.u, vs.v, vs.s, vs.w, vs.t,
+               vs.rh, st, partials, 0, 0, vec4);
     DARE_LAUNCHED(ctx);
     if (ev) DARE_CUDA(ctx, cudaEventRecord(ev[5], sm));
     return DARE_OK;

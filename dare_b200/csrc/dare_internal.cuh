@@ -153,6 +153,37 @@ __host__ __device__ inline void neighbour_ordinals(const GridDev& g, int i, int 
     nb[6] = k < g.n[2] - 1 ? c + 1 : (g.periodic[2] ? c - (g.n[2] - 1) : c);
 }
 
+// ---- programmatic dependent launch ----------------------------------------
+// Kernels of the network and of the solver's iterations follow one another
+// every 3-50 us.  Launched this way, a kernel's blocks may be placed while the
+// one before it still runs; they meet it at pdl_wait(), which every thread
+// passes before it touches anything that an earlier kernel writes, and which
+// ends when the earlier kernel has ended and its stores are visible.  Only
+// then do they let the next kernel in (pdl_launch): so when a kernel's first
+// instructions run, every kernel but the one directly before it is complete,
+// and what those wrote (the convolutions' weights) may be read ahead of the
+// wait.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// A launch that need not wait for the kernel before it to end (`overlap` off:
+// an ordinary one)
+template <typename... P, typename... A>
+inline void launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, bool overlap,
+                       A&&... args) {
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c{};
+    c.gridDim = grid;
+    c.blockDim = block;
+    c.dynamicSmemBytes = smem;
+    c.stream = stream;
+    c.attrs = at;
+    c.numAttrs = overlap ? 1 : 0;
+    cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);   // an error is picked up by DARE_LAUNCHED
+}
+
 inline int grid_blocks(const dare_ctx* ctx, int64_t work, int threads, int per_sm) {
     int64_t b = (work + threads - 1) / threads;
     int64_t cap = (int64_t)ctx->num_sms * per_sm;

@@ -247,6 +247,8 @@ __global__ void __launch_bounds__(256) k_init(int64_t n, Vecs vs, SolverState* s
 
 // (3), (4): rho1 = <rh, r>, beta
 __global__ void __launch_bounds__(256) k_rho(int64_t n, Vecs vs, SolverState* st, double* partials) {
+    pdl_wait();
+    pdl_launch();
     if (st->done) return;
     double acc[1] = {0.};
     GRID_LOOP(q, n / 4) acc[0] += dot4(ld4(vs.rh, q), ld4(vs.r, q));
@@ -264,6 +266,8 @@ __global__ void __launch_bounds__(256) k_rho(int64_t n, Vecs vs, SolverState* st
 
 // (5) u = r - beta u
 __global__ void k_upd_u(int64_t n, Vecs vs, const SolverState* st) {
+    pdl_wait();
+    pdl_launch();
     if (st->done) return;
     const float beta = (float)st->beta;
     GRID_LOOP(q, n / 4) st4(vs.u, q, axmy(ld4(vs.r, q), beta, ld4(vs.u, q)));
@@ -271,6 +275,8 @@ __global__ void k_upd_u(int64_t n, Vecs vs, const SolverState* st) {
 
 // (8): r -= alpha v (the matching x update is folded into k_upd_final)
 __global__ void k_upd_r(int64_t n, Vecs vs, const SolverState* st) {
+    pdl_wait();
+    pdl_launch();
     if (st->done) return;
     const float alpha = (float)st->alpha;
     GRID_LOOP(q, n / 4) st4(vs.r, q, axmy(ld4(vs.r, q), alpha, ld4(vs.v, q)));
@@ -278,6 +284,8 @@ __global__ void k_upd_r(int64_t n, Vecs vs, const SolverState* st) {
 
 // (12) v = s - beta v
 __global__ void k_upd_v(int64_t n, Vecs vs, const SolverState* st) {
+    pdl_wait();
+    pdl_launch();
     if (st->done) return;
     const float beta = (float)st->beta;
     GRID_LOOP(q, n / 4) st4(vs.v, q, axmy(ld4(vs.s, q), beta, ld4(vs.v, q)));
@@ -285,6 +293,8 @@ __global__ void k_upd_v(int64_t n, Vecs vs, const SolverState* st) {
 
 // (15)-(17)
 __global__ void k_upd3(int64_t n, Vecs vs, const SolverState* st) {
+    pdl_wait();
+    pdl_launch();
     if (st->done) return;
     const float alpha = (float)st->alpha, beta = (float)st->beta;
     GRID_LOOP(q, n / 4) {
@@ -298,6 +308,8 @@ __global__ void k_upd3(int64_t n, Vecs vs, const SolverState* st) {
 // (10), (24) in flexible form: d += (a1 - a2 b1) zu + (a2 + w1) zr - w1 a2 zv + w2 zs;
 // (25): r -= w1 s + w2 t; u -= w1 v + w2 w; convergence test on ||r||
 __global__ void __launch_bounds__(256) k_upd_final(int64_t n, Vecs vs, SolverState* st, double* partials) {
+    pdl_wait();
+    pdl_launch();
     if (st->done) return;
     const double a1 = st->alpha1, a2 = st->alpha, b1 = st->beta1, om1 = st->omega1, om2 = st->omega2;
     const float cu = (float)(a1 - a2 * b1), cr = (float)(a2 + om1), cv = (float)(-om1 * a2), cs = (float)om2;
@@ -367,21 +379,21 @@ static int launch_iteration(dare_ctx* ctx, dare_unet* net, const GridDev& g, con
         f.out = out;
         return launch_march(ctx, g, m, f, st, partials);
     };
-    k_rho<<<eb, 256, 0, s>>>(n, vs, st, partials);
+    launch_pdl(k_rho, dim3(eb), dim3(256), 0, s, true, n, vs, st, partials);
     DARE_LAUNCHED(ctx);
-    k_upd_u<<<eb, 256, 0, s>>>(n, vs, st);
+    launch_pdl(k_upd_u, dim3(eb), dim3(256), 0, s, true, n, vs, st);
     DARE_LAUNCHED(ctx);
     if ((rc = unet::apply(net, vs.u, vs.zu))) return rc;
     if ((rc = spmv_dot(FLSpmvDot<0, 7>{}, vs.zu, vs.v))) return rc;
-    k_upd_r<<<eb, 256, 0, s>>>(n, vs, st);
+    launch_pdl(k_upd_r, dim3(eb), dim3(256), 0, s, true, n, vs, st);
     DARE_LAUNCHED(ctx);
     if ((rc = unet::apply(net, vs.r, vs.zr))) return rc;
     if ((rc = spmv_dot(FLSpmvDot<1, 11>{}, vs.zr, vs.s))) return rc;
-    k_upd_v<<<eb, 256, 0, s>>>(n, vs, st);
+    launch_pdl(k_upd_v, dim3(eb), dim3(256), 0, s, true, n, vs, st);
     DARE_LAUNCHED(ctx);
     if ((rc = unet::apply(net, vs.v, vs.zv))) return rc;
     if ((rc = spmv_dot(FLSpmvDot<0, 14>{}, vs.zv, vs.w))) return rc;
-    k_upd3<<<eb, 256, 0, s>>>(n, vs, st);
+    launch_pdl(k_upd3, dim3(eb), dim3(256), 0, s, true, n, vs, st);
     DARE_LAUNCHED(ctx);
     if ((rc = unet::apply(net, vs.s, vs.zs))) return rc;
     FLSpmvOmega fo{};
@@ -391,7 +403,7 @@ static int launch_iteration(dare_ctx* ctx, dare_unet* net, const GridDev& g, con
     fo.ps[7] = vs.s;
     fo.t = vs.t;
     if ((rc = launch_march(ctx, g, m, fo, st, partials))) return rc;
-    k_upd_final<<<eb, 256, 0, s>>>(n, vs, st, partials);
+    launch_pdl(k_upd_final, dim3(eb), dim3(256), 0, s, true, n, vs, st, partials);
     DARE_LAUNCHED(ctx);
     return DARE_OK;
 }

@@ -616,6 +616,8 @@ __global__ void __launch_bounds__(256, MarchMinBlocks<K, CPT>::value) k_march(Gr
     static_assert(!PAIR || VEC % CPT == 0, "16-byte staging: a copy covers whole thread segments");
     constexpr int IC = PAIR ? VEC : CPT;        // first interior column of a staged operand row
     constexpr int CB = CPT * (int)sizeof(T);    // bytes of one thread's row segment
+    pdl_wait();
+    pdl_launch();
     if (K::kCheckDone && st->done) return;
     K k = kern;
     k.load(st);
@@ -1039,7 +1041,7 @@ inline int launch_march_k(dare_ctx* ctx, const GridDev& g, const MarchCfg& m0, c
     int blocks = per_sm * ctx->num_sms;
     if (m.nitems_total == 0) march_split(g, m, blocks, kMaxBlocks);   // (slabs share the slots of their runs)
     if (blocks > m.nitems) blocks = m.nitems;
-    k_march<K, CPT, HALO, PAIR><<<blocks, m.block, smem, ctx->stream>>>(g, kern, st, partials, m);
+    launch_pdl(k_march<K, CPT, HALO, PAIR>, dim3(blocks), m.block, smem, ctx->stream, true, g, kern, st, partials, m);
     DARE_LAUNCHED(ctx);
     return DARE_OK;
 }
@@ -1155,6 +1157,8 @@ __global__ void __launch_bounds__(256) k_step5(int64_t n, T* __restrict__ x, T* 
                                                const T* __restrict__ w, const T* __restrict__ t,
                                                const T* __restrict__ rh, SolverState* st, double* partials, int base,
                                                int total, int vec4) {
+    pdl_wait();
+    pdl_launch();
     if (st->done) return;
     const Step5<T> f(st);
     double acc[2] = {0., 0.};

@@ -222,6 +222,8 @@ __global__ void __launch_bounds__(fwd_threads(MT)) k_conv_fwd(FwdArgs a) {
     __syncthreads();
     fence_after_sync();
     const uint32_t tmem = *tslot;
+    pdl_wait();     // the weights above are not the last kernel's; everything from here on may be
+    pdl_launch();
     // slot row 0 is position P0 - 1 - W; D row m of tile mt (position
     // P0 - 1 + 126 mt + m) reads slot rows 126 mt + m + dj W
     const int pbase = P0 - 1 - g.W;
@@ -566,6 +568,8 @@ __global__ void __launch_bounds__(in_threads()) k_conv_in(const __grid_constant_
     __syncthreads();
     fence_after_sync();
     const uint32_t tmem = *tslot;
+    pdl_wait();     // the weights above are not the last kernel's; everything from here on may be
+    pdl_launch();
 
     if (warp == 13) {
         // ---- producer: one TMA box per group of planes ----
@@ -815,6 +819,8 @@ __global__ void __launch_bounds__(out_threads(MT)) k_conv_out(OutArgs a) {
     __syncthreads();
     fence_after_sync();
     const uint32_t tmem = *tslot;
+    pdl_wait();     // the weights above are not the last kernel's; everything from here on may be
+    pdl_launch();
     // segment row 0 is position P0 - 1 - W: D row m of tile mt (position
     // P0 - 1 + 126 mt + m) reads segment rows 126 mt + m + dj W
     const int pbase = P0 - 1 - g.W;
@@ -1227,6 +1233,8 @@ __global__ void __launch_bounds__(kWgr1Warps * 32) k_wgrad_1ch(Wgr1Args a) {
 // added into the finer level
 template <int C>
 __global__ void k_restrict(Geom f, Geom c, const bf16* __restrict__ fine, bf16* __restrict__ coarse, float scale) {
+    pdl_wait();
+    pdl_launch();
     constexpr int KC = C / 8;
     const int64_t total = (int64_t)c.n0 * c.n1 * c.n2 * KC;
     for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
@@ -1266,6 +1274,8 @@ __global__ void k_restrict(Geom f, Geom c, const bf16* __restrict__ fine, bf16* 
 // i, j) line of fine cells, its threads along k
 template <int C>
 __global__ void k_prolong_add(Geom f, Geom c, const bf16* __restrict__ coarse, bf16* __restrict__ fine, float scale) {
+    pdl_wait();
+    pdl_launch();
     constexpr int KC = C / 8;
     const int lines = f.n0 * f.n1;
     for (int line = blockIdx.x; line < lines * KC; line += gridDim.x) {
@@ -1469,6 +1479,8 @@ __global__ void k_warm(int64_t n, const double* __restrict__ diag, const double*
 // (the coarse sizes are multiples of 8, so rows split into whole pairs).
 __global__ void __launch_bounds__(256) k_pool8(int c0, int c1, int c2, const float* __restrict__ f,
                                                float* __restrict__ c) {
+    pdl_wait();
+    pdl_launch();
     const int h2 = c2 / 2;
     const int64_t nq = (int64_t)c0 * c1 * h2;
     const int64_t F2 = 2 * (int64_t)c2, F1 = 2 * (int64_t)c1;
@@ -1493,6 +1505,8 @@ __global__ void __launch_bounds__(256) k_pool8(int c0, int c1, int c2, const flo
 __global__ void __launch_bounds__(256) k_coarse_add(int c0, int c1, int c2, const float* __restrict__ u,
                                                     const float* __restrict__ zc, const float* __restrict__ uc,
                                                     float* __restrict__ z) {
+    pdl_wait();
+    pdl_launch();
     const int h2 = c2 / 2;
     const int64_t F2 = 2 * (int64_t)c2, F1 = 2 * (int64_t)c1;
     const int64_t nq = (int64_t)2 * c0 * F1 * h2;   // fine cells / 4
@@ -1622,7 +1636,7 @@ static int launch_fwd_t(dare_ctx* ctx, LaunchCfg& lc, int nz, const FwdArgs& a0)
     FwdArgs a = a0;
     a.ppc = lc.ppc;
     a.slots = lc.slots;
-    kern<<<lc.grid, fwd_threads(MT), lc.smem, ctx->stream>>>(a);
+    launch_pdl(kern, lc.grid, dim3(fwd_threads(MT)), lc.smem, ctx->stream, true, a);
     DARE_LAUNCHED(ctx);
     return DARE_OK;
 }
@@ -1762,7 +1776,7 @@ static int encode_tiled(dare_ctx* ctx, CUtensorMap* m, CUtensorMapDataType type,
 constexpr int kInMT = 1;
 
 template <int MT>
-static int launch_in_t(dare_ctx* ctx, LaunchCfg& lc, InArgs& a) {
+static int launch_in_t(dare_ctx* ctx, LaunchCfg& lc, InArgs& a, bool overlap) {
     auto kern = k_conv_in<MT>;
     if (!lc.ready) {
         const uint32_t cols = kInAcc * kInB * MT * 64;
@@ -1783,7 +1797,7 @@ static int launch_in_t(dare_ctx* ctx, LaunchCfg& lc, InArgs& a) {
         lc.ready = true;
     }
     a.ppc = lc.ppc;
-    kern<<<lc.grid, in_threads(), lc.smem, ctx->stream>>>(a);
+    launch_pdl(kern, lc.grid, dim3(in_threads()), lc.smem, ctx->stream, overlap, a);
     DARE_LAUNCHED(ctx);
     return DARE_OK;
 }
@@ -1791,7 +1805,7 @@ static int launch_in_t(dare_ctx* ctx, LaunchCfg& lc, InArgs& a) {
 // The kernel reads in32 (FP32 over the internal cells) through a TMA map;
 // a row pitch that is not a multiple of 16 bytes (n2 % 4 != 0) or a base
 // that is not 16-byte aligned goes through a pitched copy in `stage` first.
-static int launch_in(dare_ctx* ctx, LaunchCfg& lc, InArgs& a, const float* in32, float* stage) {
+static int launch_in(dare_ctx* ctx, LaunchCfg& lc, InArgs& a, const float* in32, float* stage, bool overlap) {
     const Geom& g = a.g;
     const float* base = in32;
     int64_t pitch = g.n2;
@@ -1807,7 +1821,7 @@ static int launch_in(dare_ctx* ctx, LaunchCfg& lc, InArgs& a, const float* in32,
     const cuuint32_t es[3] = {1, 1, 1};
     int rc;
     if ((rc = encode_tiled(ctx, &a.x, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, base, dims, strides, box, es))) return rc;
-    return launch_in_t<kInMT>(ctx, lc, a);
+    return launch_in_t<kInMT>(ctx, lc, a, overlap);
 }
 
 // shared memory of k_conv_out with `slots` staged groups of kOutB planes
@@ -1862,7 +1876,7 @@ static int launch_out_t(dare_ctx* ctx, LaunchCfg& lc, const OutArgs& a0) {
     OutArgs a = a0;
     a.ppc = lc.ppc;
     a.slots = lc.slots;
-    kern<<<lc.grid, out_threads(MT), lc.smem, ctx->stream>>>(a);
+    launch_pdl(kern, lc.grid, dim3(out_threads(MT)), lc.smem, ctx->stream, true, a);
     DARE_LAUNCHED(ctx);
     return DARE_OK;
 }
@@ -1879,8 +1893,10 @@ static int pick_nt(int cink, int coutk, const Geom& g) {
 static inline int eblocks(const dare_ctx* ctx, int64_t work) { return grid_blocks(ctx, work, 256, 8); }
 
 // ---- network passes ----------------------------------------------------------
+// (`overlap`, enc0: the kernel before this one on the stream is one of the
+// chain; the others always follow one)
 static int conv_forward(dare_unet* net, int l, const bf16* in, const float* in32, int outm, bf16* out, bf16* fine,
-                        float* out32, const float* res32) {
+                        float* out32, const float* res32, bool overlap = true) {
     Layer& L = net->layer[l];
     if (l == ENC0) {
         InArgs a{};
@@ -1892,7 +1908,7 @@ static int conv_forward(dare_unet* net, int l, const bf16* in, const float* in32
         a.pool_scale = 0.125f;
         a.err = net->err;
         a.wait_limit = net->wait_limit;
-        return launch_in(net->ctx, L.fwd, a, in32, net->X0);
+        return launch_in(net->ctx, L.fwd, a, in32, net->X0, overlap);
     }
     if (l == DEC0) {
         OutArgs a{};
@@ -1933,7 +1949,7 @@ static int conv_dgrad(dare_unet* net, int l, const bf16* dy, const float* dy32, 
         a.pool_scale = 1.f;
         a.err = net->err;
         a.wait_limit = net->wait_limit;
-        return launch_in(net->ctx, L.bwd, a, dy32, net->X0);
+        return launch_in(net->ctx, L.bwd, a, dy32, net->X0, true);
     }
     FwdArgs a{};
     a.g = net->geo[L.level];
@@ -1986,8 +2002,8 @@ template <int C>
 static int restrict_to(dare_unet* net, int fl, const bf16* fine, bf16* coarse, float scale) {
     dare_ctx* ctx = net->ctx;
     const Geom& c = net->geo[fl + 1];
-    k_restrict<C><<<eblocks(ctx, (int64_t)c.n0 * c.n1 * c.n2 * (C / 8)), 256, 0, ctx->stream>>>(net->geo[fl], c, fine,
-                                                                                                coarse, scale);
+    launch_pdl(k_restrict<C>, dim3(eblocks(ctx, (int64_t)c.n0 * c.n1 * c.n2 * (C / 8))), dim3(256), 0, ctx->stream, true,
+               net->geo[fl], c, fine, coarse, scale);
     DARE_LAUNCHED(ctx);
     return DARE_OK;
 }
@@ -1997,17 +2013,18 @@ static int prolong_add(dare_unet* net, int fl, const bf16* coarse, bf16* fine, f
     dare_ctx* ctx = net->ctx;
     const Geom& f = net->geo[fl];
     const int64_t lines = (int64_t)f.n0 * f.n1 * (C / 8);
-    k_prolong_add<C><<<(int)std::min<int64_t>(lines, (int64_t)ctx->num_sms * 16), 128, 0, ctx->stream>>>(
-        f, net->geo[fl + 1], coarse, fine, scale);
+    launch_pdl(k_prolong_add<C>, dim3((unsigned)std::min<int64_t>(lines, (int64_t)ctx->num_sms * 16)), dim3(128), 0,
+               ctx->stream, true, f, net->geo[fl + 1], coarse, fine, scale);
     DARE_LAUNCHED(ctx);
     return DARE_OK;
 }
 
-// z = u + U(u) on the network's own grid
-static int apply_grid(dare_unet* net, const float* u, float* z) {
+// z = u + U(u) on the network's own grid (`overlap`: right after a kernel that
+// does not write the weights)
+static int apply_grid(dare_unet* net, const float* u, float* z, bool overlap) {
     int rc;
     // enc0 also writes P1, the average pool of S0
-    if ((rc = conv_forward(net, ENC0, nullptr, u, OUT_STORE, net->S0, nullptr, nullptr, nullptr))) return rc;
+    if ((rc = conv_forward(net, ENC0, nullptr, u, OUT_STORE, net->S0, nullptr, nullptr, nullptr, overlap))) return rc;
     if ((rc = conv_forward(net, ENC1, net->P1, nullptr, OUT_STORE, net->S1, nullptr, nullptr, nullptr))) return rc;
     if ((rc = restrict_to<32>(net, 1, net->S1, net->P2, 0.125f))) return rc;
     if ((rc = conv_forward(net, ENC2, net->P2, nullptr, OUT_STORE, net->S2, nullptr, nullptr, nullptr))) return rc;
@@ -2024,7 +2041,7 @@ static int apply_grid(dare_unet* net, const float* u, float* z) {
 }
 
 int apply(dare_unet* net, const float* u, float* z) {
-    if (!net->coarse) return apply_grid(net, u, z);
+    if (!net->coarse) return apply_grid(net, u, z, false);
     // coarse form: z = u + P (N_c(R u) - R u), N_c(v) = v + U(v) on the coarse grid
     dare_ctx* ctx = net->ctx;
     float* uc = net->cbuf;
@@ -2040,12 +2057,13 @@ int apply(dare_unet* net, const float* u, float* z) {
         uin = net->fbuf;
         zout = net->fbuf + net->fine_ncell;
     }
-    k_pool8<<<eblocks(ctx, net->ncell / 2), 256, 0, ctx->stream>>>(net->n[0], net->n[1], net->n[2], uin, uc);
+    launch_pdl(k_pool8, dim3(eblocks(ctx, net->ncell / 2)), dim3(256), 0, ctx->stream, true, net->n[0], net->n[1],
+               net->n[2], uin, uc);
     DARE_LAUNCHED(ctx);
-    int rc = apply_grid(net, uc, zc);
+    int rc = apply_grid(net, uc, zc, true);
     if (rc) return rc;
-    k_coarse_add<<<eblocks(ctx, net->fine_ncell / 4), 256, 0, ctx->stream>>>(net->n[0], net->n[1], net->n[2], uin, zc,
-                                                                              uc, zout);
+    launch_pdl(k_coarse_add, dim3(eblocks(ctx, net->fine_ncell / 4)), dim3(256), 0, ctx->stream, true, net->n[0],
+               net->n[1], net->n[2], uin, zc, uc, zout);
     DARE_LAUNCHED(ctx);
     if (zout != z)
         DARE_CUDA(ctx, cudaMemcpyAsync(z, zout, net->fine_ncell * sizeof(float), cudaMemcpyDeviceToDevice, ctx->stream));
@@ -2276,7 +2294,7 @@ static int queue_loss_grad(dare_unet* net, const float* const* r, const float* c
                 if (!ln->layer[l].bwd.ready) ln->layer[l].bwd = first->layer[l].bwd;
             }
         }
-        if ((rc = apply_grid(ln, r[b], ln->z)) == DARE_OK) {   // pairs live on the network's grid
+        if ((rc = apply_grid(ln, r[b], ln->z, false)) == DARE_OK) {   // pairs live on the network's grid
             k_loss_grad<<<eblocks(ctx, net->ncell), 256, 0, lc->stream>>>(net->ncell, ln->z, e[b], en2[b], scale, ln->g,
                                                                           net->dscal);
             lc->launches++;
