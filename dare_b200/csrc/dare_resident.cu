@@ -1,6 +1,6 @@
 // dare_resident.cu -- the plain FP64 BiCGStab(2) solve of a small system as
-// one cooperative kernel (dare_team.cuh): the fold, the iterations and the
-// exit, with CopyTo and the periodic ghosts in a time step.
+// one kernel, a cooperative launch or a single cluster (dare_team.cuh): the
+// fold, the iterations and the exit, with CopyTo and the periodic ghosts in a time step.
 //
 // What bounds a small solve is not its bytes: a 64^3 iteration moves 109 MB
 // through L2 but its five kernels, each a launch with a queue of items and a
@@ -123,7 +123,8 @@ struct ResidentOp {
     }
 };
 
-template <bool UNIT, int CPT>
+// CLUSTER: the blocks are one cluster, otherwise those of a cooperative launch
+template <bool UNIT, int CPT, bool CLUSTER>
 __global__ void __launch_bounds__(kResidentThreads, 1) k_resident(ResidentArgs A) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ TeamShared sh;
@@ -137,7 +138,13 @@ __global__ void __launch_bounds__(kResidentThreads, 1) k_resident(ResidentArgs A
     ResidentOp<UNIT, CPT> op{A.geo, smem,      smem + (size_t)NC * ch,
                              reinterpret_cast<unsigned char*>(smem + (size_t)(NC + 1) * ch + 2 * A.geo.sy),
                              A.ncell, ch, m, c0};
-    GridTeam team{A.buf, &sh, (int)blockIdx.x, (int)gridDim.x, 0u};
+    const auto make_team = [&]() {
+        if constexpr (CLUSTER)
+            return ClusterTeam::here(&sh);
+        else
+            return GridTeam{A.buf, &sh, (int)blockIdx.x, (int)gridDim.x, 0u};
+    };
+    auto team = make_team();
     team.start();
     if (tid == 0) {
         SolverState z{};
@@ -153,7 +160,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1) k_resident(ResidentArgs A
     bool ok = true;
     const double none[1] = {0.};
     __syncthreads();
-    if (UNIT) ok = team.sum<1>(none, [](const double*) {});   // invd of every block
+    if (UNIT) ok = team.template sum<1>(none, [](const double*) {});   // invd of every block
     // Ahat = A D^-1 (columns scaled) into shared memory; r = b - Ahat y,
     // r_hat_0 = r, u = 0
     if (ok) {
@@ -177,7 +184,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1) k_resident(ResidentArgs A
                     a2[0] += rr * rr;
                     a2[1] += bc * bc;
                 });
-        ok = team.sum<2>(a2, [&](const double* t) { finish_init(st, t); }) && team_iterations(team, op, A.v, st);
+        ok = team.template sum<2>(a2, [&](const double* t) { finish_init(st, t); }) && team_iterations(team, op, A.v, st);
     }
     if (ok) {
         // the exit: step (10) when the solve stopped between it and the last
@@ -215,7 +222,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1) k_resident(ResidentArgs A
             }
         });
         if (A.want_residual) {   // ||b - A x||_2 with the assembled rows
-            ok = team.sum<1>(none, [](const double*) {});
+            ok = team.template sum<1>(none, [](const double*) {});
             double a1[1] = {0.};
             if (ok) {
                 op.template each<1>([&](int c) {
@@ -231,7 +238,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1) k_resident(ResidentArgs A
                     const double r = A.b[c] - apply_pre<double, false>(p, z);
                     a1[0] += r * r;
                 });
-                ok = team.sum<1>(a1, [&](const double* t) { st->tres = sqrt(t[0]); });
+                ok = team.template sum<1>(a1, [&](const double* t) { st->tres = sqrt(t[0]); });
             }
         }
     }
@@ -248,6 +255,9 @@ __global__ void __launch_bounds__(kResidentThreads, 1) k_resident(ResidentArgs A
 // shared memory: beyond that the marching kernels are the faster path (their
 // vectors no longer stay in L2 either).
 constexpr int kResidentCells = 4;   // most cells a thread
+// Measured solves, cluster / device: 24^3 43 / 59 us, 32^3 58 / 60, 36^3 94 / 83;
+// two species on 90^2 76 / 103, 120^2 113 / 128, 160^2 211 / 168
+constexpr int64_t kClusterCells = 1 << 15;
 static size_t resident_smem(bool unit, int chunk, int sy) {
     return ((size_t)chunk * (unit ? 7 : 8) + 2 * (size_t)sy) * sizeof(double) + chunk;
 }
@@ -256,10 +266,13 @@ bool resident_shape(const dare_ctx* ctx, const GridDev& g, bool unit, int* block
     const int64_t n = g.ncell;
     const int nb = ctx->num_sms < kTeamMaxBlocks ? ctx->num_sms : kTeamMaxBlocks;
     if (n > (int64_t)nb * kResidentThreads * kResidentCells) return false;
-    // as many blocks as have a cell for each of half their threads: below
-    // that an SM more does not shorten a pass
+    // Up to kClusterCells cells one cluster, whose exchanges take 1 us where
+    // the device's take 3; beyond that the device, whose passes are shorter.
+    // As many blocks as have a cell for each of half their threads: below
+    // that an SM more does not shorten a pass.
     int64_t want = (n + kResidentThreads / 2 - 1) / (kResidentThreads / 2);
-    if (want > nb) want = nb;
+    const int64_t most = n <= kClusterCells ? kClusterMaxBlocks : nb;
+    if (want > most) want = most;
     int64_t ch = (n + want - 1) / want;
     ch = (ch + 31) / 32 * 32;
     if (ch > kResidentThreads * kResidentCells || g.n[2] > (1 << 15) || resident_smem(unit, (int)ch, g.n[2]) > kMost)
@@ -272,7 +285,26 @@ bool resident_shape(const dare_ctx* ctx, const GridDev& g, bool unit, int* block
 template <bool UNIT, int CPT>
 static int launch_resident_t(dare_ctx* ctx, ResidentArgs& a, int blocks) {
     const size_t smem = resident_smem(UNIT, a.chunk, a.geo.sy);
-    const auto k = k_resident<UNIT, CPT>;
+    if (blocks <= kClusterMaxBlocks) {
+        const auto k = k_resident<UNIT, CPT, true>;
+        DARE_CUDA(ctx, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        DARE_CUDA(ctx, cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = (unsigned)blocks;
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+        cudaLaunchConfig_t c{};
+        c.gridDim = dim3(blocks);
+        c.blockDim = dim3(kResidentThreads);
+        c.dynamicSmemBytes = smem;
+        c.stream = ctx->stream;
+        c.attrs = at;
+        c.numAttrs = 1;
+        DARE_CUDA(ctx, cudaLaunchKernelEx(&c, k, a));
+        DARE_LAUNCHED(ctx);
+        return DARE_OK;
+    }
+    const auto k = k_resident<UNIT, CPT, false>;
     DARE_CUDA(ctx, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     void* args[] = {&a};
     DARE_CUDA(ctx, cudaLaunchCooperativeKernel((const void*)k, dim3(blocks), dim3(kResidentThreads), args, smem,

@@ -203,6 +203,8 @@ struct ClusterTeam {
     int rank, size;
     unsigned set;
 
+    __device__ void start() {}
+    __device__ void stop() {}
     __device__ static ClusterTeam here(TeamShared* sh) {
         unsigned r, n;
         asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));

@@ -1,6 +1,6 @@
 """The one-launch solve of small systems (dare_resident.cu) at the sizes where
-its blocks are cut: one block, a remainder in the last block, one to four cells
-a thread, the largest system it takes and the first one that goes to the
+its blocks are cut: one block, a remainder in the last block, the largest single
+cluster and the first cooperative launch, one to four cells a thread, the largest system it takes and the first one that goes to the
 marching kernels; every mix of periodic and bounded directions, one to three
 dimensions, two components, with and without Jacobi.
 
@@ -47,7 +47,7 @@ def _apply(diag, x, n, periodic):
 
 CASES = [((3, 3, 3), (0, 0, 0), 1), ((8, 8, 8), (1, 1, 1), 1), ((8, 8, 9), (0, 1, 0), 1), ((17, 13, 10), (1, 0, 1), 1),
          ((5, 700), (0, 1), 1), ((3000,), (1,), 1), ((4000,), (0,), 2), ((40, 33), (1, 0), 2), ((12, 11, 9), (0, 0, 1), 2),
-         ((53, 54, 52), (1, 1, 0), 1), ((66, 65, 67), (0, 1, 1), 1), ((76, 75, 77), (1, 0, 1), 1),
+         ((32, 32, 32), (1, 0, 1), 1), ((33, 32, 32), (0, 1, 1), 1), ((53, 54, 52), (1, 1, 0), 1), ((66, 65, 67), (0, 1, 1), 1), ((76, 75, 77), (1, 0, 1), 1),
          ((83, 84, 84), (1, 1, 1), 1), ((84, 85, 84), (0, 1, 1), 1)]
 
 
