@@ -80,6 +80,153 @@ __device__ __forceinline__ void tvd_face(bool upper, double m2, double m1, doubl
     rr = ((-0.5 * psi) * (pD - pU)) * v;
 }
 
+// What one cell's functor reads: phi along i, the x faces' values (a marching
+// thread keeps them), and where the rest lies
+struct AsmLine {
+    double w[5];                             // phi(i-2 .. i+2)
+    double vx_lo, vx_up, Dx_lo, Dx_up;       // x-face velocity and diffusivity
+    int64_t loc;                             // ghosted index of the cell
+    int64_t fy_lo, fy_up, fz_lo, fz_up;      // its y and z faces
+};
+
+// One part of a cell's functor: adds `a`'s terms to coef and rhs in the
+// reference's order, then folds the boundary faces if a.fold.
+template <int DIM>
+__device__ __forceinline__ void asm_cell(const GridDev& g, const AsmParams& a, const AsmLine& L,
+                                         const double* __restrict__ phi, const double* __restrict__ phi_old, int i,
+                                         int jj, int kk, double (&coef)[7], double& rhs) {
+    const int64_t S1 = g.gn[2];
+    (void)S1;
+    if (a.dt > 0.) {                                   // DDT, weights (1, 1)
+        const double tt = a.tt;
+        if (a.sgn_ddt > 0.) {                           // from zero: C = tt, rhs = 0 + tt phi_old
+            coef[DARE_CENTER] += tt;
+            rhs += tt * phi_old[L.loc];
+        } else {                                        // MatrixBlock -=: += (-1 s)
+            coef[DARE_CENTER] += -1. * tt;
+            rhs += -1. * (tt * phi_old[L.loc]);
+        }
+    }
+
+    if (a.convection) {                                // TVD * field, then divergence
+        double nb[7], cf[7], rr[7];
+#pragma unroll
+        for (int p = 0; p < 7; p++) nb[p] = cf[p] = rr[p] = 0.;
+        double vlo, vup;
+        // x (always active)
+        if (a.convection == 1) {
+            vlo = vup = a.vel[0];
+        } else {
+            vlo = L.vx_lo;
+            vup = L.vx_up;
+        }
+        tvd_face(false, L.w[0], L.w[1], L.w[2], L.w[3], L.w[4], vlo, a.limiter, nb[DARE_WEST], cf[DARE_WEST], rr[DARE_WEST]);
+        tvd_face(true, L.w[0], L.w[1], L.w[2], L.w[3], L.w[4], vup, a.limiter, nb[DARE_EAST], cf[DARE_EAST], rr[DARE_EAST]);
+        if (DIM > 1) {
+            const double m2 = phi[L.loc - 2 * S1], m1 = phi[L.loc - S1], p1 = phi[L.loc + S1], p2 = phi[L.loc + 2 * S1];
+            if (a.convection == 1) {
+                vlo = vup = a.vel[1];
+            } else {
+                vlo = a.face_vel[1][L.fy_lo];
+                vup = a.face_vel[1][L.fy_up];
+            }
+            tvd_face(false, m2, m1, L.w[2], p1, p2, vlo, a.limiter, nb[DARE_SOUTH], cf[DARE_SOUTH], rr[DARE_SOUTH]);
+            tvd_face(true, m2, m1, L.w[2], p1, p2, vup, a.limiter, nb[DARE_NORTH], cf[DARE_NORTH], rr[DARE_NORTH]);
+        }
+        if (DIM > 2) {
+            const double m2 = phi[L.loc - 2], m1 = phi[L.loc - 1], p1 = phi[L.loc + 1], p2 = phi[L.loc + 2];
+            if (a.convection == 1) {
+                vlo = vup = a.vel[2];
+            } else {
+                vlo = a.face_vel[2][L.fz_lo];
+                vup = a.face_vel[2][L.fz_up];
+            }
+            tvd_face(false, m2, m1, L.w[2], p1, p2, vlo, a.limiter, nb[DARE_BOTTOM], cf[DARE_BOTTOM], rr[DARE_BOTTOM]);
+            tvd_face(true, m2, m1, L.w[2], p1, p2, vup, a.limiter, nb[DARE_TOP], cf[DARE_TOP], rr[DARE_TOP]);
+        }
+        double sc[7];
+        apply_divergence<DIM>(g, nb, cf, sc);
+#pragma unroll
+        for (int p = 0; p < 7; p++) sc[p] *= a.w[0];           // s_c *= weight[0]
+        double srhs = g.area[0] * (rr[DARE_EAST] - rr[DARE_WEST]);
+        if (DIM > 1) srhs += g.area[1] * (rr[DARE_NORTH] - rr[DARE_SOUTH]);
+        if (DIM > 2) srhs += g.area[2] * (rr[DARE_TOP] - rr[DARE_BOTTOM]);
+        for (int t = 1; t <= a.nexp; t++) {                // explicit levels (copies of level 0)
+            srhs += a.w[t] * g.area[0] * (rr[DARE_EAST] - rr[DARE_WEST]);
+            if (DIM > 1) srhs += a.w[t] * g.area[1] * (rr[DARE_NORTH] - rr[DARE_SOUTH]);
+            if (DIM > 2) srhs += a.w[t] * g.area[2] * (rr[DARE_TOP] - rr[DARE_BOTTOM]);
+        }
+        if (a.sgn_conv > 0.) {                           // MatrixBlock::Add
+#pragma unroll
+            for (int p = 0; p < 7; p++) coef[p] += sc[p];
+            rhs += srhs;
+        } else {                                        // MatrixBlock -=
+#pragma unroll
+            for (int p = 0; p < 7; p++) coef[p] += -1. * sc[p];
+            rhs += -1. * srhs;
+        }
+    }
+
+    if (a.diffusion) {                                 // mb -= div(D, grad(mb))
+        double Dlo[3], Dup[3];
+        if (a.diffusion == 1) {
+#pragma unroll
+            for (int d = 0; d < 3; d++) Dlo[d] = Dup[d] = a.D;
+        } else {
+            Dlo[0] = L.Dx_lo;
+            Dup[0] = L.Dx_up;
+            Dlo[1] = DIM > 1 ? a.face_D[1][L.fy_lo] : 0.;
+            Dup[1] = DIM > 1 ? a.face_D[1][L.fy_up] : 0.;
+            Dlo[2] = DIM > 2 ? a.face_D[2][L.fz_lo] : 0.;
+            Dup[2] = DIM > 2 ? a.face_D[2][L.fz_up] : 0.;
+        }
+        double nb[7], cf[7];
+#pragma unroll
+        for (int p = 0; p < 7; p++) nb[p] = cf[p] = 0.;
+#pragma unroll
+        for (int d = 0; d < DIM; d++) {
+            const double dn = a.dn[d];
+            const int lo = 2 * d + 1, up = 2 * d + 2;
+            nb[lo] = (-dn) * Dlo[d];
+            cf[lo] = dn * Dlo[d];
+            nb[up] = dn * Dup[d];
+            cf[up] = (-dn) * Dup[d];
+        }
+        double sc[7];
+        apply_divergence<DIM>(g, nb, cf, sc);
+#pragma unroll
+        for (int p = 0; p < 7; p++) sc[p] *= a.w[0];           // s_c *= weight[0]
+        if (a.sgn_diff < 0.) {                           // mb -= div(D grad(mb))
+#pragma unroll
+            for (int p = 0; p < 7; p++) coef[p] += -1. * sc[p];
+            rhs += -1. * 0.;
+        } else {
+#pragma unroll
+            for (int p = 0; p < 7; p++) coef[p] += sc[p];
+        }
+    }
+
+    const int idx[3] = {i, jj, kk};
+#pragma unroll
+    for (int d = 0; d < DIM; d++) {                    // boundary folding
+        if (g.periodic[d] || !a.fold) continue;
+#pragma unroll
+        for (int side = 0; side < 2; side++) {
+            const int face = 2 * d + 1 + side;
+            const bool on_boundary = side == 0 ? (idx[d] == 0) : (idx[d] == g.n[d] - 1);
+            if (!on_boundary || (d == 0 && ((a.xint >> side) & 1))) continue;
+            const double X = coef[face];
+            if (a.bc_type[face - 1] == DARE_BC_DIRICHLET) {
+                coef[DARE_CENTER] -= X;
+                rhs -= 2. * a.bc_value[face - 1] * X;
+            } else {
+                coef[DARE_CENTER] += X;
+            }
+            coef[face] = 0.;
+        }
+    }
+}
+
 // Column-marching assembly: a thread owns one (j,k) column and walks along i
 // through `planes` planes, keeping phi(i-2..i+2) and the x-face velocity in
 // registers; addresses advance by constant strides (no per-cell index
@@ -97,7 +244,7 @@ __global__ void __launch_bounds__(256) k_assemble(GridDev g, AsmParams a, const 
     const int i1 = min(i0 + planes, n0);
     if (i0 >= i1) return;
     const int64_t n = a.dstride;
-    const int64_t S0 = (int64_t)g.gn[1] * g.gn[2], S1 = g.gn[2];
+    const int64_t S0 = (int64_t)g.gn[1] * g.gn[2];
     const int64_t nplane = (int64_t)n1 * n2;
     const int64_t jk = (int64_t)jj * n2 + kk;
     int64_t loc = local_index(g, i0, jj, kk);
@@ -120,134 +267,14 @@ __global__ void __launch_bounds__(256) k_assemble(GridDev g, AsmParams a, const 
         for (int p = 0; p < 7; p++) coef[p] = a.acc ? diag[p * n + c] : 0.;
         double rhs = a.acc ? rhs_out[c] : 0.;
 
-        if (a.dt > 0.) {                                   // DDT, weights (1, 1)
-            const double tt = a.tt;
-            if (a.sgn_ddt > 0.) {                           // from zero: C = tt, rhs = 0 + tt phi_old
-                coef[DARE_CENTER] += tt;
-                rhs += tt * phi_old[loc];
-            } else {                                        // MatrixBlock -=: += (-1 s)
-                coef[DARE_CENTER] += -1. * tt;
-                rhs += -1. * (tt * phi_old[loc]);
-            }
-        }
+        const AsmLine L{{w0, w1, w2, w3, w4},
+                        vx_lo,
+                        a.convection == 2 ? a.face_vel[0][fx_up] : 0.,
+                        Dx_lo,
+                        a.diffusion == 2 ? a.face_D[0][fx_up] : 0.,
+                        loc, fy_lo, fy_up, fz_lo, fz_up};
+        asm_cell<DIM>(g, a, L, phi, phi_old, i, jj, kk, coef, rhs);
 
-        if (a.convection) {                                // TVD * field, then divergence
-            double nb[7], cf[7], rr[7];
-#pragma unroll
-            for (int p = 0; p < 7; p++) nb[p] = cf[p] = rr[p] = 0.;
-            double vlo, vup;
-            // x (always active)
-            if (a.convection == 1) {
-                vlo = vup = a.vel[0];
-            } else {
-                vlo = vx_lo;
-                vup = a.face_vel[0][fx_up];
-            }
-            tvd_face(false, w0, w1, w2, w3, w4, vlo, a.limiter, nb[DARE_WEST], cf[DARE_WEST], rr[DARE_WEST]);
-            tvd_face(true, w0, w1, w2, w3, w4, vup, a.limiter, nb[DARE_EAST], cf[DARE_EAST], rr[DARE_EAST]);
-            if (DIM > 1) {
-                const double m2 = phi[loc - 2 * S1], m1 = phi[loc - S1], p1 = phi[loc + S1], p2 = phi[loc + 2 * S1];
-                if (a.convection == 1) {
-                    vlo = vup = a.vel[1];
-                } else {
-                    vlo = a.face_vel[1][fy_lo];
-                    vup = a.face_vel[1][fy_up];
-                }
-                tvd_face(false, m2, m1, w2, p1, p2, vlo, a.limiter, nb[DARE_SOUTH], cf[DARE_SOUTH], rr[DARE_SOUTH]);
-                tvd_face(true, m2, m1, w2, p1, p2, vup, a.limiter, nb[DARE_NORTH], cf[DARE_NORTH], rr[DARE_NORTH]);
-            }
-            if (DIM > 2) {
-                const double m2 = phi[loc - 2], m1 = phi[loc - 1], p1 = phi[loc + 1], p2 = phi[loc + 2];
-                if (a.convection == 1) {
-                    vlo = vup = a.vel[2];
-                } else {
-                    vlo = a.face_vel[2][fz_lo];
-                    vup = a.face_vel[2][fz_up];
-                }
-                tvd_face(false, m2, m1, w2, p1, p2, vlo, a.limiter, nb[DARE_BOTTOM], cf[DARE_BOTTOM], rr[DARE_BOTTOM]);
-                tvd_face(true, m2, m1, w2, p1, p2, vup, a.limiter, nb[DARE_TOP], cf[DARE_TOP], rr[DARE_TOP]);
-            }
-            double sc[7];
-            apply_divergence<DIM>(g, nb, cf, sc);
-#pragma unroll
-            for (int p = 0; p < 7; p++) sc[p] *= a.w[0];           // s_c *= weight[0]
-            double srhs = g.area[0] * (rr[DARE_EAST] - rr[DARE_WEST]);
-            if (DIM > 1) srhs += g.area[1] * (rr[DARE_NORTH] - rr[DARE_SOUTH]);
-            if (DIM > 2) srhs += g.area[2] * (rr[DARE_TOP] - rr[DARE_BOTTOM]);
-            for (int t = 1; t <= a.nexp; t++) {                // explicit levels (copies of level 0)
-                srhs += a.w[t] * g.area[0] * (rr[DARE_EAST] - rr[DARE_WEST]);
-                if (DIM > 1) srhs += a.w[t] * g.area[1] * (rr[DARE_NORTH] - rr[DARE_SOUTH]);
-                if (DIM > 2) srhs += a.w[t] * g.area[2] * (rr[DARE_TOP] - rr[DARE_BOTTOM]);
-            }
-            if (a.sgn_conv > 0.) {                           // MatrixBlock::Add
-#pragma unroll
-                for (int p = 0; p < 7; p++) coef[p] += sc[p];
-                rhs += srhs;
-            } else {                                        // MatrixBlock -=
-#pragma unroll
-                for (int p = 0; p < 7; p++) coef[p] += -1. * sc[p];
-                rhs += -1. * srhs;
-            }
-        }
-
-        if (a.diffusion) {                                 // mb -= div(D, grad(mb))
-            double Dlo[3], Dup[3];
-            if (a.diffusion == 1) {
-#pragma unroll
-                for (int d = 0; d < 3; d++) Dlo[d] = Dup[d] = a.D;
-            } else {
-                Dlo[0] = Dx_lo;
-                Dup[0] = a.face_D[0][fx_up];
-                Dlo[1] = DIM > 1 ? a.face_D[1][fy_lo] : 0.;
-                Dup[1] = DIM > 1 ? a.face_D[1][fy_up] : 0.;
-                Dlo[2] = DIM > 2 ? a.face_D[2][fz_lo] : 0.;
-                Dup[2] = DIM > 2 ? a.face_D[2][fz_up] : 0.;
-            }
-            double nb[7], cf[7];
-#pragma unroll
-            for (int p = 0; p < 7; p++) nb[p] = cf[p] = 0.;
-#pragma unroll
-            for (int d = 0; d < DIM; d++) {
-                const double dn = a.dn[d];
-                const int lo = 2 * d + 1, up = 2 * d + 2;
-                nb[lo] = (-dn) * Dlo[d];
-                cf[lo] = dn * Dlo[d];
-                nb[up] = dn * Dup[d];
-                cf[up] = (-dn) * Dup[d];
-            }
-            double sc[7];
-            apply_divergence<DIM>(g, nb, cf, sc);
-#pragma unroll
-            for (int p = 0; p < 7; p++) sc[p] *= a.w[0];           // s_c *= weight[0]
-            if (a.sgn_diff < 0.) {                           // mb -= div(D grad(mb))
-#pragma unroll
-                for (int p = 0; p < 7; p++) coef[p] += -1. * sc[p];
-                rhs += -1. * 0.;
-            } else {
-#pragma unroll
-                for (int p = 0; p < 7; p++) coef[p] += sc[p];
-            }
-        }
-
-        const int idx[3] = {i, jj, kk};
-#pragma unroll
-        for (int d = 0; d < DIM; d++) {                    // boundary folding
-            if (g.periodic[d] || !a.fold) continue;
-#pragma unroll
-            for (int side = 0; side < 2; side++) {
-                const int face = 2 * d + 1 + side;
-                const bool on_boundary = side == 0 ? (idx[d] == 0) : (idx[d] == g.n[d] - 1);
-                if (!on_boundary || (d == 0 && ((a.xint >> side) & 1))) continue;
-                const double X = coef[face];
-                if (a.bc_type[face - 1] == DARE_BC_DIRICHLET) {
-                    coef[DARE_CENTER] -= X;
-                    rhs -= 2. * a.bc_value[face - 1] * X;
-                } else {
-                    coef[DARE_CENTER] += X;
-                }
-                coef[face] = 0.;
-            }
-        }
 #pragma unroll
         for (int p = 0; p < 7; p++) diag[p * n + c] = coef[p];
         rhs_out[c] = rhs;
@@ -260,8 +287,8 @@ __global__ void __launch_bounds__(256) k_assemble(GridDev g, AsmParams a, const 
             w2 = w3;
             w3 = w4;
             w4 = phi[loc + 3 * S0];
-            if (a.convection == 2) vx_lo = a.face_vel[0][fx_up];
-            if (a.diffusion == 2) Dx_lo = a.face_D[0][fx_up];
+            if (a.convection == 2) vx_lo = L.vx_up;
+            if (a.diffusion == 2) Dx_lo = L.Dx_up;
         }
         loc += S0;
         c += nplane;
@@ -270,6 +297,103 @@ __global__ void __launch_bounds__(256) k_assemble(GridDev g, AsmParams a, const 
         fz_lo += fz_plane;
         fz_up += fz_plane;
     }
+}
+
+// A whole composed functor on a 1-D or 2-D grid in one launch: each thread takes
+// one cell of one component through the terms in order, its coefficients in
+// registers where the launches one by one (two species of DDT, convection and
+// diffusion: eight of 5 us on 96 x 80 cells) pass them through memory.
+constexpr int kFusedTerms = 8, kFusedComps = 4;
+struct FusedTerm {
+    AsmParams a;              // acc: added to what is there (otherwise it starts the block afresh)
+    const double *coef[7], *coef_rhs;
+    double sgn;
+    int component, is_coef;
+};
+struct FusedTerms {
+    int n;
+    FusedTerm t[kFusedTerms];
+    AsmParams fold;                              // the last pass ...
+    int bc_type[kFusedComps][6];                 // ... with each component's conditions
+    double bc_value[kFusedComps][6];
+};
+template <int DIM>
+__global__ void __launch_bounds__(128) k_assemble_terms(GridDev g, const __grid_constant__ FusedTerms F,
+                                                        const double* __restrict__ phi_all,
+                                                        const double* __restrict__ old_all, double* __restrict__ diag,
+                                                        double* __restrict__ rhs_out, double* __restrict__ x0,
+                                                        int64_t dstride) {
+    const int comp = blockIdx.y;
+    const double* phi = phi_all + (size_t)comp * g.ncell_ghosted;
+    const double* old = old_all + (size_t)comp * g.ncell_ghosted;
+    const int64_t cell = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (cell >= g.ncell) return;
+    const int n1 = g.n[1], n2 = g.n[2];
+    const int64_t plane = (int64_t)n1 * n2, S0 = (int64_t)g.gn[1] * g.gn[2];
+    const int i = (int)(cell / plane), rem = (int)(cell - (int64_t)i * plane), j = rem / n2, k = rem - j * n2;
+    AsmLine L{};
+    L.loc = local_index(g, i, j, k);
+#pragma unroll
+    for (int q = 0; q < 5; q++) L.w[q] = phi[L.loc + (q - 2) * S0];
+    L.fy_lo = (int64_t)i * (n1 + 1) * n2 + (int64_t)j * n2 + k;
+    L.fy_up = (int64_t)i * (n1 + 1) * n2 + (int64_t)upper_face(g, 1, j) * n2 + k;
+    L.fz_lo = ((int64_t)i * n1 + j) * (n2 + 1) + k;
+    L.fz_up = ((int64_t)i * n1 + j) * (n2 + 1) + upper_face(g, 2, k);
+    const int64_t fx_lo = cell, fx_up = (int64_t)upper_face(g, 0, i) * plane + rem;
+    double coef[7] = {0., 0., 0., 0., 0., 0., 0.}, rhs = 0.;
+    for (int t = 0; t < F.n; t++) {
+        const FusedTerm& T = F.t[t];
+        if (T.component >= 0 && T.component != comp) continue;
+        if (T.is_coef) {
+#pragma unroll
+            for (int q = 0; q < 7; q++) {
+                const double v = T.coef[q] ? T.coef[q][cell] : 0.;
+                const double sv = T.sgn > 0. ? v : -1. * v;
+                coef[q] = T.a.acc ? coef[q] + sv : sv;
+            }
+            const double v = T.coef_rhs ? T.coef_rhs[cell] : 0.;
+            const double sv = T.sgn > 0. ? v : -1. * v;
+            rhs = T.a.acc ? rhs + sv : sv;
+            continue;
+        }
+        if (!T.a.acc) {
+#pragma unroll
+            for (int q = 0; q < 7; q++) coef[q] = 0.;
+            rhs = 0.;
+        }
+        if (T.a.convection == 2) {
+            L.vx_lo = T.a.face_vel[0][fx_lo];
+            L.vx_up = T.a.face_vel[0][fx_up];
+        }
+        if (T.a.diffusion == 2) {
+            L.Dx_lo = T.a.face_D[0][fx_lo];
+            L.Dx_up = T.a.face_D[0][fx_up];
+        }
+        asm_cell<DIM>(g, T.a, L, phi, old, i, j, k, coef, rhs);
+    }
+    const int idx[3] = {i, j, k};
+#pragma unroll
+    for (int d = 0; d < DIM; d++) {
+        if (g.periodic[d]) continue;
+#pragma unroll
+        for (int side = 0; side < 2; side++) {
+            const int face = 2 * d + 1 + side;
+            if (idx[d] != (side == 0 ? 0 : g.n[d] - 1) || (d == 0 && ((F.fold.xint >> side) & 1))) continue;
+            const double X = coef[face];
+            if (F.bc_type[comp][face - 1] == DARE_BC_DIRICHLET) {
+                coef[DARE_CENTER] -= X;
+                rhs -= 2. * F.bc_value[comp][face - 1] * X;
+            } else {
+                coef[DARE_CENTER] += X;
+            }
+            coef[face] = 0.;
+        }
+    }
+    const int64_t c = (int64_t)comp * g.ncell + cell;
+#pragma unroll
+    for (int q = 0; q < 7; q++) diag[q * dstride + c] = coef[q];
+    rhs_out[c] = rhs;
+    x0[c] = L.w[2];
 }
 
 // The conditions on the boundary faces of component c
@@ -418,6 +542,80 @@ static int launch_terms(dare_system* s, const dare_term* terms, int nterms, cons
             return set_error(ctx, DARE_ERR_BAD_ARG, "dare_assemble_terms: DDT needs dt > 0");
     }
     int rc;
+    // one term's parameters, before its place among the others is known
+    const auto term_params = [](const dare_term& T) {
+        AsmParams a{};
+        a.scheme = T.scheme;
+        a.limiter = T.limiter;
+        const double sgn = T.op == DARE_OP_SUB ? -1. : 1.;
+        a.sgn_ddt = a.sgn_conv = a.sgn_diff = sgn;
+        if (T.kind == DARE_TERM_DDT) a.dt = T.dt;
+        if (T.kind == DARE_TERM_DIFFUSION) {
+            const bool faces = T.face_D[0] || T.face_D[1] || T.face_D[2];
+            a.diffusion = faces ? 2 : 1;
+            a.D = T.D;
+            for (int d = 0; d < 3; d++) a.face_D[d] = T.face_D[d];
+        }
+        if (T.kind == DARE_TERM_CONVECTION) {
+            const bool faces = T.face_vel[0] || T.face_vel[1] || T.face_vel[2];
+            a.convection = faces ? 2 : 1;
+            for (int d = 0; d < 3; d++) {
+                a.vel[d] = T.vel[d];
+                a.face_vel[d] = T.face_vel[d];
+            }
+        }
+        a.fold = 0;
+        return a;
+    };
+    // 1-D and 2-D grids: everything in one launch, where the list fits one
+    // (a component that no term touches is zeroed by the fold pass below)
+    const GridDev& g = s->grid->dev;
+    if (g.dim < 3 && nterms <= kFusedTerms && s->ncomp <= kFusedComps) {
+        FusedTerms F{};
+        bool started[kFusedComps] = {false, false, false, false};
+        bool fits = true;
+        for (int t = 0; t < nterms; t++) {
+            const dare_term& T = terms[t];
+            FusedTerm& f = F.t[F.n++];
+            f.component = T.component;
+            f.is_coef = T.kind == DARE_TERM_COEFFS;
+            f.sgn = T.op == DARE_OP_SUB ? -1. : 1.;
+            for (int q = 0; q < 7; q++) f.coef[q] = T.coef[q];
+            f.coef_rhs = T.coef_rhs;
+            if (!f.is_coef) {
+                f.a = term_params(T);
+                if ((rc = base_params(s, f.a, "dare_assemble_terms"))) return rc;
+            }
+            // whether it adds must be the same for every component it is for
+            int adds = -1;
+            for (int c = 0; c < s->ncomp; c++) {
+                if (T.component >= 0 && T.component != c) continue;
+                const int add = started[c] && T.op != DARE_OP_SET;
+                fits = fits && (adds < 0 || adds == add);
+                adds = add;
+                started[c] = true;
+            }
+            f.a.acc = adds;
+        }
+        for (int c = 0; c < s->ncomp; c++) {
+            AsmParams a{};
+            component_bc(s, c, a);
+            for (int q = 0; q < 6; q++) {
+                F.bc_type[c][q] = a.bc_type[q];
+                F.bc_value[c][q] = a.bc_value[q];
+            }
+        }
+        F.fold.xint = s->xint;
+        if (fits) {
+            const dim3 grid((unsigned)((g.ncell + 127) / 128), (unsigned)s->ncomp);
+            if (g.dim == 2)
+                k_assemble_terms<2><<<grid, 128, 0, ctx->stream>>>(g, F, phi, phi_old, s->diag, s->rhs, s->x, s->sdev.ncell);
+            else
+                k_assemble_terms<1><<<grid, 128, 0, ctx->stream>>>(g, F, phi, phi_old, s->diag, s->rhs, s->x, s->sdev.ncell);
+            DARE_LAUNCHED(ctx);
+            return DARE_OK;
+        }
+    }
     for (int c = 0; c < s->ncomp; c++) {
         bool started = false;
         for (int t = 0; t < nterms; t++) {
@@ -427,36 +625,15 @@ static int launch_terms(dare_system* s, const dare_term* terms, int nterms, cons
                 CoefTerm ct{};
                 for (int q = 0; q < 7; q++) ct.coef[q] = T.coef[q];
                 ct.rhs = T.coef_rhs;
-                const GridDev& gd = s->grid->dev;
-                k_term_coeffs<<<grid_blocks(ctx, gd.ncell, 256, 8), 256, 0, ctx->stream>>>(
-                    gd.ncell, s->sdev.ncell, ct, T.op == DARE_OP_SUB ? -1. : 1., started && T.op != DARE_OP_SET,
-                    s->diag + (size_t)c * gd.ncell, s->rhs + (size_t)c * gd.ncell);
+                k_term_coeffs<<<grid_blocks(ctx, g.ncell, 256, 8), 256, 0, ctx->stream>>>(
+                    g.ncell, s->sdev.ncell, ct, T.op == DARE_OP_SUB ? -1. : 1., started && T.op != DARE_OP_SET,
+                    s->diag + (size_t)c * g.ncell, s->rhs + (size_t)c * g.ncell);
                 DARE_LAUNCHED(ctx);
                 started = true;
                 continue;
             }
-            AsmParams a{};
-            a.scheme = T.scheme;
-            a.limiter = T.limiter;
-            const double sgn = T.op == DARE_OP_SUB ? -1. : 1.;
-            a.sgn_ddt = a.sgn_conv = a.sgn_diff = sgn;
-            if (T.kind == DARE_TERM_DDT) a.dt = T.dt;
-            if (T.kind == DARE_TERM_DIFFUSION) {
-                const bool faces = T.face_D[0] || T.face_D[1] || T.face_D[2];
-                a.diffusion = faces ? 2 : 1;
-                a.D = T.D;
-                for (int d = 0; d < 3; d++) a.face_D[d] = T.face_D[d];
-            }
-            if (T.kind == DARE_TERM_CONVECTION) {
-                const bool faces = T.face_vel[0] || T.face_vel[1] || T.face_vel[2];
-                a.convection = faces ? 2 : 1;
-                for (int d = 0; d < 3; d++) {
-                    a.vel[d] = T.vel[d];
-                    a.face_vel[d] = T.face_vel[d];
-                }
-            }
+            AsmParams a = term_params(T);
             a.acc = started && T.op != DARE_OP_SET;   // Set starts the component's block afresh
-            a.fold = 0;
             if ((rc = base_params(s, a, "dare_assemble_terms"))) return rc;
             component_bc(s, c, a);
             if ((rc = launch_component(s, a, c, phi, phi_old))) return rc;

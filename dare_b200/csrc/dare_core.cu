@@ -23,9 +23,14 @@ int check_cuda(dare_ctx* ctx, cudaError_t e, const char* what) {
 
 // ---- kernels ---------------------------------------------------------------
 
-// Periodic face-ghost fill along dimension d (HaloBuffer self-exchange on one
-// rank; only ghosts outside the internal range in exactly this dimension).
-__global__ void k_halo_fill(GridDev g, int d, double* __restrict__ phi) {
+// Periodic face-ghost fill (HaloBuffer self-exchange on one rank; only ghosts
+// outside the internal range in exactly one dimension): dimension blockIdx.z of
+// component blockIdx.y.  Ghosts are written and internal cells read, so the
+// dimensions need no order.
+__global__ void k_halo_fill(GridDev g, double* __restrict__ phi) {
+    const int d = blockIdx.z;
+    if (!g.periodic[d]) return;
+    phi += (int64_t)blockIdx.y * g.ncell_ghosted;
     const int e1 = d == 0 ? 1 : 0;
     const int e2 = d == 2 ? 1 : 2;
     const int64_t n1 = g.n[e1], n2 = g.n[e2];
@@ -53,8 +58,10 @@ __global__ void k_halo_fill(GridDev g, int d, double* __restrict__ phi) {
     }
 }
 
-// x (internal) -> field (ghosted): Trilinos::CopyTo
+// x (internal) -> field (ghosted), component blockIdx.y: Trilinos::CopyTo
 __global__ void k_scatter_to_field(GridDev g, const double* __restrict__ x, double* __restrict__ phi) {
+    x += (int64_t)blockIdx.y * g.ncell;
+    phi += (int64_t)blockIdx.y * g.ncell_ghosted;
     const int64_t nyz = (int64_t)g.n[1] * g.n[2];
     for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < g.ncell;
          c += (int64_t)gridDim.x * blockDim.x) {
@@ -151,9 +158,9 @@ int launch_gather(dare_ctx* ctx, const GridDev& g, const double* phi, double* x)
     return DARE_OK;
 }
 
-int launch_scatter(dare_ctx* ctx, const GridDev& g, const double* x, double* phi) {
+int launch_scatter(dare_ctx* ctx, const GridDev& g, int ncomp, const double* x, double* phi) {
     int blocks = grid_blocks(ctx, g.ncell, 256, 8);
-    k_scatter_to_field<<<blocks, 256, 0, ctx->stream>>>(g, x, phi);
+    k_scatter_to_field<<<dim3(blocks, ncomp), 256, 0, ctx->stream>>>(g, x, phi);
     DARE_LAUNCHED(ctx);
     return DARE_OK;
 }
@@ -182,15 +189,17 @@ int launch_solution_to_field(dare_ctx* ctx, const GridDev& g, const double* invd
     return DARE_OK;
 }
 
-int launch_halo(dare_ctx* ctx, const GridDev& g, double* phi) {
+int launch_halo(dare_ctx* ctx, const GridDev& g, int ncomp, double* phi) {
+    int64_t most = 0;
     for (int d = 0; d < g.dim; d++) {
         if (!g.periodic[d]) continue;
         const int e1 = d == 0 ? 1 : 0, e2 = d == 2 ? 1 : 2;
         const int64_t total = (int64_t)2 * g.ng * g.n[e1] * g.n[e2];
-        int blocks = grid_blocks(ctx, total, 256, 8);
-        k_halo_fill<<<blocks, 256, 0, ctx->stream>>>(g, d, phi);
-        DARE_LAUNCHED(ctx);
+        if (total > most) most = total;
     }
+    if (!most) return DARE_OK;
+    k_halo_fill<<<dim3(grid_blocks(ctx, most, 256, 8), ncomp, g.dim), 256, 0, ctx->stream>>>(g, phi);
+    DARE_LAUNCHED(ctx);
     return DARE_OK;
 }
 
@@ -425,11 +434,7 @@ double* dare_field_device_ptr(dare_field* f, int level) {
 
 int dare_field_exchange_halo(dare_field* f) {
     if (!f) return DARE_ERR_BAD_ARG;
-    for (int c = 0; c < f->ncomp; c++) {
-        const int rc = launch_halo(f->grid->ctx, f->grid->dev, f->level[0] + (size_t)c * f->grid->dev.ncell_ghosted);
-        if (rc) return rc;
-    }
-    return DARE_OK;
+    return launch_halo(f->grid->ctx, f->grid->dev, f->ncomp, f->level[0]);
 }
 
 int dare_field_copy_to_old(dare_field* f) {
@@ -674,12 +679,7 @@ int dare_system_export_csr(dare_system* s, int64_t* rowptr, int64_t* cols, doubl
 
 int dare_system_copy_to(dare_system* s, dare_field* f) {
     if (!s || !f || f->grid != s->grid || f->ncomp != s->ncomp) return DARE_ERR_BAD_ARG;
-    const GridDev& g = s->grid->dev;
-    for (int c = 0; c < s->ncomp; c++) {
-        const int rc = launch_scatter(s->grid->ctx, g, s->x + (size_t)c * g.ncell, f->level[0] + (size_t)c * g.ncell_ghosted);
-        if (rc) return rc;
-    }
-    return DARE_OK;
+    return launch_scatter(s->grid->ctx, s->grid->dev, s->ncomp, s->x, f->level[0]);
 }
 
 int dare_face_average(dare_grid* gr, const double* cell_D, double* face_D[3]) {

@@ -15,8 +15,6 @@ namespace dare_gpu {
 int launch_assemble(dare_system* s, const dare_assembly_desc* desc, const double* phi, const double* phi_old);
 int launch_assemble_planes(dare_system* s, const dare_assembly_desc* desc, const double* phi, const double* phi_old,
                            int ib, int ie);
-int launch_scatter(dare_ctx* ctx, const GridDev& g, const double* x, double* phi);
-int launch_halo(dare_ctx* ctx, const GridDev& g, double* phi);
 }  // namespace dare_gpu
 
 extern "C" {
