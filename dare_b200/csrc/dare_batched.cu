@@ -426,25 +426,42 @@ struct BoxOp {
     const unsigned char* faces;       // boundary mask of each tile cell
     int t0, tn, c0, m;                // first cell and cells of the tile, of the block
 
+    // (two cells a thread at a time, their loads together: the L2 latency is
+    // what a pass waits for; four spill the 64 registers a thread)
     template <class ZF, class Pre, class Body>
     __device__ __forceinline__ void pass(ZF zf, Pre pre, Body body) const {
-        const int tid = threadIdx.x, nt = blockDim.x;
-#pragma unroll 4
-        for (int e = tid; e < tn; e += nt) tile[e] = invd[faces[e]] * zf(t0 + e);
+        constexpr int G = 2;
+        const int nt = blockDim.x;
+        for (int e0 = threadIdx.x; e0 < tn; e0 += G * nt) {
+            double z[G];
+#pragma unroll
+            for (int q = 0; q < G; q++)
+                if (e0 + q * nt < tn) z[q] = zf(t0 + e0 + q * nt);
+#pragma unroll
+            for (int q = 0; q < G; q++)
+                if (e0 + q * nt < tn) tile[e0 + q * nt] = invd[faces[e0 + q * nt]] * z[q];
+        }
         __syncthreads();
-#pragma unroll 2
-        for (int lc = tid; lc < m; lc += nt) {
-            const int c = c0 + lc, e = c - t0;
-            const unsigned f = faces[e];
-            const double* t = tile + e;
-            const double w = f & 1u ? 0. : t[-sx], ea = f & 2u ? 0. : t[sx];
-            const double so = f & 4u ? 0. : t[-sy], no = f & 8u ? 0. : t[sy];
-            const double bo = f & 16u ? 0. : t[-1], to = f & 32u ? 0. : t[1];
-            const double z0 = C[f] * t[0];
-            double y = z0 + off0 * (w + ea);
-            y += off1 * (so + no);
-            y += off2 * (bo + to);
-            body(c, y, z0, pre(c));
+        for (int l0 = threadIdx.x; l0 < m; l0 += G * nt) {
+            double p[G];
+#pragma unroll
+            for (int q = 0; q < G; q++)
+                if (l0 + q * nt < m) p[q] = pre(c0 + l0 + q * nt);
+#pragma unroll
+            for (int q = 0; q < G; q++) {
+                if (l0 + q * nt >= m) break;
+                const int c = c0 + l0 + q * nt, e = c - t0;
+                const unsigned f = faces[e];
+                const double* t = tile + e;
+                const double w = f & 1u ? 0. : t[-sx], ea = f & 2u ? 0. : t[sx];
+                const double so = f & 4u ? 0. : t[-sy], no = f & 8u ? 0. : t[sy];
+                const double bo = f & 16u ? 0. : t[-1], to = f & 32u ? 0. : t[1];
+                const double z0 = C[f] * t[0];
+                double y = z0 + off0 * (w + ea);
+                y += off1 * (so + no);
+                y += off2 * (bo + to);
+                body(c, y, z0, p[q]);
+            }
         }
     }
     template <int U, class Body>
@@ -714,21 +731,13 @@ static int upload_instances(dare_batch* bt) {
     return DARE_OK;
 }
 
-static int launch_class(dare_batch* bt, int c, const BVecs& vs, const BParams& prm, int block, cudaStream_t sm) {
+static int launch_boxes(dare_batch* bt, int c, const BVecs& vs, const BParams& prm, int block, cudaStream_t sm) {
     dare_ctx* ctx = bt->ctx;
     const int first = bt->class_at[c], count = bt->class_at[c + 1] - first;
-    if (c == kBoxClasses) {
-        int per_sm = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batched, block, 0);
-        const int blocks = std::min(std::max(per_sm, 1) * ctx->num_sms, count);
-        k_batched<<<blocks, block, 0, sm>>>(bt->d_inst, bt->d_order + first, count, vs, prm, bt->d_out,
-                                            bt->d_queue + c);
-        DARE_LAUNCHED(ctx);
-        return DARE_OK;
-    }
+    const auto kern = k_boxes;
     const size_t smem = bt->class_smem[c];
-    DARE_CUDA(ctx, cudaFuncSetAttribute(k_boxes, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBoxSmem));
-    DARE_CUDA(ctx, cudaFuncSetAttribute(k_boxes, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    DARE_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBoxSmem));
+    DARE_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = 1u << c;
@@ -740,18 +749,35 @@ static int launch_class(dare_batch* bt, int c, const BVecs& vs, const BParams& p
     cfg.attrs = at;
     cfg.numAttrs = 1;
     cfg.gridDim = dim3(ctx->num_sms / (1 << c) * (1 << c));
+    int& clusters = bt->class_clusters[c];
+    if (!clusters) DARE_CUDA(ctx, cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg));
+    if (clusters < 1) return set_error(ctx, DARE_ERR_UNSUPPORTED, "dare_batch: a cluster does not fit the device");
+    cfg.gridDim = dim3((unsigned)std::min(clusters, count) << c);
+    DARE_CUDA(ctx, cudaLaunchKernelEx(&cfg, kern, (const BInst*)bt->d_inst, (const int*)(bt->d_order + first), count,
+                                      vs, prm, bt->d_out, bt->d_queue + c, (int)(smem / (sizeof(double) + 1))));
+    DARE_LAUNCHED(ctx);
+    return DARE_OK;
+}
+
+static int launch_class(dare_batch* bt, int c, const BVecs& vs, const BParams& prm, int block, cudaStream_t sm) {
+    dare_ctx* ctx = bt->ctx;
+    if (c == kBoxClasses) {
+        const int first = bt->class_at[c], count = bt->class_at[c + 1] - first;
+        int per_sm = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batched, block, 0);
+        const int blocks = std::min(std::max(per_sm, 1) * ctx->num_sms, count);
+        k_batched<<<blocks, block, 0, sm>>>(bt->d_inst, bt->d_order + first, count, vs, prm, bt->d_out,
+                                            bt->d_queue + c);
+        DARE_LAUNCHED(ctx);
+        return DARE_OK;
+    }
     if (bt->clusters_block != block) {
         std::fill(bt->class_clusters, bt->class_clusters + kBoxClasses, 0);
         bt->clusters_block = block;
     }
-    int& clusters = bt->class_clusters[c];
-    if (!clusters) DARE_CUDA(ctx, cudaOccupancyMaxActiveClusters(&clusters, k_boxes, &cfg));
-    if (clusters < 1) return set_error(ctx, DARE_ERR_UNSUPPORTED, "dare_batch: a cluster does not fit the device");
-    cfg.gridDim = dim3((unsigned)std::min(clusters, count) << c);
-    DARE_CUDA(ctx, cudaLaunchKernelEx(&cfg, k_boxes, (const BInst*)bt->d_inst, (const int*)(bt->d_order + first), count,
-                                      vs, prm, bt->d_out, bt->d_queue + c, (int)(smem / (sizeof(double) + 1))));
-    DARE_LAUNCHED(ctx);
-    return DARE_OK;
+    // (clusters of four and more leave one block an SM: it takes all the threads
+    // there are; 64^3 boxes 5.8 ms for 128, 8.5 with 512 threads a block)
+    return launch_boxes(bt, c, vs, prm, c >= 2 ? 1024 : block, sm);
 }
 
 // All classes at the same time: the largest clusters on the context's stream,
@@ -933,9 +959,9 @@ int dare_batch_solve(dare_batch* bt, const dare_solver_params* p, dare_batch_rep
     return DARE_OK;
 }
 
-// Tunes (1) cells per thread per sweep for each size class, from single-class
-// sub-batches, and (2) the block size for the whole batch, by timing solves
-// of copies of the current fields (restored afterwards).
+// Tunes the block size for the whole batch and the cells a block takes (1, 2 or
+// 4 times 4096) for each size class, by timing solves of copies of the current
+// fields (restored afterwards).
 int dare_batch_autotune(dare_batch* bt, const dare_solver_params* p, int* chosen_block) {
     using namespace dare_gpu;
     if (!bt || !p) return DARE_ERR_BAD_ARG;
@@ -949,9 +975,12 @@ int dare_batch_autotune(dare_batch* bt, const dare_solver_params* p, int* chosen
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
     auto timed = [&](int block) -> double {
-        cudaMemcpyAsync(bt->arena, saved, bytes, cudaMemcpyDeviceToDevice, ctx->stream);
-        cudaEventRecord(e0, ctx->stream);
-        if (launch_batch(bt, p, block)) return 1e30;
+        // the second of two: the first asks for the setting's occupancy
+        for (int k = 0; k < 2; k++) {
+            cudaMemcpyAsync(bt->arena, saved, bytes, cudaMemcpyDeviceToDevice, ctx->stream);
+            cudaEventRecord(e0, ctx->stream);
+            if (launch_batch(bt, p, block)) return 1e30;
+        }
         cudaEventRecord(e1, ctx->stream);
         cudaEventSynchronize(e1);
         float ms = 0.f;
@@ -960,7 +989,7 @@ int dare_batch_autotune(dare_batch* bt, const dare_solver_params* p, int* chosen
     };
     static const int blocks[3] = {256, 512, 1024};
     static const int vecs[3] = {1, 2, 4};
-    int best_block = bt->block;
+    int best_block = bt->block, base_vec = bt->vec_by_size[0];
     double best_t = 1e30;
     for (int bi = 0; bi < 3; bi++) {
         // per size class: pick cells per thread with all instances at that setting
@@ -971,12 +1000,11 @@ int dare_batch_autotune(dare_batch* bt, const dare_solver_params* p, int* chosen
             if (tm < best_t) {
                 best_t = tm;
                 best_block = blocks[bi];
-                for (int c = 0; c < 8; c++) bt->vec_by_size[c] = vecs[vi];
+                base_vec = vecs[vi];
             }
         }
     }
     // keep the best uniform setting, then refine each size class separately
-    int base_vec = bt->vec_by_size[0];
     for (int c = 0; c < 8; c++) bt->vec_by_size[c] = base_vec;
     for (int c = 0; c < 8; c++) {
         bool present = false;

@@ -378,7 +378,8 @@ DARE_API int dare_face_average(dare_grid* g, const double* cell_D, double* face_
  * (DDT + div(D grad), Dirichlet/Neumann folding per face: the functor of
  * test/Verification/counter_diffusion1D.cpp:113-146 in 3D), each solved by
  * Jacobi-BiCGStab(2) (BiCGStab2.inl:166-582) with its own tolerance check and
- * status, all in one persistent launch.  Fields are internal cells,
+ * status, all in persistent launches side by side, one per number of blocks a
+ * box takes.  Fields are internal cells,
  * ordinal (i*ny + j)*nz + k; the field is the initial guess and phi_old. */
 typedef struct {
     int64_t n[3];          /* cells per dimension (>= 3 each) */
@@ -410,8 +411,9 @@ DARE_API int dare_batch_zero_fields(dare_batch* bt);
 /* Solves every instance (p: tol, tol_relative, max_it; Jacobi, FP64). The
  * fields are replaced by the solutions; reports (host, count entries) may be NULL. */
 DARE_API int dare_batch_solve(dare_batch* bt, const dare_solver_params* p, dare_batch_report* reports);
-/* Picks the block size and the cells each thread handles per sweep (per size
- * class) by timing solves of the current fields, which are restored. */
+/* Picks the block size and the cells a thread handles (1, 2 or 4, relative, per
+ * size class: a box goes to as few blocks of at most 4096 times that many cells
+ * as it needs) by timing solves of the current fields, which are restored. */
 DARE_API int dare_batch_autotune(dare_batch* bt, const dare_solver_params* p, int* chosen_block);
 DARE_API int dare_batch_get_tuning(const dare_batch* bt, int* block, int vec_by_size[8]);
 
