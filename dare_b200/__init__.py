@@ -21,6 +21,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import struct
 from dataclasses import dataclass
 
 import numpy as np
@@ -217,6 +218,10 @@ class BatchInstance(C.Structure):
 class BatchReport(C.Structure):
     _fields_ = [("iters", C.c_int), ("converged", C.c_int), ("status", C.c_int), ("breakdown_step", C.c_int),
                 ("res_abs", C.c_double), ("b_norm", C.c_double), ("tol_abs", C.c_double)]
+
+
+_BATCH_REPORT = struct.Struct("@iiiiddd")   # BatchReport's layout
+assert _BATCH_REPORT.size == C.sizeof(BatchReport)
 
 _lib = None
 
@@ -806,7 +811,7 @@ def face_average(grid: Grid, cell_D_ptr: int, face_ptrs) -> None:
 
 
 class Batch:
-    """Many independent implicit diffusion steps solved in one persistent launch.
+    """Many independent implicit diffusion steps solved in persistent launches side by side.
 
     ``instances``: dicts with ``n`` (3 ints), ``size`` (3 floats), ``D``, ``dt``,
     ``bc`` = {face: (kind, value)} for faces WEST..TOP (Dirichlet/Neumann).
@@ -847,7 +852,7 @@ class Batch:
 
     def get_field(self, idx: int) -> np.ndarray:
         a = np.empty(self.num_cells(idx), dtype=np.float64)
-        _check(lib().dare_batch_get_field(self.h, idx, _ptr(a)), self.ctx.h, "batch_get_field")
+        _check(lib().dare_batch_get_field(self.h, idx, a.ctypes.data), self.ctx.h, "batch_get_field")
         return a
 
     def zero_fields(self):
@@ -858,9 +863,11 @@ class Batch:
         _check(lib().dare_batch_solve(self.h, C.byref(solver.params), rep), self.ctx.h, "batch_solve")
         if not reports:
             return None
-        return [{"iters": r.iters, "converged": bool(r.converged), "status": SOLVE_STATUS.get(r.status, r.status),
-                 "breakdown_step": r.breakdown_step, "res_abs": r.res_abs, "b_norm": r.b_norm, "tol_abs": r.tol_abs}
-                for r in rep]
+        # unpacked in one go: field by field through ctypes the dicts of 1024
+        # boxes took 0.45 ms, as long as their solve
+        return [{"iters": it, "converged": bool(ok), "status": SOLVE_STATUS.get(st, st), "breakdown_step": step,
+                 "res_abs": res, "b_norm": bn, "tol_abs": tol}
+                for it, ok, st, step, res, bn, tol in _BATCH_REPORT.iter_unpack(rep)]
 
     def autotune(self, solver: "BiCGStab2") -> dict:
         blk = C.c_int()
