@@ -29,7 +29,8 @@
 //
 // One inner iteration is one CUDA graph: 4 network applications (13
 // tensor-core/level-transfer kernels each), 4 SpMV kernels with fused dot
-// products (plane-marching, dare_march.cuh), 6 vector kernels.  The FP64
+// products (plane-marching, dare_march.cuh), 5 vector kernels, four of them with
+// the coarse form's restriction.  The FP64
 // residual of the refinement also runs in the marching engine and is read
 // back with the inner solve's state.
 // The inner solve may stop after its first iteration (the reference's
@@ -208,7 +209,16 @@ __device__ __forceinline__ float4 axmy(float4 a, float c, float4 b) {
     return make_float4(a.x - c * b.x, a.y - c * b.y, a.z - c * b.z, a.w - c * b.w);
 }
 
-// start of an inner solve: r = rh = rin, u = v = w = d = 0
+// (3), (4) given rho1 = <rh, r>: beta
+__device__ __forceinline__ void next_rho(SolverState* st, double rho1) {
+    st->rho0 = -st->omega2 * st->rho0;
+    if (st->rho0 == 0.) return fail(st, 3);
+    st->beta = st->alpha * rho1 / st->rho0;
+    st->rho0 = rho1;
+    if (st->rho0 == 0.) fail(st, 4);
+}
+
+// start of an inner solve: r = rh = rin, u = v = w = d = 0; (3), (4)
 __global__ void __launch_bounds__(256) k_init(int64_t n, Vecs vs, SolverState* st, double* partials, double rel_tol,
                                               int max_it) {
     double acc[1] = {0.};
@@ -242,71 +252,75 @@ __global__ void __launch_bounds__(256) k_init(int64_t n, Vecs vs, SolverState* s
             st->done = 1;
             st->status = ST_NAN;
         }
+        if (!st->done) next_rho(st, tot[0]);   // <rh, r> = <r, r>
     }
 }
 
-// (3), (4): rho1 = <rh, r>, beta
-__global__ void __launch_bounds__(256) k_rho(int64_t n, Vecs vs, SolverState* st, double* partials) {
-    pdl_wait();
-    pdl_launch();
-    if (st->done) return;
-    double acc[1] = {0.};
-    GRID_LOOP(q, n / 4) acc[0] += dot4(ld4(vs.rh, q), ld4(vs.r, q));
-    double tot[1];
-    if (!grid_reduce<1>(acc, partials, &st->count, tot)) return;
-    if (threadIdx.x == 0) {
-        st->rho0 = -st->omega2 * st->rho0;
-        if (st->rho0 == 0.) return fail(st, 3);
-        const double rho1 = tot[0];
-        st->beta = st->alpha * rho1 / st->rho0;
-        st->rho0 = rho1;
-        if (st->rho0 == 0.) return fail(st, 4);
+// The vector update before each application of the network: (5) u = r - beta u;
+// (8) r -= alpha v (the matching x update is folded into k_upd_final); (12) v =
+// s - beta v; (15)-(17) u, r and s.  The last vector updated is what the network
+// is applied to.
+enum : int { UPD_U = 0, UPD_R = 1, UPD_V = 2, UPD_S = 3 };
+template <int MODE>
+__device__ __forceinline__ float4 update4(const Vecs& vs, int64_t q, float alpha, float beta) {
+    float4 o;
+    if constexpr (MODE == UPD_U) {
+        o = axmy(ld4(vs.r, q), beta, ld4(vs.u, q));
+        st4(vs.u, q, o);
+    } else if constexpr (MODE == UPD_R) {
+        o = axmy(ld4(vs.r, q), alpha, ld4(vs.v, q));
+        st4(vs.r, q, o);
+    } else if constexpr (MODE == UPD_V) {
+        o = axmy(ld4(vs.s, q), beta, ld4(vs.v, q));
+        st4(vs.v, q, o);
+    } else {
+        const float4 r = ld4(vs.r, q);
+        st4(vs.u, q, axmy(r, beta, ld4(vs.u, q)));
+        st4(vs.r, q, axmy(r, alpha, ld4(vs.v, q)));
+        o = axmy(ld4(vs.s, q), alpha, ld4(vs.w, q));
+        st4(vs.s, q, o);
     }
+    return o;
 }
-
-// (5) u = r - beta u
-__global__ void k_upd_u(int64_t n, Vecs vs, const SolverState* st) {
-    pdl_wait();
-    pdl_launch();
-    if (st->done) return;
-    const float beta = (float)st->beta;
-    GRID_LOOP(q, n / 4) st4(vs.u, q, axmy(ld4(vs.r, q), beta, ld4(vs.u, q)));
-}
-
-// (8): r -= alpha v (the matching x update is folded into k_upd_final)
-__global__ void k_upd_r(int64_t n, Vecs vs, const SolverState* st) {
-    pdl_wait();
-    pdl_launch();
-    if (st->done) return;
-    const float alpha = (float)st->alpha;
-    GRID_LOOP(q, n / 4) st4(vs.r, q, axmy(ld4(vs.r, q), alpha, ld4(vs.v, q)));
-}
-
-// (12) v = s - beta v
-__global__ void k_upd_v(int64_t n, Vecs vs, const SolverState* st) {
-    pdl_wait();
-    pdl_launch();
-    if (st->done) return;
-    const float beta = (float)st->beta;
-    GRID_LOOP(q, n / 4) st4(vs.v, q, axmy(ld4(vs.s, q), beta, ld4(vs.v, q)));
-}
-
-// (15)-(17)
-__global__ void k_upd3(int64_t n, Vecs vs, const SolverState* st) {
+template <int MODE>
+__global__ void k_upd(int64_t n, Vecs vs, const SolverState* st) {
     pdl_wait();
     pdl_launch();
     if (st->done) return;
     const float alpha = (float)st->alpha, beta = (float)st->beta;
-    GRID_LOOP(q, n / 4) {
-        const float4 r = ld4(vs.r, q);
-        st4(vs.u, q, axmy(r, beta, ld4(vs.u, q)));
-        st4(vs.r, q, axmy(r, alpha, ld4(vs.v, q)));
-        st4(vs.s, q, axmy(ld4(vs.s, q), alpha, ld4(vs.w, q)));
+    GRID_LOOP(q, n / 4) update4<MODE>(vs, q, alpha, beta);
+}
+// The same with the coarse form's restriction R of the result (to `rest`, c0 x
+// c1 x c2 cells): a thread takes the 16 fine cells of two coarse ones, in the
+// order of the network's own restriction, so the bits are the same; the
+// separate pass read the vector again (4.5 us at 128^3 beside 6.5 here).
+template <int MODE>
+__global__ void __launch_bounds__(256) k_upd_pool(int c0, int c1, int c2, Vecs vs, const SolverState* st,
+                                                  float* __restrict__ rest) {
+    pdl_wait();
+    pdl_launch();
+    if (st->done) return;
+    const float alpha = (float)st->alpha, beta = (float)st->beta;
+    const int h2 = c2 / 2;
+    const int64_t F1 = 2 * (int64_t)c1;
+    GRID_LOOP(e, (int64_t)c0 * c1 * h2) {
+        const int64_t K2 = e % h2, JI = e / h2, J = JI % c1, I = JI / c1;
+        float s0 = 0.f, s1 = 0.f;
+#pragma unroll
+        for (int a = 0; a < 2; a++)
+#pragma unroll
+            for (int b = 0; b < 2; b++) {
+                const float4 v = update4<MODE>(vs, ((2 * I + a) * F1 + 2 * J + b) * h2 + K2, alpha, beta);
+                s0 += v.x + v.y;
+                s1 += v.z + v.w;
+            }
+        *reinterpret_cast<float2*>(rest + JI * c2 + 2 * K2) = make_float2(0.125f * s0, 0.125f * s1);
     }
 }
 
 // (10), (24) in flexible form: d += (a1 - a2 b1) zu + (a2 + w1) zr - w1 a2 zv + w2 zs;
-// (25): r -= w1 s + w2 t; u -= w1 v + w2 w; convergence test on ||r||
+// (25): r -= w1 s + w2 t; u -= w1 v + w2 w; convergence test on ||r||; the next
+// iteration's (3), (4) from <rh, r>
 __global__ void __launch_bounds__(256) k_upd_final(int64_t n, Vecs vs, SolverState* st, double* partials) {
     pdl_wait();
     pdl_launch();
@@ -314,7 +328,7 @@ __global__ void __launch_bounds__(256) k_upd_final(int64_t n, Vecs vs, SolverSta
     const double a1 = st->alpha1, a2 = st->alpha, b1 = st->beta1, om1 = st->omega1, om2 = st->omega2;
     const float cu = (float)(a1 - a2 * b1), cr = (float)(a2 + om1), cv = (float)(-om1 * a2), cs = (float)om2;
     const float w1 = (float)om1, w2 = (float)om2;
-    double acc[1] = {0.};
+    double acc[2] = {0., 0.};
     GRID_LOOP(q, n / 4) {
         const float4 zu = ld4(vs.zu, q), zr = ld4(vs.zr, q), zv = ld4(vs.zv, q), zs = ld4(vs.zs, q);
         float4 d = ld4(vs.d, q);
@@ -335,9 +349,10 @@ __global__ void __launch_bounds__(256) k_upd_final(int64_t n, Vecs vs, SolverSta
         u.w -= w1 * v.w + w2 * w.w;
         st4(vs.u, q, u);
         acc[0] += sq4(rn);
+        acc[1] += dot4(ld4(vs.rh, q), rn);
     }
-    double tot[1];
-    if (!grid_reduce<1>(acc, partials, &st->count, tot)) return;
+    double tot[2];
+    if (!grid_reduce<2>(acc, partials, &st->count, tot)) return;
     if (threadIdx.x == 0) {
         const double rn = sqrt(tot[0]);
         st->rnorm = rn;
@@ -350,6 +365,8 @@ __global__ void __launch_bounds__(256) k_upd_final(int64_t n, Vecs vs, SolverSta
         } else if (++st->k > st->max_it) {
             st->done = 1;
             st->status = ST_MAXIT;
+        } else {
+            next_rho(st, tot[1]);
         }
     }
 }
@@ -379,23 +396,27 @@ static int launch_iteration(dare_ctx* ctx, dare_unet* net, const GridDev& g, con
         f.out = out;
         return launch_march(ctx, g, m, f, st, partials);
     };
-    launch_pdl(k_rho, dim3(eb), dim3(256), 0, s, true, n, vs, st, partials);
-    DARE_LAUNCHED(ctx);
-    launch_pdl(k_upd_u, dim3(eb), dim3(256), 0, s, true, n, vs, st);
-    DARE_LAUNCHED(ctx);
-    if ((rc = unet::apply(net, vs.u, vs.zu))) return rc;
+    // a vector update and N of its result
+    auto updated = [&](auto mode, const float* x, float* z) {
+        constexpr int MODE = decltype(mode)::value;
+        if (net->coarse) {
+            const int *c = net->n;
+            launch_pdl(k_upd_pool<MODE>, dim3(grid_blocks(ctx, net->ncell / 2, 256, 8)), dim3(256), 0, s, true, c[0], c[1],
+                       c[2], vs, st, unet::pooled(net));
+            DARE_LAUNCHED(ctx);
+            return unet::apply_pooled(net, x, z);
+        }
+        launch_pdl(k_upd<MODE>, dim3(eb), dim3(256), 0, s, true, n, vs, st);
+        DARE_LAUNCHED(ctx);
+        return unet::apply(net, x, z);
+    };
+    if ((rc = updated(std::integral_constant<int, UPD_U>{}, vs.u, vs.zu))) return rc;
     if ((rc = spmv_dot(FLSpmvDot<0, 7>{}, vs.zu, vs.v))) return rc;
-    launch_pdl(k_upd_r, dim3(eb), dim3(256), 0, s, true, n, vs, st);
-    DARE_LAUNCHED(ctx);
-    if ((rc = unet::apply(net, vs.r, vs.zr))) return rc;
+    if ((rc = updated(std::integral_constant<int, UPD_R>{}, vs.r, vs.zr))) return rc;
     if ((rc = spmv_dot(FLSpmvDot<1, 11>{}, vs.zr, vs.s))) return rc;
-    launch_pdl(k_upd_v, dim3(eb), dim3(256), 0, s, true, n, vs, st);
-    DARE_LAUNCHED(ctx);
-    if ((rc = unet::apply(net, vs.v, vs.zv))) return rc;
+    if ((rc = updated(std::integral_constant<int, UPD_V>{}, vs.v, vs.zv))) return rc;
     if ((rc = spmv_dot(FLSpmvDot<0, 14>{}, vs.zv, vs.w))) return rc;
-    launch_pdl(k_upd3, dim3(eb), dim3(256), 0, s, true, n, vs, st);
-    DARE_LAUNCHED(ctx);
-    if ((rc = unet::apply(net, vs.s, vs.zs))) return rc;
+    if ((rc = updated(std::integral_constant<int, UPD_S>{}, vs.s, vs.zs))) return rc;
     FLSpmvOmega fo{};
     fo.zs[0] = vs.zs;
     for (int q = 0; q < 6; q++) fo.ps[q] = ah + (size_t)q * n;

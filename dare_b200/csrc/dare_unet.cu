@@ -2040,12 +2040,24 @@ static int apply_grid(dare_unet* net, const float* u, float* z, bool overlap) {
     return conv_forward(net, DEC0, net->S0, nullptr, OUT_F32, nullptr, nullptr, z, u);
 }
 
+float* pooled(dare_unet* net) { return net->cbuf; }
+
+int apply_pooled(dare_unet* net, const float* u, float* z) {
+    dare_ctx* ctx = net->ctx;
+    float* uc = net->cbuf;
+    float* zc = net->cbuf + net->ncell;
+    int rc = apply_grid(net, uc, zc, true);
+    if (rc) return rc;
+    launch_pdl(k_coarse_add, dim3(eblocks(ctx, net->fine_ncell / 4)), dim3(256), 0, ctx->stream, true, net->n[0],
+               net->n[1], net->n[2], u, (const float*)zc, (const float*)uc, z);
+    DARE_LAUNCHED(ctx);
+    return DARE_OK;
+}
+
 int apply(dare_unet* net, const float* u, float* z) {
     if (!net->coarse) return apply_grid(net, u, z, false);
     // coarse form: z = u + P (N_c(R u) - R u), N_c(v) = v + U(v) on the coarse grid
     dare_ctx* ctx = net->ctx;
-    float* uc = net->cbuf;
-    float* zc = net->cbuf + net->ncell;
     // (16-byte accesses: u and z must be 16-byte aligned; an unaligned
     // caller vector is copied first)
     const float* uin = u;
@@ -2058,16 +2070,12 @@ int apply(dare_unet* net, const float* u, float* z) {
         zout = net->fbuf + net->fine_ncell;
     }
     launch_pdl(k_pool8, dim3(eblocks(ctx, net->ncell / 2)), dim3(256), 0, ctx->stream, true, net->n[0], net->n[1],
-               net->n[2], uin, uc);
+               net->n[2], uin, net->cbuf);
     DARE_LAUNCHED(ctx);
-    int rc = apply_grid(net, uc, zc, true);
+    const int rc = apply_pooled(net, uin, zout);
     if (rc) return rc;
-    launch_pdl(k_coarse_add, dim3(eblocks(ctx, net->fine_ncell / 4)), dim3(256), 0, ctx->stream, true, net->n[0],
-               net->n[1], net->n[2], uin, zc, uc, zout);
-    DARE_LAUNCHED(ctx);
     if (zout != z)
         DARE_CUDA(ctx, cudaMemcpyAsync(z, zout, net->fine_ncell * sizeof(float), cudaMemcpyDeviceToDevice, ctx->stream));
-    DARE_LAUNCHED(ctx);
     return DARE_OK;
 }
 

@@ -193,5 +193,9 @@ namespace unet {
 // z = N(u) on the context's stream (no synchronisation); used by the solver.
 // u and z live on the system's grid (the fine grid of a coarse-form network).
 int apply(dare_unet* net, const float* u, float* z);
+// Coarse form: the restriction R u, where apply() puts it; apply_pooled() is
+// apply() with it already there (u and z 16-byte aligned).
+float* pooled(dare_unet* net);
+int apply_pooled(dare_unet* net, const float* u, float* z);
 }  // namespace unet
 }  // namespace dare_gpu
