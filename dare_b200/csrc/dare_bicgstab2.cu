@@ -143,8 +143,6 @@ template int launch_init<double, true>(dare_ctx*, const GridDev&, const MarchCfg
                                        const VecsT<double>&, SolverState*, double*);
 template int launch_init<double, false>(dare_ctx*, const GridDev&, const MarchCfg&, const OpT<double>&,
                                         const VecsT<double>&, SolverState*, double*);
-template int launch_init<float, true>(dare_ctx*, const GridDev&, const MarchCfg&, const OpT<float>&,
-                                      const VecsT<float>&, SolverState*, double*);
 
 // One iteration (`par`: its place in the pair a graph holds; every iteration
 // uses the same buffers).  `ev` (optional, profiling): ev[0] before the first

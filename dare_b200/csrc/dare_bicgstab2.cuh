@@ -195,7 +195,7 @@ struct dare_solver_ws {
     void* team_buf = nullptr;   // exchanges of the one-launch solve (dare_team.cuh)
     // FP32 inner solver of the refinement driver (dare_mixed.cu)
     float* ahat32 = nullptr;     // 6 * n
-    float* vec32 = nullptr;      // (kNumSolverVecs + 2) * n: work vectors, the correction, the right-hand side
+    float* vec32 = nullptr;      // (kNumSolverVecs + 1) * n: work vectors, the correction
     dare_gpu::MarchCfg march32;
     // learned-preconditioner solver (dare_learned.cu)
     struct dare_learned_ws* learned = nullptr;

@@ -41,41 +41,42 @@ static __global__ void k_to_precond_var(int64_t n, const double* __restrict__ dc
         x[c] = dc[c] * x[c];
 }
 
-// ||b||^2 -> *out (sqrt)
-static __global__ void __launch_bounds__(256) k_norm(int64_t n, const double* __restrict__ b, SolverState* st,
-                                                     double* partials, double* out) {
-    double acc[1] = {0.};
-    for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n; c += (int64_t)gridDim.x * blockDim.x)
-        acc[0] += b[c] * b[c];
-    double tot[1];
-    if (!grid_reduce<1>(acc, partials, &st->count, tot)) return;
-    if (threadIdx.x == 0) *out = sqrt(tot[0]);
-}
-
-// r = b - A x in FP64; r32 = (float) r; dy = 0; ||r||_2 -> *out
+// r = b - A x in FP64, ||r||_2 and ||b||_2 -> out, and the start of the inner
+// solve of Ahat dy = r from dy = 0: its r and r_hat_0 are r rounded to FP32, u =
+// dy = 0, and its first scalars.  (An init kernel of the inner solve would read
+// the operator and the zero vector to form the same r: 52 more bytes a cell.)
 struct FRefResidual {
     using type = double;
-    static constexpr int Q = 1, NZ = 1, NP = 8;
+    static constexpr int Q = 3, NZ = 1, NP = 8;
     static constexpr bool kCheckDone = false;
     static constexpr bool kPairs = false;
     const double* zs[2];   // x
     const double* ps[NP];  // 7 coefficients, b
-    float* r32;
-    float* dy;
+    float *r32, *rh, *u, *dy;
     double* out;
     __device__ void load(const SolverState*) {}
     __device__ double zc(double a, double) const { return a; }
     __device__ void center(int64_t c, const double (&zz)[7], const double* p, double* acc) const {
         const double r = p[7] - apply_pre<double, false>(p, zz);
-        r32[c] = (float)r;
+        const float rf = (float)r;
+        r32[c] = rf;
+        rh[c] = rf;
+        u[c] = 0.f;
         dy[c] = 0.f;
         acc[0] += r * r;
+        acc[1] += p[7] * p[7];
+        acc[2] += (double)rf * (double)rf;
     }
-    __device__ void done(SolverState*, const double* tot) const { *out = sqrt(tot[0]); }
+    __device__ void done(SolverState* st, const double* tot) const {
+        out[0] = sqrt(tot[0]);
+        out[1] = sqrt(tot[1]);
+        const double start[2] = {tot[2], tot[2]};
+        finish_init(st, start);
+    }
 };
 
-static int read_scalar(dare_ctx* ctx, const double* dptr, double* out) {
-    DARE_CUDA(ctx, cudaMemcpyAsync(out, dptr, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+static int read_norms(dare_ctx* ctx, const double* dptr, double (&out)[2]) {
+    DARE_CUDA(ctx, cudaMemcpyAsync(out, dptr, sizeof(out), cudaMemcpyDeviceToHost, ctx->stream));
     DARE_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     return DARE_OK;
 }
@@ -94,7 +95,7 @@ int dare_bicgstab2_refine(dare_system* s, const dare_solver_params* p, dare_solv
     const int64_t n = g.ncell;
     if (!ws->ahat32) {
         cudaError_t e = cudaMalloc(&ws->ahat32, (size_t)n * 6 * sizeof(float));
-        if (e == cudaSuccess) e = cudaMalloc(&ws->vec32, (size_t)n * (kNumSolverVecs + 2) * sizeof(float));
+        if (e == cudaSuccess) e = cudaMalloc(&ws->vec32, (size_t)n * (kNumSolverVecs + 1) * sizeof(float));
         if (e != cudaSuccess) {
             dare_mixed_ws_free(ws);
             return check_cuda(ctx, e, "refinement workspace");
@@ -110,34 +111,38 @@ int dare_bicgstab2_refine(dare_system* s, const dare_solver_params* p, dare_solv
     if ((rc = launch_fold32(ctx, g, m, s->diag, ws->invd, ws->ahat32, ws->st, ws->partials))) return rc;
     OpT<float> op32{nullptr, ws->ahat32, n};
     float* dy = ws->vec32 + kNumSolverVecs * n;
-    float* r32 = ws->vec32 + (kNumSolverVecs + 1) * n;
-    VecsT<float> vs32 = carve_vecs<float>(ws->vec32, n, dy, r32);
+    VecsT<float> vs32 = carve_vecs<float>(ws->vec32, n, dy, nullptr);
 
     double* scratch = ws->partials + (size_t)kMaxQ * kMaxBlocks;
-    SolverState zero{};
-    DARE_CUDA(ctx, cudaMemcpyAsync(ws->st, &zero, sizeof(zero), cudaMemcpyHostToDevice, ctx->stream));
-    k_norm<<<eb, 256, 0, ctx->stream>>>(n, s->rhs, ws->st, ws->partials, scratch);
-    DARE_LAUNCHED(ctx);
-    double bnorm = 0.;
-    if ((rc = read_scalar(ctx, scratch, &bnorm))) return rc;
-    const double tol_abs = p->tol_relative ? p->tol * bnorm : p->tol;
-
     std::memset(rep, 0, sizeof(*rep));
-    rep->b_norm = bnorm;
-    rep->tol_abs = tol_abs;
-    double rnorm = 0., prev = INFINITY;
+    double tol_abs = 0., rnorm = 0., prev = INFINITY;
     bool converged = false;
     int refinements = 0, inner_total = 0;
     for (int it = 0; it <= p->max_refinements; it++) {
+        // the inner FP32 BiCGStab2 on Ahat dy = r: relative tolerance, FP64 dots
+        SolverState init{};
+        init.tol = p->inner_rel_tol;
+        init.tol_relative = 1;
+        init.max_it = p->inner_max_it;
+        DARE_CUDA(ctx, cudaMemcpyAsync(ws->st, &init, sizeof(init), cudaMemcpyHostToDevice, ctx->stream));
         FRefResidual fr{};
         fr.zs[0] = s->x;
         set_coef_streams<double, false, 8>(full, fr.ps);
         fr.ps[7] = s->rhs;
-        fr.r32 = r32;
+        fr.r32 = vs32.r;
+        fr.rh = vs32.rh;
+        fr.u = vs32.u;
         fr.dy = dy;
         fr.out = scratch;
         if ((rc = launch_march(ctx, g, m, fr, ws->st, ws->partials))) return rc;
-        if ((rc = read_scalar(ctx, scratch, &rnorm))) return rc;
+        double norms[2] = {0., 0.};
+        if ((rc = read_norms(ctx, scratch, norms))) return rc;
+        rnorm = norms[0];
+        if (it == 0) {
+            rep->b_norm = norms[1];
+            tol_abs = p->tol_relative ? p->tol * norms[1] : p->tol;
+            rep->tol_abs = tol_abs;
+        }
         if (rnorm <= tol_abs) {
             converged = true;
             break;
@@ -146,13 +151,6 @@ int dare_bicgstab2_refine(dare_system* s, const dare_solver_params* p, dare_solv
             break;
         }
         prev = rnorm;
-        // inner FP32 BiCGStab2 on Ahat dy = r, relative tolerance, FP64 dots
-        SolverState init{};
-        init.tol = p->inner_rel_tol;
-        init.tol_relative = 1;
-        init.max_it = p->inner_max_it;
-        DARE_CUDA(ctx, cudaMemcpyAsync(ws->st, &init, sizeof(init), cudaMemcpyHostToDevice, ctx->stream));
-        if ((rc = launch_init<float, true>(ctx, g, m32, op32, vs32, ws->st, ws->partials))) return rc;
         if ((rc = run_iterations<float, true>(ctx, g, m32, ws->stream_blocks, op32, vs32, ws->st, ws->st_host,
                                               ws->partials, &ws->graph[2][0], p->inner_max_it, p->check_every, 9)))
             return rc;
@@ -182,6 +180,7 @@ int dare_bicgstab2_refine(dare_system* s, const dare_solver_params* p, dare_solv
     q.precision = DARE_PRECISION_FP64;
     q.tol = tol_abs;
     q.tol_relative = 0;
+    const double bnorm = rep->b_norm;
     dare_solve_report r2;
     if ((rc = dare_bicgstab2_fp64(s, &q, &r2))) return rc;
     *rep = r2;
