@@ -7,8 +7,8 @@
 // a device queue.  Inside an item the block walks along i.  Every plane is
 // staged in shared memory by asynchronous copies (cp.async): the inputs of the
 // fused SpMV operand with a one-cell j/k halo, and the per-cell streams of the
-// centre step (coefficients, vectors).  A ring of three stages keeps the
-// copies of planes i+1 and i+2 in flight while plane i computes, so HBM
+// centre step (coefficients, vectors).  A ring of stages keeps the
+// copies of the next planes in flight while plane i computes, so HBM
 // latency hides behind the arithmetic without holding data in registers.
 // Dot-product partials are kept per item and summed in item order by the
 // last item, so results do not depend on which block took which item.
@@ -542,6 +542,31 @@ __device__ __forceinline__ void cp_async(void* smem, const void* gmem, bool vali
     asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;\n" ::"r"(s), "l"(gmem), "n"(BYTES), "r"(src)
                  : "memory");
 }
+// The 16-byte copies of the operator's off-diagonals: their kernel reads them
+// once and the next one only after all the others, so they are the first to leave
+// L2 and the vectors that one kernel wrote are still there for the next (FP64
+// 128^3 time step 1.76 -> 1.68 ms; no difference at 192^3 and 256^3, where the
+// vectors alone are larger than L2).  L1: FP64 copies go through L1 (past it
+// 256^3 took 12.6 ms for 12.1), the FP32 ones past it (256^3 refined solve
+// 6.35 -> 6.23 ms; with every copy past it 1 % slower again).
+__device__ __forceinline__ uint64_t evict_first_policy() {
+    uint64_t p;
+    asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;\n" : "=l"(p));
+    return p;
+}
+template <bool L1>
+__device__ __forceinline__ void cp_async16_once(void* smem, const void* gmem, bool valid, uint64_t policy) {
+    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+    const int src = valid ? 16 : 0;
+    if constexpr (L1)
+        asm volatile("cp.async.ca.shared.global.L2::cache_hint [%0], [%1], 16, %2, %3;\n" ::"r"(s), "l"(gmem), "r"(src),
+                     "l"(policy)
+                     : "memory");
+    else
+        asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2, %3;\n" ::"r"(s), "l"(gmem), "r"(src),
+                     "l"(policy)
+                     : "memory");
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
@@ -554,10 +579,21 @@ template <class K>
 __host__ __device__ constexpr size_t march_stage_elems(int tw, int tj, int ic) {
     return (size_t)K::NZ * (tw + 2 * ic) * (tj + 2) + (size_t)K::NP * tw * tj;
 }
+// Stages of the ring of planes.  While plane i is computed from planes i and
+// i + 1, the stages up to i + depth - 1 are on their way: with two blocks a SM a
+// kernel of the FP64 iteration has about 74 KB a SM in flight with four stages
+// (256^3: steps at 5.7 TB/s with three; time step 12.08 -> 11.83 ms with four;
+// five leave one block a SM, 15.2 ms).  The FP32 kernels run three blocks a SM
+// with three stages (four stages, two blocks: 0.5 to 1 % slower).
+template <typename T>
+struct MarchDepth {
+    static constexpr int value = sizeof(T) == 8 ? 4 : 3;
+};
 template <class K>
 inline size_t march_smem_bytes(const MarchCfg& m) {
     const int ic = m.cpt;   // first interior column: one row segment of padding
-    return 3 * march_stage_elems<K>(m.block.x * m.cpt, m.block.y, ic) * sizeof(typename K::type);
+    return MarchDepth<typename K::type>::value * march_stage_elems<K>(m.block.x * m.cpt, m.block.y, ic) *
+           sizeof(typename K::type);
 }
 
 // two consecutive elements of shared memory in one load (16-byte aligned for
@@ -616,6 +652,8 @@ __global__ void __launch_bounds__(256, MarchMinBlocks<K, CPT>::value) k_march(Gr
     static_assert(!PAIR || VEC % CPT == 0, "16-byte staging: a copy covers whole thread segments");
     constexpr int IC = PAIR ? VEC : CPT;        // first interior column of a staged operand row
     constexpr int CB = CPT * (int)sizeof(T);    // bytes of one thread's row segment
+    constexpr int D = MarchDepth<T>::value;
+    const uint64_t once = evict_first_policy();
     pdl_wait();
     pdl_launch();
     if (K::kCheckDone && st->done) return;
@@ -737,7 +775,7 @@ __global__ void __launch_bounds__(256, MarchMinBlocks<K, CPT>::value) k_march(Gr
         }
         return G;
     };
-    auto slot_of = [&](const Geo& G, int p) { return (p - G.i0 + 1) % 3; };
+    auto slot_of = [&](const Geo& G, int p) { return (p - G.i0 + 1) % D; };
     // Stage plane p into its ring slot: operand inputs with halo, and (when
     // `full`) the per-cell streams.  Out-of-range planes are zeros.
     auto stage = [&](const Geo& G, int p, bool full) {
@@ -791,8 +829,13 @@ __global__ void __launch_bounds__(256, MarchMinBlocks<K, CPT>::value) k_march(Gr
                 T* pt = sb + NZ * ZT + pr_row * TW + pr_col;
 #pragma unroll
                 for (int q = 0; q < NP; q++)
-                    if ((q & 1) == par)
-                        cp_async<16>(pt + q * NCT, k.ps[q] + base + (G.o_pair < 0 ? 0 : G.o_pair), G.o_pair >= 0);
+                    if ((q & 1) == par) {
+                        const T* src = k.ps[q] + base + (G.o_pair < 0 ? 0 : G.o_pair);
+                        if (q < 6)   // off-diagonals
+                            cp_async16_once<sizeof(T) == 8>(pt + q * NCT, src, G.o_pair >= 0, once);
+                        else
+                            cp_async<16>(pt + q * NCT, src, G.o_pair >= 0);
+                    }
             }
             return;
         }
@@ -802,14 +845,17 @@ __global__ void __launch_bounds__(256, MarchMinBlocks<K, CPT>::value) k_march(Gr
             for (int q = 0; q < NP; q++) cp_async<CB>(pt + q * NCT, k.ps[q] + base + G.o_own, true);
         }
     };
-    // prologue of an item: planes i0-1 (operand only), i0, i0+1
+    // prologue of an item: planes i0-1 (operand only), i0 .. i0+D-2
     auto prologue = [&](const Geo& G) {
         stage(G, G.i0 - 1, false);
         cp_async_commit();
         stage(G, G.i0, true);
         cp_async_commit();
-        stage(G, G.i0 + 1, G.i0 + 1 < G.i1);
-        cp_async_commit();
+#pragma unroll
+        for (int d = 1; d < D - 1; d++) {
+            if (G.i0 + d <= G.i1) stage(G, G.i0 + d, G.i0 + d < G.i1);
+            cp_async_commit();
+        }
     };
     auto zval = [&](const T* sb, int row, int col) -> T {
         const T a = sb[row * W + col];
@@ -832,27 +878,38 @@ __global__ void __launch_bounds__(256, MarchMinBlocks<K, CPT>::value) k_march(Gr
         double acc[QA];
 #pragma unroll
         for (int q = 0; q < QA; q++) acc[q] = 0.;
-        cp_async_wait<2>();
+        cp_async_wait<D - 2>();                 // planes i0-1 and i0
         __syncthreads();
         constexpr bool SPLIT = SplitOperands<K>::value;
-        T zprev[CPT];
-        T zprev_b = T(0);   // split operands: the second array's value at plane i - 1
+        // the thread's operand values of planes i - 1 and i (split operands: of
+        // both arrays), kept from the plane before: L1 and shared memory run at
+        // 70 % of their rate, and reading plane i's again cost 1.3 % at 256^3
+        T zprev[CPT], zthis[CPT];
+        T zprev_b = T(0), zthis_b = T(0);
+        const T* sp = smem + (size_t)slot_of(G, G.i0 - 1) * STAGE;
+        const T* s0 = smem + (size_t)slot_of(G, G.i0) * STAGE;
         if constexpr (SPLIT) {
-            const T* s0 = smem + (size_t)slot_of(G, G.i0 - 1) * STAGE + (ty + 1) * W + IC + tx;
-            zprev[0] = G.inside ? s0[0] : T(0);
-            zprev_b = G.inside ? s0[ZT] : T(0);
+            const int at = (ty + 1) * W + IC + tx;
+            zprev[0] = G.inside ? sp[at] : T(0);
+            zprev_b = G.inside ? sp[ZT + at] : T(0);
+            zthis[0] = G.inside ? s0[at] : T(0);
+            zthis_b = G.inside ? s0[ZT + at] : T(0);
         } else {
 #pragma unroll
-            for (int c = 0; c < CPT; c++)
-                zprev[c] =
-                    G.inside ? zval(smem + (size_t)slot_of(G, G.i0 - 1) * STAGE, ty + 1, IC + CPT * tx + c) : T(0);
+            for (int c = 0; c < CPT; c++) {
+                zprev[c] = G.inside ? zval(sp, ty + 1, IC + CPT * tx + c) : T(0);
+                zthis[c] = G.inside ? zval(s0, ty + 1, IC + CPT * tx + c) : T(0);
+            }
         }
-        __syncthreads();
         for (int i = G.i0; i < G.i1; i++) {
-            if (i + 2 <= G.i1) stage(G, i + 2, i + 2 < G.i1);   // reuses the slot of plane i-1
+            if constexpr (D > 3) cp_async_wait<D - 3>();   // planes i and i+1 have landed
+            __syncthreads();                    // and every thread is done with plane i-1
+            if (i + D - 1 <= G.i1) stage(G, i + D - 1, i + D - 1 < G.i1);   // in the slot of plane i-1
             cp_async_commit();
-            cp_async_wait<1>();                 // planes i and i+1 have landed
-            __syncthreads();
+            if constexpr (D == 3) {             // plane i+1 has too
+                cp_async_wait<1>();
+                __syncthreads();
+            }
             const T* sb = smem + (size_t)slot_of(G, i) * STAGE;
             const T* sn = smem + (size_t)slot_of(G, i + 1) * STAGE;
             if (G.inside) {
@@ -860,10 +917,11 @@ __global__ void __launch_bounds__(256, MarchMinBlocks<K, CPT>::value) k_march(Gr
                     static_assert(CPT == 1, "split operands run one cell per thread");
                     const int col = IC + tx;
                     auto raw = [&](const T* b, int z, int row, int cc) { return b[z * ZT + row * W + cc]; };
-                    const T a0 = raw(sb, 0, ty + 1, col), b0 = raw(sb, 1, ty + 1, col);
-                    const T za[7] = {a0, zprev[0], raw(sn, 0, ty + 1, col), raw(sb, 0, ty, col), raw(sb, 0, ty + 2, col),
+                    const T a0 = zthis[0], b0 = zthis_b;
+                    const T an = raw(sn, 0, ty + 1, col), bn = raw(sn, 1, ty + 1, col);
+                    const T za[7] = {a0, zprev[0], an, raw(sb, 0, ty, col), raw(sb, 0, ty + 2, col),
                                      raw(sb, 0, ty + 1, col - 1), raw(sb, 0, ty + 1, col + 1)};
-                    const T zb[7] = {b0, zprev_b, raw(sn, 1, ty + 1, col), raw(sb, 1, ty, col), raw(sb, 1, ty + 2, col),
+                    const T zb[7] = {b0, zprev_b, bn, raw(sb, 1, ty, col), raw(sb, 1, ty + 2, col),
                                      raw(sb, 1, ty + 1, col - 1), raw(sb, 1, ty + 1, col + 1)};
                     T pv[NP];
 #pragma unroll
@@ -871,10 +929,12 @@ __global__ void __launch_bounds__(256, MarchMinBlocks<K, CPT>::value) k_march(Gr
                     k.center2((int64_t)i * plane + G.o_own, za, zb, pv, acc);
                     zprev[0] = a0;
                     zprev_b = b0;
+                    zthis[0] = an;
+                    zthis_b = bn;
                 } else if constexpr (CPT == 1) {
                     const int col = IC + tx;
-                    const T zcur = zval(sb, ty + 1, col);
-                    const T z7[7] = {zcur, zprev[0], zval(sn, ty + 1, col), zval(sb, ty, col), zval(sb, ty + 2, col),
+                    const T zcur = zthis[0], znext = zval(sn, ty + 1, col);
+                    const T z7[7] = {zcur, zprev[0], znext, zval(sb, ty, col), zval(sb, ty + 2, col),
                                      zval(sb, ty + 1, col - 1), zval(sb, ty + 1, col + 1)};
                     T pv[NP];
 #pragma unroll
@@ -884,6 +944,7 @@ __global__ void __launch_bounds__(256, MarchMinBlocks<K, CPT>::value) k_march(Gr
                     else
                         k.center((int64_t)i * plane + G.o_own, z7, pv, acc);
                     zprev[0] = zcur;
+                    zthis[0] = znext;
                 } else if constexpr (CPT == 2) {
                     // the thread's two cells as one 16-byte (8-byte for FP32)
                     // shared-memory load per row: consecutive threads read
@@ -896,8 +957,8 @@ __global__ void __launch_bounds__(256, MarchMinBlocks<K, CPT>::value) k_march(Gr
                         z0 = k.zc(a.x, c2.x);
                         z1 = k.zc(a.y, c2.y);
                     };
-                    T zc0, zc1, zn0, zn1, zs0, zs1, zt0, zt1;
-                    zpair(sb, ty + 1, zc0, zc1);
+                    const T zc0 = zthis[0], zc1 = zthis[1];
+                    T zn0, zn1, zs0, zs1, zt0, zt1;
                     zpair(sn, ty + 1, zn0, zn1);
                     zpair(sb, ty, zs0, zs1);
                     zpair(sb, ty + 2, zt0, zt1);
@@ -921,6 +982,8 @@ __global__ void __launch_bounds__(256, MarchMinBlocks<K, CPT>::value) k_march(Gr
                     }
                     zprev[0] = zc0;
                     zprev[1] = zc1;
+                    zthis[0] = zn0;
+                    zthis[1] = zn1;
                 } else {
                     // four FP32 cells per thread: every row segment one 16-byte
                     // copy and one 16-byte shared-memory load
@@ -935,8 +998,8 @@ __global__ void __launch_bounds__(256, MarchMinBlocks<K, CPT>::value) k_march(Gr
                         z[2] = k.zc(a.z, c2.z);
                         z[3] = k.zc(a.w, c2.w);
                     };
-                    T zc[4], zn[4], zs[4], zt[4];
-                    zquad(sb, ty + 1, zc);
+                    T zn[4], zs[4], zt[4];
+                    const T (&zc)[4] = zthis;
                     zquad(sn, ty + 1, zn);
                     zquad(sb, ty, zs);
                     zquad(sb, ty + 2, zt);
@@ -960,12 +1023,15 @@ __global__ void __launch_bounds__(256, MarchMinBlocks<K, CPT>::value) k_march(Gr
                             k.center((int64_t)i * plane + G.o_own + c, z7, pv[c], acc);
                     }
 #pragma unroll
-                    for (int c = 0; c < 4; c++) zprev[c] = zc[c];
+                    for (int c = 0; c < 4; c++) {
+                        zprev[c] = zthis[c];
+                        zthis[c] = zn[c];
+                    }
                 }
             }
-            __syncthreads();                    // slot of plane i is free for plane i+3
         }
         cp_async_wait<0>();
+        __syncthreads();                        // every plane of this item has been read
         const int next = s_next;                // written before this item's barriers
         Geo GN = G;
         if (next < m.nitems) {
@@ -1026,7 +1092,8 @@ inline int launch_march_k(dare_ctx* ctx, const GridDev& g, const MarchCfg& m0, c
                           double* partials) {
     MarchCfg m = m0;
     const int ic = PAIR ? 16 / (int)sizeof(typename K::type) : m.cpt;   // first interior column of an operand row
-    const size_t smem = 3 * march_stage_elems<K>(m.block.x * m.cpt, m.block.y, ic) * sizeof(typename K::type);
+    const size_t smem = MarchDepth<typename K::type>::value * march_stage_elems<K>(m.block.x * m.cpt, m.block.y, ic) *
+                        sizeof(typename K::type);
     static int per_sm = 0;
     static size_t per_sm_smem = 0;
     if (per_sm == 0 || per_sm_smem != smem) {
