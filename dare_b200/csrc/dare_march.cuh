@@ -1218,6 +1218,25 @@ struct Step5 {
 //     array 16-byte aligned): four cells per thread and 16-byte accesses
 //     (512^3: 0.92 ms; with 4-byte accesses the FP32 kernel took 1.22 ms,
 //     81 % of copy bandwidth, both with nine arrays read).
+//     In FP64 the products and x, which the next kernels do not read, are
+//     loaded and stored as the first to leave L2, so that r, u and rh stay for
+//     step 1 (128^3 time step 1.62 -> 1.57 ms, 192^3 4.52 -> 4.48; in FP32 the
+//     256^3 refined solve lost 0.4 %).  Two cells a thread and loop trip gave 0.6 %
+//     at 256^3 and took the gain at 128^3 away (an odd last trip).
+template <typename T>
+__device__ __forceinline__ T ld_once(const T* p) {
+    if constexpr (sizeof(T) == 8)
+        return __ldcs(p);
+    else
+        return *p;
+}
+template <typename T>
+__device__ __forceinline__ void st_once(T* p, T v) {
+    if constexpr (sizeof(T) == 8)
+        __stcs(p, v);
+    else
+        *p = v;
+}
 template <typename T>
 __global__ void __launch_bounds__(256) k_step5(int64_t n, T* __restrict__ x, T* __restrict__ r, T* __restrict__ u,
                                                const T* __restrict__ v, const T* __restrict__ s,
@@ -1259,9 +1278,9 @@ __global__ void __launch_bounds__(256) k_step5(int64_t n, T* __restrict__ x, T* 
         }
     }
     for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n; c += (int64_t)gridDim.x * blockDim.x) {
-        T xc = x[c], rc = r[c], uc = u[c];
-        f.cell(xc, rc, uc, v[c], s[c], w[c], t[c]);
-        x[c] = xc;
+        T xc = ld_once(x + c), rc = r[c], uc = u[c];
+        f.cell(xc, rc, uc, ld_once(v + c), ld_once(s + c), ld_once(w + c), ld_once(t + c));
+        st_once(x + c, xc);
         r[c] = rc;
         u[c] = uc;
         acc[0] += (double)rc * (double)rc;
