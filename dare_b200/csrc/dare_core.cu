@@ -80,52 +80,72 @@ __global__ void k_scatter_to_field(GridDev g, const double* __restrict__ x, doub
 // written are those of k_scale, k_scatter_to_field and k_halo_fill in turn
 // (needs og[d] == ng and n[d] >= ng on the periodic dimensions).  Threads
 // run along k, block rows along (i, j).
-// A thread takes the same k of kSolRows rows, its loads before its stores: with
-// one row at a time, too little was in flight (256^3: 200 -> 145 us, 128^3: 27.7 ->
-// 22.0; eight rows cost registers and blocks, 207 us).
-constexpr int kSolRows = 4;
+// A block takes a run of rows, a thread the same k of kSolRows of them at a time,
+// loads before stores; the images' offsets are unrolled over the dimensions (as an
+// indexed array they lived in local memory, stored for every cell).  128^3: 27.7 ->
+// 14.9 us; 256^3 without invd 131 -> 79 us (four rows: 85).
+constexpr int kSolRows = 2;
+// the periodic images of a cell at offset `at` of the ghosted level
+__device__ __forceinline__ void write_images(const GridDev& g, int i, int j, int k, int64_t at, double v,
+                                             double* __restrict__ phi) {
+    const int q[3] = {i, j, k};
+    const int64_t st[3] = {(int64_t)g.gn[1] * g.gn[2], g.gn[2], 1};
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+        if (d >= g.dim || !g.periodic[d]) continue;
+        if (q[d] < g.ng) phi[at + g.n[d] * st[d]] = v;
+        if (q[d] >= g.n[d] - g.ng) phi[at - g.n[d] * st[d]] = v;
+    }
+}
 __global__ void __launch_bounds__(256) k_solution_to_field(GridDev g, const double* __restrict__ invd,
                                                            double* __restrict__ x, double* __restrict__ phi) {
     const int n0 = g.n[0], n1 = g.n[1], n2 = g.n[2];
-    const int64_t rows = (int64_t)n0 * n1;
-    const int64_t rstep = (int64_t)gridDim.x * blockDim.y;
     const bool hx = g.periodic[0], hy = g.dim > 1 && g.periodic[1], hz = g.dim > 2 && g.periodic[2];
-    for (int64_t r0 = (int64_t)blockIdx.x * blockDim.y + threadIdx.y; r0 < rows; r0 += kSolRows * rstep) {
+    const int64_t rows = (int64_t)n0 * n1;
+    const int64_t per = (rows + gridDim.x - 1) / gridDim.x;      // a block's run of rows
+    const int64_t ra = blockIdx.x * per, rb = ra + per < rows ? ra + per : rows;
+    if (ra >= rb) return;
+    int64_t r = ra + threadIdx.y;
+    int i = (int)(r / n1), j = (int)(r - (int64_t)i * n1);
+    const int by = blockDim.y, di = by / n1, dj = by - di * n1;
+    for (; r < rb; r += (int64_t)kSolRows * by) {
         for (int k = threadIdx.x; k < n2; k += blockDim.x) {
             double v[kSolRows], f[kSolRows];
 #pragma unroll
             for (int u = 0; u < kSolRows; u++) {
-                const int64_t r = r0 + u * rstep;
-                v[u] = r < rows ? x[r * n2 + k] : 0.;
-                if (invd) f[u] = r < rows ? invd[r * n2 + k] : 0.;
+                const bool in = r + u * by < rb;
+                v[u] = in ? x[(r + u * by) * n2 + k] : 0.;
+                f[u] = in && invd ? invd[(r + u * by) * n2 + k] : 0.;
             }
+            int iu = i, ju = j;
+            const bool hk = hz && (k < g.ng || k >= n2 - g.ng);
 #pragma unroll
             for (int u = 0; u < kSolRows; u++) {
-                const int64_t r = r0 + u * rstep;
-                if (r >= rows) break;
-                if (invd) {
-                    v[u] = f[u] * v[u];
-                    x[r * n2 + k] = v[u];
-                }
-                const int i = (int)(r / n1), j = (int)(r - (int64_t)i * n1);
-                const int q[3] = {i, j, k};
-                const int ind[3] = {i + g.og[0], j + g.og[1], k + g.og[2]};
-                phi[((int64_t)ind[0] * g.gn[1] + ind[1]) * g.gn[2] + ind[2]] = v[u];
-                if (!((hx && (i < g.ng || i >= n0 - g.ng)) || (hy && (j < g.ng || j >= n1 - g.ng)) ||
-                      (hz && (k < g.ng || k >= n2 - g.ng))))
-                    continue;
-                for (int d = 0; d < g.dim; d++) {
-                    if (!g.periodic[d]) continue;
-                    int t[3] = {ind[0], ind[1], ind[2]};
-                    if (q[d] < g.ng) {
-                        t[d] = g.og[d] + g.n[d] + q[d];
-                        phi[((int64_t)t[0] * g.gn[1] + t[1]) * g.gn[2] + t[2]] = v[u];
+                if (r + u * by < rb) {
+                    if (invd) {
+                        v[u] = f[u] * v[u];
+                        x[(r + u * by) * n2 + k] = v[u];
                     }
-                    if (q[d] >= g.n[d] - g.ng) {
-                        t[d] = q[d] - g.n[d] + g.ng;
-                        phi[((int64_t)t[0] * g.gn[1] + t[1]) * g.gn[2] + t[2]] = v[u];
-                    }
+                    const int64_t at = ((int64_t)(iu + g.og[0]) * g.gn[1] + ju + g.og[1]) * g.gn[2] + k + g.og[2];
+                    phi[at] = v[u];
+                    if (hk || (hx && (iu < g.ng || iu >= n0 - g.ng)) || (hy && (ju < g.ng || ju >= n1 - g.ng)))
+                        write_images(g, iu, ju, k, at, v[u], phi);
                 }
+                iu += di;
+                ju += dj;
+                if (ju >= n1) {
+                    ju -= n1;
+                    iu++;
+                }
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < kSolRows; u++) {
+            i += di;
+            j += dj;
+            if (j >= n1) {
+                j -= n1;
+                i++;
             }
         }
     }
