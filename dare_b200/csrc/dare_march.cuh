@@ -799,8 +799,9 @@ __global__ void __launch_bounds__(256, MarchMinBlocks<K, CPT>::value) k_march(Gr
             bool zv = pv;
             if constexpr (HALO) {
                 const int hside = p - G.cb < 0 ? 0 : (p - G.cb >= n0c ? 1 : -1);   // a plane past the slab
-                if (hside >= 0 && m.halo[z][hside]) {   // the neighbour's plane, exchanged into a local buffer
-                    src = static_cast<const T*>(m.halo[z][hside]) + (int64_t)(G.cb / n0c) * plane;   // [component][plane]
+                const void* nb = hside == 0 ? m.halo[z][0] : (hside == 1 ? m.halo[z][1] : nullptr);
+                if (nb) {   // the neighbour's plane, exchanged into a local buffer
+                    src = static_cast<const T*>(nb) + (int64_t)(G.cb / n0c) * plane;   // [component][plane]
                     zb = 0;
                     zv = true;
                 }
