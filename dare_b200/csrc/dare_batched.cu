@@ -484,6 +484,7 @@ __global__ void __launch_bounds__(1024, 1) k_boxes(const BInst* __restrict__ ins
     double* tile = reinterpret_cast<double*>(smem_raw);
     unsigned char* faces = smem_raw + (size_t)tile_cells * sizeof(double);
     ClusterTeam team = ClusterTeam::here(&sh);
+    team.start();
     for (;;) {
         if (team.rank == 0 && tid == 0) {
             const int next = (int)atomicAdd(queue, 1u);

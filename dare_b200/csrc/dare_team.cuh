@@ -203,7 +203,10 @@ struct ClusterTeam {
     int rank, size;
     unsigned set;
 
-    __device__ void start() {}
+    // Before the first store to another block's shared memory: the blocks of a
+    // cluster are placed together but need not have started together, and the
+    // shared memory of one that has not may not be touched.
+    __device__ void start() const { barrier(); }
     __device__ void stop() {}
     __device__ static ClusterTeam here(TeamShared* sh) {
         unsigned r, n;
