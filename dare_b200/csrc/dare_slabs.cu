@@ -536,9 +536,7 @@ int dare_slabs_solve(dare_slabs* sl, const dare_solver_params* p, dare_solve_rep
         dare_grid whole = *sl->grids[0];
         whole.dev.periodic[0] = view.sdev.periodic[0] = sl->global.periodic[0];
         view.grid = &whole;
-        dare_solver_params q = *p;
-        q.compute_true_residual = 0;   // a slab solve reports none
-        rc = dare_bicgstab2_fp64(&view, &q, rep);
+        rc = dare_bicgstab2_fp64(&view, p, rep);
         sl->systems[0]->ws = view.ws;
         return rc;
     }
