@@ -118,7 +118,8 @@ int dare_bicgstab2_refine(dare_system* s, const dare_solver_params* p, dare_solv
     double tol_abs = 0., rnorm = 0., prev = INFINITY;
     bool converged = false;
     int refinements = 0, inner_total = 0;
-    for (int it = 0; it <= p->max_refinements; it++) {
+    // (the first residual pass always runs: the tolerance and the fallback need its ||b||)
+    for (int it = 0; it == 0 || it <= p->max_refinements; it++) {
         // the inner FP32 BiCGStab2 on Ahat dy = r: relative tolerance, FP64 dots
         SolverState init{};
         init.tol = p->inner_rel_tol;
@@ -143,11 +144,11 @@ int dare_bicgstab2_refine(dare_system* s, const dare_solver_params* p, dare_solv
             tol_abs = p->tol_relative ? p->tol * norms[1] : p->tol;
             rep->tol_abs = tol_abs;
         }
-        if (rnorm <= tol_abs) {
+        if (rnorm <= tol_abs && p->max_refinements >= 0) {
             converged = true;
             break;
         }
-        if (!(rnorm < 0.5 * prev) || it == p->max_refinements) {  // not contracting (or NaN)
+        if (!(rnorm < 0.5 * prev) || it >= p->max_refinements) {  // not contracting (or NaN)
             break;
         }
         prev = rnorm;
