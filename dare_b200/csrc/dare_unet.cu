@@ -1711,7 +1711,8 @@ static int launch_wgr(dare_ctx* ctx, LaunchCfg& lc, int cin, int cout, const Wgr
 static int launch_wgr1(dare_ctx* ctx, LaunchCfg& lc, Wgr1Args a, size_t* part_need) {
     if (!lc.ready) {
         const size_t smem = wgr1_smem(a.g);
-        DARE_CUDA(ctx, cudaFuncSetAttribute(k_wgrad_1ch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        // (the limit is the kernel's, not this network's: a narrower network must not lower it)
+        DARE_CUDA(ctx, cudaFuncSetAttribute(k_wgrad_1ch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem));
         const int segs = (a.g.plane + kWgr1Seg - 1) / kWgr1Seg;
         lc.ppc = std::max(1, (int)((int64_t)a.g.n0 * segs / ((int64_t)ctx->num_sms * 4)));
         lc.tpg = kTaps;
