@@ -1095,17 +1095,8 @@ inline int launch_march_k(dare_ctx* ctx, const GridDev& g, const MarchCfg& m0, c
     const int ic = PAIR ? 16 / (int)sizeof(typename K::type) : m.cpt;   // first interior column of an operand row
     const size_t smem = MarchDepth<typename K::type>::value * march_stage_elems<K>(m.block.x * m.cpt, m.block.y, ic) *
                         sizeof(typename K::type);
-    static int per_sm = 0;
-    static size_t per_sm_smem = 0;
-    if (per_sm == 0 || per_sm_smem != smem) {
-        if (smem > 48 * 1024)
-            DARE_CUDA(ctx, cudaFuncSetAttribute(k_march<K, CPT, HALO, PAIR>,
-                                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_march<K, CPT, HALO, PAIR>, m.block.x * m.block.y,
-                                                      smem);
-        if (per_sm < 1) per_sm = 1;
-        per_sm_smem = smem;
-    }
+    int per_sm = 0;
+    DARE_CUDA(ctx, blocks_per_sm((const void*)k_march<K, CPT, HALO, PAIR>, m.block.x * m.block.y, smem, &per_sm));
     int blocks = per_sm * ctx->num_sms;
     if (m.nitems_total == 0) march_split(g, m, blocks, kMaxBlocks);   // (slabs share the slots of their runs)
     if (blocks > m.nitems) blocks = m.nitems;

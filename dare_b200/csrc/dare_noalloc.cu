@@ -138,14 +138,10 @@ extern "C" int dare_residual_norm_noalloc(int dim, const int64_t n[3], const int
     f.out = norm_out;
     const size_t smem = march_smem_bytes<FResidual<double>>(m);
     int per_sm = 0;
-    if (smem > 48 * 1024 &&
-        cudaFuncSetAttribute(k_march<FResidual<double>>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-            cudaSuccess) {
+    if (blocks_per_sm((const void*)k_march<FResidual<double>>, m.block.x * m.block.y, smem, &per_sm) != cudaSuccess) {
         cudaGetLastError();
         return fail(err, err_len, DARE_ERR_CUDA, "dare_residual_norm_noalloc: shared memory attribute");
     }
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_march<FResidual<double>>, m.block.x * m.block.y, smem);
-    if (per_sm < 1) per_sm = 1;
     int blocks = per_sm * num_sms;
     if (blocks > m.nitems) blocks = m.nitems;
     k_march<FResidual<double>><<<blocks, m.block, smem, sm>>>(g, f, st, partials, m);
