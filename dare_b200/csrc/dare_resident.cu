@@ -261,8 +261,8 @@ constexpr int64_t kClusterCells = 1 << 15;
 static size_t resident_smem(bool unit, int chunk, int sy) {
     return ((size_t)chunk * (unit ? 7 : 8) + 2 * (size_t)sy) * sizeof(double) + chunk;
 }
+constexpr size_t kResidentSmem = 227 * 1024 - sizeof(TeamShared) - sizeof(SolverState) - 1024;
 bool resident_shape(const dare_ctx* ctx, const GridDev& g, bool unit, int* blocks, int* chunk) {
-    constexpr size_t kMost = 227 * 1024 - sizeof(TeamShared) - sizeof(SolverState) - 1024;
     const int64_t n = g.ncell;
     const int nb = ctx->num_sms < kTeamMaxBlocks ? ctx->num_sms : kTeamMaxBlocks;
     if (n > (int64_t)nb * kResidentThreads * kResidentCells) return false;
@@ -275,7 +275,7 @@ bool resident_shape(const dare_ctx* ctx, const GridDev& g, bool unit, int* block
     if (want > most) want = most;
     int64_t ch = (n + want - 1) / want;
     ch = (ch + 31) / 32 * 32;
-    if (ch > kResidentThreads * kResidentCells || g.n[2] > (1 << 15) || resident_smem(unit, (int)ch, g.n[2]) > kMost)
+    if (ch > kResidentThreads * kResidentCells || g.n[2] > (1 << 15) || resident_smem(unit, (int)ch, g.n[2]) > kResidentSmem)
         return false;
     *chunk = (int)ch;
     *blocks = (int)((n + ch - 1) / ch);
@@ -285,9 +285,11 @@ bool resident_shape(const dare_ctx* ctx, const GridDev& g, bool unit, int* block
 template <bool UNIT, int CPT>
 static int launch_resident_t(dare_ctx* ctx, ResidentArgs& a, int blocks) {
     const size_t smem = resident_smem(UNIT, a.chunk, a.geo.sy);
+    // (the kernels' limit is the most that any system takes, not this one's need:
+    // it belongs to the kernel, and other threads launch it for other systems)
     if (blocks <= kClusterMaxBlocks) {
         const auto k = k_resident<UNIT, CPT, true>;
-        DARE_CUDA(ctx, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        DARE_CUDA(ctx, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kResidentSmem));
         DARE_CUDA(ctx, cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
         cudaLaunchAttribute at[1];
         at[0].id = cudaLaunchAttributeClusterDimension;
@@ -305,7 +307,7 @@ static int launch_resident_t(dare_ctx* ctx, ResidentArgs& a, int blocks) {
         return DARE_OK;
     }
     const auto k = k_resident<UNIT, CPT, false>;
-    DARE_CUDA(ctx, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    DARE_CUDA(ctx, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kResidentSmem));
     void* args[] = {&a};
     DARE_CUDA(ctx, cudaLaunchCooperativeKernel((const void*)k, dim3(blocks), dim3(kResidentThreads), args, smem,
                                                ctx->stream));
