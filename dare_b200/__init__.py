@@ -90,6 +90,8 @@ _SIGS = [
     ("dare_ctx_set_stream", C.c_int, [_P, _P]),
     ("dare_ctx_get_stream", _P, [_P]),
     ("dare_ctx_synchronize", C.c_int, [_P]),
+    ("dare_ctx_set_wait_limit", C.c_int, [_P, C.c_int64]),
+    ("dare_ctx_debug_give_up", C.c_int, [_P, C.c_int]),
     ("dare_ctx_last_error", C.c_char_p, [_P]),
     ("dare_ctx_launch_count", C.c_int64, [_P]),
     ("dare_ctx_set_profiling", C.c_int, [_P, C.c_int]),
@@ -298,6 +300,14 @@ class Context:
 
     def set_stream(self, stream_ptr: int | None):
         _check(lib().dare_ctx_set_stream(self.h, stream_ptr), self.h, "set_stream")
+
+    def set_wait_limit(self, polls: int):
+        """Polls after which a wait between the blocks of a one-launch solve gives up (0: the default)."""
+        _check(lib().dare_ctx_set_wait_limit(self.h, polls), self.h, "set_wait_limit")
+
+    def debug_give_up(self, block: int):
+        """Test hook: this block gives up at its first exchange of the next one-launch solve."""
+        _check(lib().dare_ctx_debug_give_up(self.h, block), self.h, "debug_give_up")
 
     @property
     def stream(self) -> int:

@@ -106,7 +106,8 @@ int ensure_solver_ws(dare_system* s) {
         ws->st = reinterpret_cast<SolverState*>(base + at_st);
         e = cudaMemsetAsync(ws->team_buf, 0, total - at_team, ctx->stream);
     }
-    if (e == cudaSuccess) e = cudaMallocHost(&ws->st_host, sizeof(SolverState));
+    if (e == cudaSuccess) e = cudaMallocHost(&ws->st_host, sizeof(SolverState) + sizeof(int));
+    if (e == cudaSuccess) ws->gave_up = reinterpret_cast<int*>(ws->st_host + 1);
     if (e != cudaSuccess) {
         dare_solver_ws_free(ws);
         return check_cuda(ctx, e, "bicgstab2 workspace");
@@ -400,7 +401,7 @@ int dare_bicgstab2_fp64_to(dare_system* s, const dare_solver_params* p, dare_sol
             ctx->stat_ms[KID_SOLVE] += ms;
             ctx->stat_n[KID_SOLVE] += 1;
         }
-        if (!ws->st_host->done) {   // a wait between its blocks ran out: start the exchanges over
+        if (*ws->gave_up) {   // a wait between its blocks ran out: start the exchanges over
             DARE_CUDA(ctx, cudaMemsetAsync(ws->team_buf, 0, sizeof(TeamBuffer), ctx->stream));
             return set_error(ctx, DARE_ERR_TIMEOUT, "bicgstab2: a wait between blocks ran out");
         }

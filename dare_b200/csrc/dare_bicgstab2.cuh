@@ -189,6 +189,7 @@ struct dare_solver_ws {
     double* partials = nullptr;  // kMaxQ * kMaxBlocks (+ scratch)
     dare_gpu::SolverState* st = nullptr;
     dare_gpu::SolverState* st_host = nullptr;  // pinned
+    int* gave_up = nullptr;                    // pinned, after st_host (dare_resident.cu)
     cudaGraphExec_t graph[3][2] = {{nullptr, nullptr}, {nullptr, nullptr}, {nullptr, nullptr}};
     dare_gpu::MarchCfg march;
     int stream_blocks = 0;

@@ -323,6 +323,18 @@ int dare_ctx_destroy(dare_ctx* ctx) {
     return DARE_OK;
 }
 
+int dare_ctx_set_wait_limit(dare_ctx* ctx, int64_t polls) {
+    if (!ctx || polls < 0 || polls > 0x7FFFFFFFll) return DARE_ERR_BAD_ARG;
+    ctx->team_polls = (int)polls;
+    return DARE_OK;
+}
+
+int dare_ctx_debug_give_up(dare_ctx* ctx, int block) {
+    if (!ctx) return DARE_ERR_BAD_ARG;
+    ctx->debug_quitter = block;
+    return DARE_OK;
+}
+
 int dare_ctx_set_stream(dare_ctx* ctx, void* stream) {
     if (!ctx) return DARE_ERR_BAD_ARG;
     ctx->stream = stream ? (cudaStream_t)stream : ctx->own_stream;

@@ -70,6 +70,9 @@ struct dare_ctx {
     cudaStream_t stream = nullptr;
     std::string last_error;
     int64_t launches = 0;
+    // waits between the blocks of a one-launch solve (dare_ctx_set_wait_limit,
+    // dare_ctx_debug_give_up)
+    int team_polls = 0, debug_quitter = -1;
     // per-kernel CUDA-event timing (dare_ctx_set_profiling)
     int profiling = 0;
     cudaEvent_t ev[16] = {nullptr};

@@ -32,7 +32,9 @@ struct ResidentArgs {
     double tol;
     int max_it, tol_relative, want_residual;
     TeamBuffer* buf;
+    int polls, quitter;            // limit of a block's waits; the block whose limit is 0 (-1: none)
     SolverState *st, *st_host;     // results (device copy, pinned host copy)
+    int* gave_up;                  // pinned host word that a block sets when a wait of it ran out
 };
 
 // 1024 threads and one block per SM: 64 registers each, and 32 warps to hide
@@ -142,7 +144,8 @@ __global__ void __launch_bounds__(kResidentThreads, 1) k_resident(ResidentArgs A
         if constexpr (CLUSTER)
             return ClusterTeam::here(&sh);
         else
-            return GridTeam{A.buf, &sh, (int)blockIdx.x, (int)gridDim.x, 0u};
+            return GridTeam{A.buf, &sh, (int)blockIdx.x, (int)gridDim.x, (int)blockIdx.x == A.quitter ? 0 : A.polls,
+                            0u};
     };
     auto team = make_team();
     team.start();
@@ -242,10 +245,12 @@ __global__ void __launch_bounds__(kResidentThreads, 1) k_resident(ResidentArgs A
             }
         }
     }
-    // a block that gave up leaves `done` 0 in its copy; block 0 reports
+    // Block 0 reports the state, and every block whose wait ran out says so
+    // itself: at the last exchange block 0 may get the total that another one
+    // has given up waiting for, with its cells unfinished.
     team.stop();
+    if (!ok && tid == 0) *A.gave_up = 1;
     if (blockIdx.x == 0 && tid == 0) {
-        if (!ok) st->done = 0;
         *A.st = *st;
         *A.st_host = *st;
     }
@@ -346,8 +351,13 @@ int launch_resident(dare_system* s, const dare_solver_params* p, const VecsT<dou
     a.tol_relative = p->tol_relative;
     a.want_residual = p->compute_true_residual;
     a.buf = static_cast<TeamBuffer*>(ws->team_buf);
+    a.polls = ctx->team_polls > 0 ? ctx->team_polls : kTeamPolls;
+    a.quitter = ctx->debug_quitter;
+    ctx->debug_quitter = -1;
     a.st = ws->st;
     a.st_host = ws->st_host;
+    a.gave_up = ws->gave_up;
+    *ws->gave_up = 0;   // (no kernel of this workspace is running)
     return p->precond == DARE_PREC_JACOBI ? launch_resident_u<true>(ctx, a, blocks)
                                           : launch_resident_u<false>(ctx, a, blocks);
 }

@@ -23,7 +23,7 @@ namespace dare_gpu {
 
 constexpr int kTeamMaxBlocks = 160;   // blocks of a grid team
 constexpr int kClusterMaxBlocks = 16; // blocks of a cluster team (the largest cluster)
-constexpr int kTeamPolls = 1 << 22;   // polls of a wait before the block gives up
+constexpr int kTeamPolls = 1 << 22;   // polls of a wait before the block gives up, unless the context has a limit of its own
 
 __device__ __forceinline__ double team_xor(double v, int o) { return __shfl_xor_sync(0xffffffffu, v, o); }
 
@@ -116,12 +116,13 @@ struct TeamShared {
 // blocks that all read all 148 partial sums queue at the few L2 slices that
 // hold them (4000 cycles on top of 1200, every other exchange), which is why
 // one does.
-// Every wait ends: after kTeamPolls polls the block gives up, and so do the
-// blocks that wait for it.
+// Every wait ends: after `limit` polls the block gives up, and so do the
+// blocks that wait for it.  (limit 0, a test's: it gives up at its first
+// exchange, after counting itself in.)
 struct GridTeam {
     TeamBuffer* buf;
     TeamShared* sh;
-    int rank, size;
+    int rank, size, limit;
     unsigned set;   // partial-sum set of the last exchange
 
     __device__ void start() {   // before the block's first barrier
@@ -182,10 +183,11 @@ struct GridTeam {
                     asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(hi) : "l"(total + 1) : "memory");
                     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(have) : "l"(n) : "memory");
                     wait = (unsigned)(lo >> 32) != target || (unsigned)(hi >> 32) != target || (int)(have - target) < 0;
-                } while (wait && ++polls < kTeamPolls);
+                } while (wait && ++polls < limit);
                 if (wait) sh->timeout = 1;
                 sh->tot[wid] = __longlong_as_double((long long)((lo & 0xffffffffull) | (hi << 32)));
             }
+            if (limit == 0 && lane == 0) sh->timeout = 1;
         }
         if (Q > 1) __syncthreads();   // (one value: thread 0's own warp)
         if (threadIdx.x == 0 && !sh->timeout) fin(sh->tot);

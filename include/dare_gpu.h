@@ -193,6 +193,14 @@ DARE_API int dare_ctx_destroy(dare_ctx* ctx);
 DARE_API int dare_ctx_set_stream(dare_ctx* ctx, void* stream);
 DARE_API void* dare_ctx_get_stream(dare_ctx* ctx);
 DARE_API int dare_ctx_synchronize(dare_ctx* ctx);
+/* Polls after which a wait between the thread blocks of a solve that runs as
+ * one kernel gives up; 0 restores the default (seconds).  The solve then
+ * returns DARE_ERR_TIMEOUT, with the solution undefined, and the next one
+ * starts clean. */
+DARE_API int dare_ctx_set_wait_limit(dare_ctx* ctx, int64_t polls);
+/* Test hook: in the next such solve on the whole device, thread block `block`
+ * gives up at its first exchange. */
+DARE_API int dare_ctx_debug_give_up(dare_ctx* ctx, int block);
 DARE_API const char* dare_ctx_last_error(const dare_ctx* ctx);
 /* Kernel launches this context issued since creation (for launch accounting). */
 DARE_API int64_t dare_ctx_launch_count(const dare_ctx* ctx);
