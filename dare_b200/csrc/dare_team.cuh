@@ -154,6 +154,7 @@ struct GridTeam {
                 asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(old) : "l"(n) : "memory");
             }
             if (__shfl_sync(0xffffffffu, old + 1u == target, 0)) {
+                __syncwarp();   // lane 0 has acquired the others' sums: now every lane may read them
                 double s = 0.;
                 for (int b = lane; b < size; b += 32) {
                     double p;
