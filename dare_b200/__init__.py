@@ -91,6 +91,7 @@ _SIGS = [
     ("dare_ctx_get_stream", _P, [_P]),
     ("dare_ctx_synchronize", C.c_int, [_P]),
     ("dare_ctx_set_wait_limit", C.c_int, [_P, C.c_int64]),
+    ("dare_ctx_set_team_blocks", C.c_int, [_P, C.c_int, C.c_int]),
     ("dare_ctx_debug_give_up", C.c_int, [_P, C.c_int]),
     ("dare_ctx_last_error", C.c_char_p, [_P]),
     ("dare_ctx_launch_count", C.c_int64, [_P]),
@@ -304,6 +305,11 @@ class Context:
     def set_wait_limit(self, polls: int):
         """Polls after which a wait between the blocks of a one-launch solve gives up (0: the default)."""
         _check(lib().dare_ctx_set_wait_limit(self.h, polls), self.h, "set_wait_limit")
+
+    def set_team_blocks(self, cluster: int = -1, grid: int = -1):
+        """The most thread blocks a one-launch solve takes in a cluster and over
+        the device (negative: as many as the device holds; 0: none)."""
+        _check(lib().dare_ctx_set_team_blocks(self.h, cluster, grid), self.h, "set_team_blocks")
 
     def debug_give_up(self, block: int):
         """Test hook: this block gives up at its first exchange of the next one-launch solve."""

@@ -389,11 +389,11 @@ int dare_bicgstab2_fp64_to(dare_system* s, const dare_solver_params* p, dare_sol
     bool field_current = to_field;
     double* tres = &ws->st->tres;
     // Small systems run in one launch (timed as one kernel when profiling)
-    int blocks = 0, chunk = 0;
-    if (resident_shape(ctx, g, jacobi, &blocks, &chunk)) {
+    const ResidentPlan& plan = resident_plan(ctx, g, jacobi, ws);
+    if (plan.blocks > 0) {
         const bool prof = ctx->profiling != 0;
         if (prof) DARE_CUDA(ctx, cudaEventRecord(ctx->ev[0], ctx->stream));
-        if ((rc = launch_resident(s, p, vs, blocks, chunk, to_field ? f->level[0] : nullptr))) return rc;
+        if ((rc = launch_resident(s, p, vs, plan, to_field ? f->level[0] : nullptr))) return rc;
         if (prof) DARE_CUDA(ctx, cudaEventRecord(ctx->ev[1], ctx->stream));
         DARE_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
         float ms = 0.f;

@@ -170,8 +170,13 @@ int launch_fold32(dare_ctx* ctx, const GridDev& g, const MarchCfg& m, const doub
                   SolverState* st, double* partials);
 int launch_scale(dare_ctx* ctx, int64_t n, const double* invd, double* x);
 // The one-launch solve of small systems (dare_resident.cu)
-bool resident_shape(const dare_ctx* ctx, const GridDev& g, bool unit, int* blocks, int* chunk);
-int launch_resident(dare_system* s, const dare_solver_params* p, const VecsT<double>& vs, int blocks, int chunk,
+struct ResidentPlan {
+    bool known = false, cluster = false;       // cluster: one cluster, else a cooperative launch
+    int most_cluster = -1, most_grid = -1;     // the context's limits it was made for
+    int blocks = 0, chunk = 0;                 // blocks (0: no such solve), cells of each
+};
+const ResidentPlan& resident_plan(const dare_ctx* ctx, const GridDev& g, bool unit, dare_solver_ws* ws);
+int launch_resident(dare_system* s, const dare_solver_params* p, const VecsT<double>& vs, const ResidentPlan& plan,
                     double* field);
 // Apply step (10) when the solve stopped between it and the last kernel of
 // its iteration (st_host: the final state read back)
@@ -190,6 +195,7 @@ struct dare_solver_ws {
     dare_gpu::SolverState* st = nullptr;
     dare_gpu::SolverState* st_host = nullptr;  // pinned
     int* gave_up = nullptr;                    // pinned, after st_host (dare_resident.cu)
+    dare_gpu::ResidentPlan resident[2];        // without, with Jacobi
     cudaGraphExec_t graph[3][2] = {{nullptr, nullptr}, {nullptr, nullptr}, {nullptr, nullptr}};
     dare_gpu::MarchCfg march;
     int stream_blocks = 0;

@@ -329,6 +329,13 @@ int dare_ctx_set_wait_limit(dare_ctx* ctx, int64_t polls) {
     return DARE_OK;
 }
 
+int dare_ctx_set_team_blocks(dare_ctx* ctx, int cluster_blocks, int grid_blocks) {
+    if (!ctx) return DARE_ERR_BAD_ARG;
+    ctx->team_cluster = cluster_blocks;
+    ctx->team_grid = grid_blocks;
+    return DARE_OK;
+}
+
 int dare_ctx_debug_give_up(dare_ctx* ctx, int block) {
     if (!ctx) return DARE_ERR_BAD_ARG;
     ctx->debug_quitter = block;

@@ -73,6 +73,9 @@ struct dare_ctx {
     // waits between the blocks of a one-launch solve (dare_ctx_set_wait_limit,
     // dare_ctx_debug_give_up)
     int team_polls = 0, debug_quitter = -1;
+    // the most blocks of a one-launch solve, in one cluster and over the device
+    // (dare_ctx_set_team_blocks; negative: what the device holds)
+    int team_cluster = -1, team_grid = -1;
     // per-kernel CUDA-event timing (dare_ctx_set_profiling)
     int profiling = 0;
     cudaEvent_t ev[16] = {nullptr};

@@ -13,6 +13,7 @@
 // 172 us.  What is left of a pass with its exchange (64^3, 6 us): forming the
 // operand 1.8 us, the rows 1 us, the block's sum 0.4 us, publishing it 1.1 us
 // and the total coming back 1.9 us, all of them L2 round trips of ~0.5 us.
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 
@@ -256,82 +257,108 @@ __global__ void __launch_bounds__(kResidentThreads, 1) k_resident(ResidentArgs A
     }
 }
 
-// The team's shape for a system, or false when a block's rows do not fit its
-// shared memory: beyond that the marching kernels are the faster path (their
-// vectors no longer stay in L2 either).
 constexpr int kResidentCells = 4;   // most cells a thread
 // Measured solves, cluster / device: 24^3 43 / 59 us, 32^3 58 / 60, 36^3 94 / 83;
 // two species on 90^2 76 / 103, 120^2 113 / 128, 160^2 211 / 168
 constexpr int64_t kClusterCells = 1 << 15;
+constexpr size_t kResidentSmem = 227 * 1024 - sizeof(TeamShared) - sizeof(SolverState) - 1024;
 static size_t resident_smem(bool unit, int chunk, int sy) {
     return ((size_t)chunk * (unit ? 7 : 8) + 2 * (size_t)sy) * sizeof(double) + chunk;
 }
-constexpr size_t kResidentSmem = 227 * 1024 - sizeof(TeamShared) - sizeof(SolverState) - 1024;
-bool resident_shape(const dare_ctx* ctx, const GridDev& g, bool unit, int* blocks, int* chunk) {
-    const int64_t n = g.ncell;
-    const int nb = ctx->num_sms < kTeamMaxBlocks ? ctx->num_sms : kTeamMaxBlocks;
-    if (n > (int64_t)nb * kResidentThreads * kResidentCells) return false;
-    // Up to kClusterCells cells one cluster, whose exchanges take 1 us where
-    // the device's take 3; beyond that the device, whose passes are shorter.
-    // As many blocks as have a cell for each of half their threads: below
-    // that an SM more does not shorten a pass.
-    int64_t want = (n + kResidentThreads / 2 - 1) / (kResidentThreads / 2);
-    const int64_t most = n <= kClusterCells ? kClusterMaxBlocks : nb;
-    if (want > most) want = most;
-    int64_t ch = (n + want - 1) / want;
-    ch = (ch + 31) / 32 * 32;
-    if (ch > kResidentThreads * kResidentCells || g.n[2] > (1 << 15) || resident_smem(unit, (int)ch, g.n[2]) > kResidentSmem)
-        return false;
-    *chunk = (int)ch;
-    *blocks = (int)((n + ch - 1) / ch);
-    return true;
+
+template <bool UNIT, bool CLUSTER>
+static const void* resident_kernel_t(int chunk) {
+    switch ((chunk + kResidentThreads - 1) / kResidentThreads) {
+    case 1: return (const void*)k_resident<UNIT, 1, CLUSTER>;
+    case 2: return (const void*)k_resident<UNIT, 2, CLUSTER>;
+    case 3: return (const void*)k_resident<UNIT, 3, CLUSTER>;
+    default: return (const void*)k_resident<UNIT, kResidentCells, CLUSTER>;
+    }
+}
+static const void* resident_kernel(bool unit, const ResidentPlan& P) {
+    if (unit) return P.cluster ? resident_kernel_t<true, true>(P.chunk) : resident_kernel_t<true, false>(P.chunk);
+    return P.cluster ? resident_kernel_t<false, true>(P.chunk) : resident_kernel_t<false, false>(P.chunk);
+}
+static cudaLaunchConfig_t resident_config(const dare_ctx* ctx, const ResidentPlan& P, size_t smem,
+                                          cudaLaunchAttribute* at) {
+    if (P.cluster) {
+        at->id = cudaLaunchAttributeClusterDimension;
+        at->val.clusterDim.x = (unsigned)P.blocks;
+        at->val.clusterDim.y = at->val.clusterDim.z = 1;
+    } else {
+        at->id = cudaLaunchAttributeCooperative;
+        at->val.cooperative = 1;
+    }
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3(P.blocks);
+    c.blockDim = dim3(kResidentThreads);
+    c.dynamicSmemBytes = smem;
+    c.stream = ctx->stream;
+    c.attrs = at;
+    c.numAttrs = 1;
+    return c;
+}
+// (the kernels' limit is the most that any system takes, not one system's need:
+// it belongs to the kernel, and other threads launch it for other systems)
+static cudaError_t resident_limits(const void* k, bool cluster) {
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kResidentSmem);
+    if (e == cudaSuccess && cluster) e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    return e;
 }
 
-template <bool UNIT, int CPT>
-static int launch_resident_t(dare_ctx* ctx, ResidentArgs& a, int blocks) {
-    const size_t smem = resident_smem(UNIT, a.chunk, a.geo.sy);
-    // (the kernels' limit is the most that any system takes, not this one's need:
-    // it belongs to the kernel, and other threads launch it for other systems)
-    if (blocks <= kClusterMaxBlocks) {
-        const auto k = k_resident<UNIT, CPT, true>;
-        DARE_CUDA(ctx, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kResidentSmem));
-        DARE_CUDA(ctx, cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-        cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = (unsigned)blocks;
-        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-        cudaLaunchConfig_t c{};
-        c.gridDim = dim3(blocks);
-        c.blockDim = dim3(kResidentThreads);
-        c.dynamicSmemBytes = smem;
-        c.stream = ctx->stream;
-        c.attrs = at;
-        c.numAttrs = 1;
-        DARE_CUDA(ctx, cudaLaunchKernelEx(&c, k, a));
-        DARE_LAUNCHED(ctx);
-        return DARE_OK;
-    }
-    const auto k = k_resident<UNIT, CPT, false>;
-    DARE_CUDA(ctx, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kResidentSmem));
-    void* args[] = {&a};
-    DARE_CUDA(ctx, cudaLaunchCooperativeKernel((const void*)k, dim3(blocks), dim3(kResidentThreads), args, smem,
-                                               ctx->stream));
-    DARE_LAUNCHED(ctx);
-    return DARE_OK;
+// A team of at most `most` blocks: as many as have a cell for each of half
+// their threads (below that an SM more does not shorten a pass).  False when a
+// block's rows do not fit its shared memory, or the device (or this process's
+// share of it) cannot hold the team's blocks at the same time.
+static bool resident_team(const dare_ctx* ctx, const GridDev& g, bool unit, bool cluster, int64_t most,
+                          ResidentPlan& P) {
+    const int64_t n = g.ncell;
+    if (most < 1 || n > most * kResidentThreads * kResidentCells || g.n[2] > (1 << 15)) return false;
+    const int64_t want = std::min(most, (n + kResidentThreads / 2 - 1) / (kResidentThreads / 2));
+    const int64_t ch = ((n + want - 1) / want + 31) / 32 * 32;
+    const size_t smem = resident_smem(unit, (int)ch, g.n[2]);
+    if (ch > kResidentThreads * kResidentCells || smem > kResidentSmem) return false;
+    P.cluster = cluster;
+    P.chunk = (int)ch;
+    P.blocks = (int)((n + ch - 1) / ch);
+    const void* k = resident_kernel(unit, P);
+    cudaLaunchAttribute at[1];
+    const cudaLaunchConfig_t c = resident_config(ctx, P, smem, at);
+    int fit = 0;
+    cudaError_t e = resident_limits(k, cluster);
+    if (e == cudaSuccess)
+        e = cluster ? cudaOccupancyMaxActiveClusters(&fit, k, &c)
+                    : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, k, kResidentThreads, smem);
+    if (e != cudaSuccess) cudaGetLastError();
+    if (e == cudaSuccess && (cluster ? fit >= 1 : (int64_t)fit * ctx->num_sms >= P.blocks)) return true;
+    P.blocks = 0;
+    return false;
 }
-template <bool UNIT>
-static int launch_resident_u(dare_ctx* ctx, ResidentArgs& a, int blocks) {
-    switch ((a.chunk + kResidentThreads - 1) / kResidentThreads) {
-    case 1: return launch_resident_t<UNIT, 1>(ctx, a, blocks);
-    case 2: return launch_resident_t<UNIT, 2>(ctx, a, blocks);
-    case 3: return launch_resident_t<UNIT, 3>(ctx, a, blocks);
-    default: return launch_resident_t<UNIT, kResidentCells>(ctx, a, blocks);
-    }
+
+// The team that solves a system in one launch, found at its first solve;
+// blocks = 0 when there is none, and the marching kernels solve it (beyond that
+// size they are the faster path, their vectors no longer stay in L2 either).
+// Up to kClusterCells cells one cluster, whose exchanges take 1 us where the
+// device's take 3; beyond that, or without room for the cluster, blocks of the
+// whole device, whose passes are shorter.
+const ResidentPlan& resident_plan(const dare_ctx* ctx, const GridDev& g, bool unit, dare_solver_ws* ws) {
+    ResidentPlan& P = ws->resident[unit];
+    if (P.known && P.most_cluster == ctx->team_cluster && P.most_grid == ctx->team_grid) return P;
+    P = ResidentPlan{};
+    P.most_cluster = ctx->team_cluster;
+    P.most_grid = ctx->team_grid;
+    const auto at_most = [](int blocks, int limit) { return limit < 0 ? blocks : std::min(blocks, limit); };
+    const bool found = (g.ncell <= kClusterCells &&
+                        resident_team(ctx, g, unit, true, at_most(kClusterMaxBlocks, P.most_cluster), P)) ||
+                       resident_team(ctx, g, unit, false, at_most(std::min(ctx->num_sms, kTeamMaxBlocks), P.most_grid), P);
+    if (!found) P.blocks = 0;
+    P.known = true;
+    return P;
 }
 
 // The whole solve of system s in one launch: x (and field level 0 when given)
 // and the final state, in ws->st_host once the stream is synchronized.
-int launch_resident(dare_system* s, const dare_solver_params* p, const VecsT<double>& vs, int blocks, int chunk,
+int launch_resident(dare_system* s, const dare_solver_params* p, const VecsT<double>& vs, const ResidentPlan& P,
                     double* field) {
     dare_ctx* ctx = s->grid->ctx;
     dare_solver_ws* ws = s->ws;
@@ -340,7 +367,7 @@ int launch_resident(dare_system* s, const dare_solver_params* p, const VecsT<dou
     a.geo = team_geo(g);
     a.grid = s->grid->dev;
     a.ncell = (int)g.ncell;
-    a.chunk = chunk;
+    a.chunk = P.chunk;
     a.diag = s->diag;
     a.b = s->rhs;
     a.invd = ws->invd;
@@ -358,8 +385,15 @@ int launch_resident(dare_system* s, const dare_solver_params* p, const VecsT<dou
     a.st_host = ws->st_host;
     a.gave_up = ws->gave_up;
     *ws->gave_up = 0;   // (no kernel of this workspace is running)
-    return p->precond == DARE_PREC_JACOBI ? launch_resident_u<true>(ctx, a, blocks)
-                                          : launch_resident_u<false>(ctx, a, blocks);
+    const bool unit = p->precond == DARE_PREC_JACOBI;
+    const void* k = resident_kernel(unit, P);
+    cudaLaunchAttribute at[1];
+    const cudaLaunchConfig_t c = resident_config(ctx, P, resident_smem(unit, P.chunk, a.geo.sy), at);
+    void* args[] = {&a};
+    DARE_CUDA(ctx, resident_limits(k, P.cluster));
+    DARE_CUDA(ctx, cudaLaunchKernelExC(&c, k, args));
+    DARE_LAUNCHED(ctx);
+    return DARE_OK;
 }
 
 }  // namespace dare_gpu

@@ -198,6 +198,13 @@ DARE_API int dare_ctx_synchronize(dare_ctx* ctx);
  * returns DARE_ERR_TIMEOUT, with the solution undefined, and the next one
  * starts clean. */
 DARE_API int dare_ctx_set_wait_limit(dare_ctx* ctx, int64_t polls);
+/* The most thread blocks that a solve which runs as one kernel takes: of one
+ * thread-block cluster (small systems, the boxes of a batch) and of a
+ * cooperative launch (larger ones).  Negative: as many as the device holds;
+ * 0: none, such systems are then solved by the kernels for larger ones.  The
+ * blocks of such a solve are resident until it ends, so a limit leaves room
+ * for other work on the device. */
+DARE_API int dare_ctx_set_team_blocks(dare_ctx* ctx, int cluster_blocks, int grid_blocks);
 /* Test hook: in the next such solve on the whole device, thread block `block`
  * gives up at its first exchange. */
 DARE_API int dare_ctx_debug_give_up(dare_ctx* ctx, int block);
