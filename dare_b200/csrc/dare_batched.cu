@@ -74,6 +74,7 @@ struct dare_batch {
     size_t class_smem[dare_gpu::kBoxClasses] = {0};
     int class_clusters[dare_gpu::kBoxClasses] = {0};        // resident at a time (0: not asked yet) ...
     int clusters_block = 0;                                  // ... with this block size
+    int classes = -1, most_cluster = -1;     // cluster sizes in use, for this limit of the context's
     dare_gpu::BInst* d_inst = nullptr;
     int* d_order = nullptr;
     dare_gpu::BOut* d_out = nullptr;
@@ -686,8 +687,41 @@ static size_t box_smem(int64_t tile) { return (size_t)(tile + 15) / 16 * 16 * (s
 // exchanges show, more and the box's eight vectors times the boxes in flight
 // leave L2.  Batches too small to fill the device take larger clusters, down
 // to a block of 512 cells.
+// Cluster sizes that the device holds, asked for with the most threads and
+// shared memory a block may take (larger boxes, and all where it holds none, go
+// to k_batched), and that the context allows.
+static int box_classes(const dare_ctx* ctx) {
+    const auto kern = k_boxes;
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBoxSmem);
+    cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.blockDim = dim3(1024);
+    cfg.dynamicSmemBytes = kBoxSmem;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int c = kBoxClasses;
+    for (; c > 0; c--) {
+        const int blocks = 1 << (c - 1);
+        if (ctx->team_cluster >= 0 && blocks > ctx->team_cluster) continue;
+        at[0].val.clusterDim.x = (unsigned)blocks;
+        cfg.gridDim = dim3((unsigned)blocks);
+        int fit = 0;
+        if (cudaOccupancyMaxActiveClusters(&fit, kern, &cfg) == cudaSuccess && fit >= 1) break;
+    }
+    cudaGetLastError();   // a size that does not fit is an answer
+    return c;
+}
+
 static int upload_instances(dare_batch* bt) {
     dare_ctx* ctx = bt->ctx;
+    if (bt->classes < 0 || bt->most_cluster != ctx->team_cluster) {
+        bt->classes = box_classes(ctx);
+        bt->most_cluster = ctx->team_cluster;
+    }
+    const int nc = bt->classes;
     std::vector<int> cls(bt->count);
     for (int grow = 0;; grow++) {
         int64_t blocks = 0;
@@ -697,11 +731,13 @@ static int upload_instances(dare_batch* bt) {
             const int64_t cells = (int64_t)I.n0 * I.n1 * I.n2, plane = (int64_t)I.n1 * I.n2;
             I.vec = bt->vec_by_size[size_class(std::max(I.n0, std::max(I.n1, I.n2)))];
             int c = 0;
-            while (c < kBoxClasses - 1 && cells > ((int64_t)4096 * I.vec << c)) c++;
-            while (c < kBoxClasses && box_smem(box_tile(cells, plane, box_chunk(cells, 1 << c))) > kBoxSmem) c++;
-            if (c < kBoxClasses)
-                for (int k = 0; k < grow && c < kBoxClasses - 1 && cells >= (int64_t)1024 << c; k++) c++;
-            if (c < kBoxClasses - 1 && cells >= (int64_t)1024 << c) more = true;
+            while (c < nc - 1 && cells > ((int64_t)4096 * I.vec << c)) c++;
+            while (c < nc && box_smem(box_tile(cells, plane, box_chunk(cells, 1 << c))) > kBoxSmem) c++;
+            if (c < nc)
+                for (int k = 0; k < grow && c < nc - 1 && cells >= (int64_t)1024 << c; k++) c++;
+            else
+                c = kBoxClasses;
+            if (c < nc - 1 && cells >= (int64_t)1024 << c) more = true;
             cls[q] = c;
             I.chunk = c < kBoxClasses ? (int)box_chunk(cells, 1 << c) : 0;
             blocks += c < kBoxClasses ? 1 << c : 1;
@@ -785,6 +821,8 @@ static int launch_class(dare_batch* bt, int c, const BVecs& vs, const BParams& p
 // the others on the batch's own between two events.
 static int launch_batch(dare_batch* bt, const dare_solver_params* p, int block) {
     dare_ctx* ctx = bt->ctx;
+    if (bt->most_cluster != ctx->team_cluster)   // the context's limit has changed
+        if (int rc = upload_instances(bt)) return rc;
     BVecs vs;
     double* base = bt->arena;
     const int64_t T = bt->total;
