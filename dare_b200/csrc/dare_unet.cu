@@ -2254,6 +2254,28 @@ static int ensure_lane(dare_unet* net, int l) {
     return DARE_OK;
 }
 
+// The lanes of a minibatch of `count` pairs with their buffers: as many as the
+// device has room for, the network itself at least.  All that a minibatch
+// allocates is allocated here, outside any stream capture.
+static int prepare_lanes(dare_unet* net, int count, int* lanes) {
+    int rc = ensure_part(net);
+    if (rc) return rc;
+    const int want = lanes_for(net, count);
+    int l = 1;
+    for (; l < want; l++) {
+        const bool had = net->lane[l];
+        if ((rc = ensure_lane(net, l)) == DARE_OK && (rc = ensure_part(&net->lane[l]->net)) && !had) {
+            free_lane(net->lane[l]);
+            net->lane[l] = nullptr;
+        }
+        if (rc) break;
+    }
+    if (rc && rc != DARE_ERR_OOM) return rc;
+    if (rc) cudaGetLastError();   // no room for another lane is an answer
+    *lanes = l;
+    return DARE_OK;
+}
+
 // out = ((g[0] + g[1]) + ...), the lanes' gradients in the order of their first pairs
 struct LaneGrads {
     const float* g[kLanes];
@@ -2267,26 +2289,23 @@ __global__ void __launch_bounds__(256) k_sum_grads(int64_t n, LaneGrads s, float
     }
 }
 
-// Queues the loss (dscal[0]) and its mean gradient over `count` pairs; grad is
-// zeroed first.  Pair b runs on lane (count - 1 - b) mod lanes, so the last
-// pair's activations stay in the network's own buffers.
+// Queues the loss (dscal[0]) and its mean gradient over `count` pairs on
+// `lanes` lanes (prepare_lanes); grad is zeroed first.  Pair b runs on lane
+// (count - 1 - b) mod lanes, so the last pair's activations stay in the
+// network's own buffers.
 static int queue_loss_grad(dare_unet* net, const float* const* r, const float* const* e, const float* const* en2,
-                           int count) {
+                           int count, int lanes) {
     dare_ctx* ctx = net->ctx;
     int rc;
-    const int lanes = lanes_for(net, count);
-    if ((rc = ensure_part(net))) return rc;
     DARE_CUDA(ctx, cudaMemsetAsync(net->grad, 0, net->nparam * sizeof(float), ctx->stream));
     DARE_CUDA(ctx, cudaMemsetAsync(net->dscal, 0, sizeof(double), ctx->stream));
     const float scale = 1.f / (float)count;
     dare_unet* on[kLanes] = {net};
     for (int l = 1; l < lanes; l++) {
-        if ((rc = ensure_lane(net, l))) return rc;
         on[l] = &net->lane[l]->net;
         on[l]->wait_limit = net->wait_limit;
         on[l]->debug_skip = 0;
         net->lane[l]->ctx.launches = 0;
-        if ((rc = ensure_part(on[l]))) return set_error(ctx, rc, on[l]->ctx->last_error);
         if (l == 1) DARE_CUDA(ctx, cudaEventRecord(net->fork, ctx->stream));
         cudaStream_t s = on[l]->ctx->stream;
         DARE_CUDA(ctx, cudaStreamWaitEvent(s, net->fork, 0));
@@ -2356,7 +2375,7 @@ static void drop_loss_graph(dare_unet* net) {
 // The graph of a minibatch of `count` pairs: ~42 kernels a pair, most shorter
 // than the 4 us it takes to launch them one by one (4 pairs of 16^3: 680 us of
 // launches).  Captured on a stream of its own, so that the context's may be any.
-static int build_loss_graph(dare_unet* net, int count) {
+static int build_loss_graph(dare_unet* net, int count, int lanes) {
     dare_ctx* ctx = net->ctx;
     const int64_t n = net->ncell;
     drop_loss_graph(net);
@@ -2382,7 +2401,7 @@ static int build_loss_graph(dare_unet* net, int count) {
     int rc = DARE_OK;
     cudaError_t ce = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
     if (ce == cudaSuccess) {
-        rc = queue_loss_grad(net, rp.data(), ep.data(), np.data(), count);
+        rc = queue_loss_grad(net, rp.data(), ep.data(), np.data(), count, lanes);
         const cudaError_t c2 = cudaStreamEndCapture(cap, &graph);
         if (ce == cudaSuccess) ce = c2;
     }
@@ -2408,10 +2427,18 @@ static int loss_grad(dare_unet* net, const float* const* r, const float* const* 
     int rc;
     // the graph from the second minibatch of a size on: the first sets the
     // launch configurations and the buffers, and may be the only one
-    const bool replay = count <= kGraphPairs && net->lg_last == count && !net->debug_skip;
+    bool replay = count <= kGraphPairs && net->lg_last == count && !net->debug_skip;
+    int lanes = 1;
+    if (!replay || net->lg_count != count) {
+        if ((rc = prepare_lanes(net, count, &lanes))) return rc;
+        if (replay && (rc = build_loss_graph(net, count, lanes))) {
+            if (rc != DARE_ERR_OOM) return rc;
+            cudaGetLastError();   // no room for the graph or its inputs: launch by launch
+            replay = false;
+        }
+    }
     net->lg_last = count;
     if (replay) {
-        if (net->lg_count != count && (rc = build_loss_graph(net, count))) return rc;
         PairPtrs p{};
         for (int b = 0; b < count; b++) {
             p.r[b] = r[b];
@@ -2425,7 +2452,7 @@ static int loss_grad(dare_unet* net, const float* const* r, const float* const* 
         DARE_LAUNCHED(ctx);
         DARE_CUDA(ctx, cudaGraphLaunch(net->lg_graph, ctx->stream));
         ctx->launches += net->lg_launches;
-    } else if ((rc = queue_loss_grad(net, r, e, en2, count))) {
+    } else if ((rc = queue_loss_grad(net, r, e, en2, count, lanes))) {
         return rc;
     }
     if (loss) {
