@@ -2350,7 +2350,6 @@ static int queue_loss_grad(dare_unet* net, const float* const* r, const float* c
 }
 
 // The inputs of a minibatch into the graph's own buffers
-constexpr int kGraphPairs = 8;
 struct PairPtrs {
     const float *r[kGraphPairs], *e[kGraphPairs], *en[kGraphPairs];
 };
@@ -2366,24 +2365,28 @@ __global__ void __launch_bounds__(256) k_gather_pairs(int64_t n, int count, Pair
     if (blockIdx.x == 0 && threadIdx.x == 0) en[blockIdx.y] = *p.en[blockIdx.y];
 }
 
-static void drop_loss_graph(dare_unet* net) {
-    if (net->lg_graph) cudaGraphExecDestroy(net->lg_graph);
-    net->lg_graph = nullptr;
-    net->lg_count = 0;
+static void drop_loss_graphs(dare_unet* net) {
+    for (auto& g : net->lg) {
+        if (g.graph) cudaGraphExecDestroy(g.graph);
+        g.graph = nullptr;
+    }
 }
 
 // The graph of a minibatch of `count` pairs: ~42 kernels a pair, most shorter
 // than the 4 us it takes to launch them one by one (4 pairs of 16^3: 680 us of
 // launches).  Captured on a stream of its own, so that the context's may be any.
+// One graph is kept for each number of pairs: building it takes 0.9 ms, and a
+// pass over the data that ends with a smaller minibatch built two each time.
 static int build_loss_graph(dare_unet* net, int count, int lanes) {
     dare_ctx* ctx = net->ctx;
     const int64_t n = net->ncell;
-    drop_loss_graph(net);
+    dare_unet::LossGraph& lg = net->lg[count];
     if (net->lg_cap < count) {
+        float* in = nullptr;
+        DARE_CUDA(ctx, cudaMalloc(&in, ((size_t)2 * count * n + count) * sizeof(float)));
+        drop_loss_graphs(net);   // they read the inputs where they are now
         cudaFree(net->lg_in);
-        net->lg_in = nullptr;
-        net->lg_cap = 0;
-        DARE_CUDA(ctx, cudaMalloc(&net->lg_in, ((size_t)2 * count * n + count) * sizeof(float)));
+        net->lg_in = in;
         net->lg_cap = count;
     }
     float *r = net->lg_in, *e = r + (size_t)net->lg_cap * n, *en = e + (size_t)net->lg_cap * n;
@@ -2406,17 +2409,16 @@ static int build_loss_graph(dare_unet* net, int count, int lanes) {
         if (ce == cudaSuccess) ce = c2;
     }
     ctx->stream = saved;
-    net->lg_launches = ctx->launches - before;
+    lg.launches = ctx->launches - before;
     ctx->launches = before;
-    if (ce == cudaSuccess && rc == DARE_OK) ce = cudaGraphInstantiate(&net->lg_graph, graph, 0);
+    if (ce == cudaSuccess && rc == DARE_OK) ce = cudaGraphInstantiate(&lg.graph, graph, 0);
     if (graph) cudaGraphDestroy(graph);
     cudaStreamDestroy(cap);
     if (rc) return rc;
     if (ce != cudaSuccess) {
-        net->lg_graph = nullptr;
+        lg.graph = nullptr;
         return check_cuda(ctx, ce, "unet: minibatch graph");
     }
-    net->lg_count = count;
     return DARE_OK;
 }
 
@@ -2427,9 +2429,10 @@ static int loss_grad(dare_unet* net, const float* const* r, const float* const* 
     int rc;
     // the graph from the second minibatch of a size on: the first sets the
     // launch configurations and the buffers, and may be the only one
-    bool replay = count <= kGraphPairs && net->lg_last == count && !net->debug_skip;
+    dare_unet::LossGraph* lg = count <= kGraphPairs ? &net->lg[count] : nullptr;
+    bool replay = lg && lg->seen && !net->debug_skip;
     int lanes = 1;
-    if (!replay || net->lg_count != count) {
+    if (!replay || !lg->graph) {
         if ((rc = prepare_lanes(net, count, &lanes))) return rc;
         if (replay && (rc = build_loss_graph(net, count, lanes))) {
             if (rc != DARE_ERR_OOM) return rc;
@@ -2437,7 +2440,7 @@ static int loss_grad(dare_unet* net, const float* const* r, const float* const* 
             replay = false;
         }
     }
-    net->lg_last = count;
+    if (lg) lg->seen = true;
     if (replay) {
         PairPtrs p{};
         for (int b = 0; b < count; b++) {
@@ -2450,8 +2453,8 @@ static int loss_grad(dare_unet* net, const float* const* r, const float* const* 
         k_gather_pairs<<<dim3(eblocks(ctx, n), count), 256, 0, ctx->stream>>>(n, count, p, gr, ge,
                                                                               ge + (size_t)net->lg_cap * n);
         DARE_LAUNCHED(ctx);
-        DARE_CUDA(ctx, cudaGraphLaunch(net->lg_graph, ctx->stream));
-        ctx->launches += net->lg_launches;
+        DARE_CUDA(ctx, cudaGraphLaunch(lg->graph, ctx->stream));
+        ctx->launches += lg->launches;
     } else if ((rc = queue_loss_grad(net, r, e, en2, count, lanes))) {
         return rc;
     }
@@ -2517,7 +2520,7 @@ void dare_unet_train_params_default(dare_unet_train_params* p) {
 }
 
 static void unet_free(dare_unet* net) {
-    drop_loss_graph(net);
+    drop_loss_graphs(net);
     for (auto* ln : net->lane) free_lane(ln);
     cudaFree(net->lg_in);
     cudaFree(net->en);
@@ -2671,7 +2674,7 @@ int dare_unet_system_shape(const dare_unet* net, int n[3]) {
 int dare_unet_set_wait_limit(dare_unet* net, int64_t polls) {
     if (!net || polls < 0 || polls > 0xFFFFFFFFll) return DARE_ERR_BAD_ARG;
     net->wait_limit = polls == 0 ? kWaitLimit : (uint32_t)polls;
-    drop_loss_graph(net);   // it holds the old limit
+    drop_loss_graphs(net);   // they hold the old limit
     return DARE_OK;
 }
 

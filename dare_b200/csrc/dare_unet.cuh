@@ -83,6 +83,8 @@ constexpr LayerDef kDefs[kLayers] = {{0, 1, 16},  {1, 16, 32}, {2, 32, 64}, {3, 
                                      {3, 64, 64}, {2, 64, 32}, {1, 32, 16}, {0, 16, 1}};
 enum LayerId { ENC0 = 0, ENC1, ENC2, ENC3, DEC3, DEC2, DEC1, DEC0 };
 
+constexpr int kGraphPairs = 8;   // most pairs of a minibatch that is replayed as a graph
+
 enum { OUT_STORE = 0, OUT_ADDUP = 1, OUT_F32 = 2 };  // forward epilogue
 
 struct LaunchCfg {
@@ -160,9 +162,12 @@ struct dare_unet {
     cudaEvent_t fork = nullptr;
     // ... as one graph from the second minibatch of the same size on, its
     // inputs copied into lg_in ([residuals][errors][norms] of lg_cap pairs)
-    cudaGraphExec_t lg_graph = nullptr;
-    int lg_count = 0, lg_last = 0, lg_cap = 0;
-    int64_t lg_launches = 0;
+    struct LossGraph {
+        cudaGraphExec_t graph = nullptr;
+        int64_t launches = 0;
+        bool seen = false;                // a minibatch of this size has gone through
+    } lg[dare_gpu::unet::kGraphPairs + 1];                // by the number of pairs
+    int lg_cap = 0;
     float* lg_in = nullptr;
     float* X0 = nullptr;                  // k_conv_in input with a 16-byte row pitch, when the caller's has none
     float* z = nullptr;                   // forward output during training
