@@ -106,7 +106,7 @@ struct TeamShared {
     double red[32 * kMaxQ];
     double tot[kMaxQ];
     unsigned target[kMaxQ];
-    int timeout;
+    int timeout, limit;
     double parts[2][kMaxQ][kClusterMaxBlocks];   // cluster teams: the blocks' sums, stored here by each of them
 };
 
@@ -118,7 +118,8 @@ struct TeamShared {
 // one does.
 // Every wait ends: after `limit` polls the block gives up, and so do the
 // blocks that wait for it.  (limit 0, a test's: it gives up at its first
-// exchange, after counting itself in.)
+// exchange, after counting itself in.)  The limit is read from shared memory:
+// kept in a register of the loop it made the 64^3 solve 143 us for 140.
 struct GridTeam {
     TeamBuffer* buf;
     TeamShared* sh;
@@ -127,7 +128,10 @@ struct GridTeam {
 
     __device__ void start() {   // before the block's first barrier
         if (threadIdx.x < kMaxQ) sh->target[threadIdx.x] = buf->base[threadIdx.x];
-        if (threadIdx.x == 0) sh->timeout = 0;
+        if (threadIdx.x == 0) {
+            sh->timeout = limit == 0;
+            sh->limit = limit;
+        }
         set = buf->set;
     }
     __device__ void stop() {    // after the last exchange
@@ -184,11 +188,10 @@ struct GridTeam {
                     asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(hi) : "l"(total + 1) : "memory");
                     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(have) : "l"(n) : "memory");
                     wait = (unsigned)(lo >> 32) != target || (unsigned)(hi >> 32) != target || (int)(have - target) < 0;
-                } while (wait && ++polls < limit);
+                } while (wait && ++polls < sh->limit);
                 if (wait) sh->timeout = 1;
                 sh->tot[wid] = __longlong_as_double((long long)((lo & 0xffffffffull) | (hi << 32)));
             }
-            if (limit == 0 && lane == 0) sh->timeout = 1;
         }
         if (Q > 1) __syncthreads();   // (one value: thread 0's own warp)
         if (threadIdx.x == 0 && !sh->timeout) fin(sh->tot);
