@@ -74,13 +74,11 @@ struct dare_batch {
     size_t class_smem[dare_gpu::kBoxClasses] = {0};
     int class_clusters[dare_gpu::kBoxClasses] = {0};        // resident at a time (0: not asked yet) ...
     int clusters_block = 0;                                  // ... with this block size
-    int classes = -1, most_cluster = -1;     // cluster sizes in use, for this limit of the context's
+    int most_cluster = -1;                   // the context's limit the boxes were dealt for
     dare_gpu::BInst* d_inst = nullptr;
     int* d_order = nullptr;
     dare_gpu::BOut* d_out = nullptr;
     unsigned* d_queue = nullptr;     // one per class
-    cudaStream_t side[dare_gpu::kBoxClasses] = {nullptr};   // the classes run side by side
-    cudaEvent_t fork = nullptr, join[dare_gpu::kBoxClasses] = {nullptr};
     double* arena = nullptr;         // 9 vectors of `total` cells
     int block = 512;
     int vec_by_size[8] = {2, 2, 2, 2, 2, 2, 2, 2};
@@ -688,9 +686,14 @@ static size_t box_smem(int64_t tile) { return (size_t)(tile + 15) / 16 * 16 * (s
 // leave L2.  Batches too small to fill the device take larger clusters, down
 // to a block of 512 cells.
 // Cluster sizes that the device holds, asked for with the most threads and
-// shared memory a block may take (larger boxes, and all where it holds none, go
-// to k_batched), and that the context allows.
-static int box_classes(const dare_ctx* ctx) {
+// shared memory a block may take, and that the context allows (larger boxes,
+// and all where there is none, go to k_batched).
+static int box_classes(dare_ctx* ctx) {
+    if (ctx->box_classes >= 0) {
+        int c = ctx->box_classes;
+        while (c > 0 && ctx->team_cluster >= 0 && 1 << (c - 1) > ctx->team_cluster) c--;
+        return c;
+    }
     const auto kern = k_boxes;
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBoxSmem);
     cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
@@ -705,23 +708,20 @@ static int box_classes(const dare_ctx* ctx) {
     int c = kBoxClasses;
     for (; c > 0; c--) {
         const int blocks = 1 << (c - 1);
-        if (ctx->team_cluster >= 0 && blocks > ctx->team_cluster) continue;
         at[0].val.clusterDim.x = (unsigned)blocks;
         cfg.gridDim = dim3((unsigned)blocks);
         int fit = 0;
         if (cudaOccupancyMaxActiveClusters(&fit, kern, &cfg) == cudaSuccess && fit >= 1) break;
     }
     cudaGetLastError();   // a size that does not fit is an answer
-    return c;
+    ctx->box_classes = c;
+    return box_classes(ctx);
 }
 
 static int upload_instances(dare_batch* bt) {
     dare_ctx* ctx = bt->ctx;
-    if (bt->classes < 0 || bt->most_cluster != ctx->team_cluster) {
-        bt->classes = box_classes(ctx);
-        bt->most_cluster = ctx->team_cluster;
-    }
-    const int nc = bt->classes;
+    const int nc = box_classes(ctx);
+    bt->most_cluster = ctx->team_cluster;
     std::vector<int> cls(bt->count);
     for (int grow = 0;; grow++) {
         int64_t blocks = 0;
@@ -817,8 +817,17 @@ static int launch_class(dare_batch* bt, int c, const BVecs& vs, const BParams& p
     return launch_boxes(bt, c, vs, prm, c >= 2 ? 1024 : block, sm);
 }
 
+// The context's stream for a class beside the first, and its events
+static int ensure_side(dare_ctx* ctx, int c) {
+    static_assert(sizeof(ctx->side) / sizeof(ctx->side[0]) == kBoxClasses, "a stream for every cluster size");
+    if (!ctx->fork) DARE_CUDA(ctx, cudaEventCreateWithFlags(&ctx->fork, cudaEventDisableTiming));
+    if (!ctx->join[c]) DARE_CUDA(ctx, cudaEventCreateWithFlags(&ctx->join[c], cudaEventDisableTiming));
+    if (!ctx->side[c]) DARE_CUDA(ctx, cudaStreamCreateWithFlags(&ctx->side[c], cudaStreamNonBlocking));
+    return DARE_OK;
+}
+
 // All classes at the same time: the largest clusters on the context's stream,
-// the others on the batch's own between two events.
+// the others on its side streams between two events.
 static int launch_batch(dare_batch* bt, const dare_solver_params* p, int block) {
     dare_ctx* ctx = bt->ctx;
     if (bt->most_cluster != ctx->team_cluster)   // the context's limit has changed
@@ -844,14 +853,17 @@ static int launch_batch(dare_batch* bt, const dare_solver_params* p, int block) 
         if (used[c] && main_class < 0) main_class = c;
         nused += used[c];
     }
-    if (nused > 1) DARE_CUDA(ctx, cudaEventRecord(bt->fork, ctx->stream));
-    int rc = launch_class(bt, main_class, vs, prm, block, ctx->stream);
+    int rc;
+    for (int c = 0; c < main_class; c++)
+        if (used[c] && (rc = ensure_side(ctx, c))) return rc;
+    if (nused > 1) DARE_CUDA(ctx, cudaEventRecord(ctx->fork, ctx->stream));
+    rc = launch_class(bt, main_class, vs, prm, block, ctx->stream);
     for (int c = main_class - 1; c >= 0 && rc == DARE_OK; c--) {
         if (!used[c]) continue;
-        DARE_CUDA(ctx, cudaStreamWaitEvent(bt->side[c], bt->fork, 0));
-        rc = launch_class(bt, c, vs, prm, block, bt->side[c]);
-        DARE_CUDA(ctx, cudaEventRecord(bt->join[c], bt->side[c]));
-        DARE_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, bt->join[c], 0));
+        DARE_CUDA(ctx, cudaStreamWaitEvent(ctx->side[c], ctx->fork, 0));
+        rc = launch_class(bt, c, vs, prm, block, ctx->side[c]);
+        DARE_CUDA(ctx, cudaEventRecord(ctx->join[c], ctx->side[c]));
+        DARE_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, ctx->join[c], 0));
     }
     return rc;
 }
@@ -896,11 +908,6 @@ int dare_batch_create(dare_ctx* ctx, int count, const dare_batch_instance* inst,
     if (e == cudaSuccess) e = cudaMalloc(&bt->d_order, sizeof(int) * count);
     if (e == cudaSuccess) e = cudaMalloc(&bt->d_out, sizeof(BOut) * count);
     if (e == cudaSuccess) e = cudaMalloc(&bt->d_queue, (kBoxClasses + 1) * sizeof(unsigned));
-    for (int c = 0; c < kBoxClasses; c++) {
-        if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&bt->side[c], cudaStreamNonBlocking);
-        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&bt->join[c], cudaEventDisableTiming);
-    }
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&bt->fork, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaMalloc(&bt->arena, sizeof(double) * 9 * (size_t)bt->total);
     if (e == cudaSuccess) e = cudaMemsetAsync(bt->arena, 0, sizeof(double) * (size_t)bt->total, ctx->stream);
     if (e != cudaSuccess) {
@@ -924,11 +931,6 @@ int dare_batch_destroy(dare_batch* bt) {
     cudaFree(bt->d_out);
     cudaFree(bt->d_queue);
     cudaFree(bt->arena);
-    for (auto& q : bt->side)
-        if (q) cudaStreamDestroy(q);
-    for (auto& q : bt->join)
-        if (q) cudaEventDestroy(q);
-    if (bt->fork) cudaEventDestroy(bt->fork);
     delete bt;
     return DARE_OK;
 }

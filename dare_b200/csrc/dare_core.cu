@@ -318,6 +318,11 @@ int dare_ctx_destroy(dare_ctx* ctx) {
     cudaSetDevice(ctx->device);
     for (auto& e : ctx->ev)
         if (e) cudaEventDestroy(e);
+    for (auto& q : ctx->side)
+        if (q) cudaStreamDestroy(q);
+    for (auto& q : ctx->join)
+        if (q) cudaEventDestroy(q);
+    if (ctx->fork) cudaEventDestroy(ctx->fork);
     if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
     delete ctx;
     return DARE_OK;

@@ -76,6 +76,13 @@ struct dare_ctx {
     // the most blocks of a one-launch solve, in one cluster and over the device
     // (dare_ctx_set_team_blocks; negative: what the device holds)
     int team_cluster = -1, team_grid = -1;
+    // The cluster sizes of a batch run side by side on streams of the context,
+    // made when a solve first uses them (dare_batched.cu): a batch of one small
+    // box took 0.58 ms to make and destroy with five streams of its own, 0.36
+    // without.  The number of cluster sizes the device holds (-1: not asked yet).
+    cudaStream_t side[5] = {nullptr};
+    cudaEvent_t fork = nullptr, join[5] = {nullptr};
+    int box_classes = -1;
     // per-kernel CUDA-event timing (dare_ctx_set_profiling)
     int profiling = 0;
     cudaEvent_t ev[16] = {nullptr};
