@@ -886,6 +886,9 @@ class Batch:
                 for it, ok, st, step, res, bn, tol in _BATCH_REPORT.iter_unpack(rep)]
 
     def autotune(self, solver: "BiCGStab2") -> dict:
+        """The block size and, per size class, the factor of 1, 2 or 4 that
+        dare_batch_autotune picks (under its first name, cells a thread: it is
+        that for boxes beyond about 65^3, for others the 4096-cell units a block takes)."""
         blk = C.c_int()
         _check(lib().dare_batch_autotune(self.h, C.byref(solver.params), C.byref(blk)), self.ctx.h, "autotune")
         vec = (C.c_int * 8)()

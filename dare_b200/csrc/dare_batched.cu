@@ -80,7 +80,8 @@ struct dare_batch {
     dare_gpu::BOut* d_out = nullptr;
     unsigned* d_queue = nullptr;     // one per class
     double* arena = nullptr;         // 9 vectors of `total` cells
-    int block = 512;
+    int block = 512;   // threads of a block (clusters of four and more: 1024)
+    // by size class: 4096-cell units a block of a cluster takes, or cells a thread (k_batched)
     int vec_by_size[8] = {2, 2, 2, 2, 2, 2, 2, 2};
 };
 

@@ -10,7 +10,8 @@
 // L2, an exchange between blocks takes the place of a launch, and the kernel
 // ends when the solve does.  A time step, before and after: 64^3 diffusion 376
 // -> 167 us, 97 x 61 x 75 TVD 737 -> 360 us, 96 x 80 with two species 364 ->
-// 172 us.  What is left of a pass with its exchange (64^3, 6 us): forming the
+// 109 us (as one cluster; the solve is 76 of it).  The solve alone takes 140 us
+// at 64^3, 293 for 97 x 61 x 75.  What is left of a pass with its exchange (64^3, 6 us): forming the
 // operand 1.8 us, the rows 1 us, the block's sum 0.4 us, publishing it 1.1 us
 // and the total coming back 1.9 us, all of them L2 round trips of ~0.5 us.
 #include <algorithm>

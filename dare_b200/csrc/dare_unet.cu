@@ -1093,7 +1093,7 @@ __global__ void __launch_bounds__(kThreads) k_conv_wgrad(WgrArgs a) {
 // grad[t][co][ci] += scale * sum over the CTAs of tap group t / tpg (fixed
 // order).  Threads x take consecutive values, threads y parts of the CTAs, about
 // eight each: one thread a value left the 432-value layers with two blocks
-// that each read 560 partials in turn (47 us; 4 now).
+// that each read 560 partials in turn (47 us; 7 now).
 constexpr int kRedThreads = 256;
 __global__ void __launch_bounds__(kRedThreads) k_wgrad_reduce(const float* __restrict__ part, int nxy, int tpg,
                                                              int CINK, int COUTK, int cin, int cout, float scale,
@@ -2158,7 +2158,6 @@ static int ensure_part(dare_unet* net) {
         most = std::max(most, need);
     }
     DARE_CUDA(net->ctx, cudaMalloc(&net->part, most * sizeof(float)));
-    net->part_floats = most;
     return DARE_OK;
 }
 

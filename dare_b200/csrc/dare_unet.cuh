@@ -173,7 +173,6 @@ struct dare_unet {
     float* z = nullptr;                   // forward output during training
     float* g = nullptr;                   // dL/dz
     float* part = nullptr;                // weight-gradient partial sums
-    size_t part_floats = 0;
     double* dscal = nullptr;              // [0] loss accumulator
     double* en = nullptr;                 // ||e||^2 of en_cap pairs of a public loss call, then as floats
     int en_cap = 0;

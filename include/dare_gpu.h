@@ -426,9 +426,12 @@ DARE_API int dare_batch_zero_fields(dare_batch* bt);
 /* Solves every instance (p: tol, tol_relative, max_it; Jacobi, FP64). The
  * fields are replaced by the solutions; reports (host, count entries) may be NULL. */
 DARE_API int dare_batch_solve(dare_batch* bt, const dare_solver_params* p, dare_batch_report* reports);
-/* Picks the block size and the cells a thread handles (1, 2 or 4, relative, per
- * size class: a box goes to as few blocks of at most 4096 times that many cells
- * as it needs) by timing solves of the current fields, which are restored. */
+/* Picks, by timing solves of the current fields, which are restored, the threads
+ * of a block (of boxes that take one or two blocks, and of those beyond about
+ * 65^3; larger clusters always use 1024) and per size class a factor of 1, 2 or 4:
+ * a box goes to as few blocks of at most 4096 times that many cells as it needs.
+ * For boxes beyond about 65^3 the factor is the cells a thread takes at a time.
+ * Size classes by the longest side: up to 16, 24, 32, 48, 64, 96, 128, larger. */
 DARE_API int dare_batch_autotune(dare_batch* bt, const dare_solver_params* p, int* chosen_block);
 DARE_API int dare_batch_get_tuning(const dare_batch* bt, int* block, int vec_by_size[8]);
 
