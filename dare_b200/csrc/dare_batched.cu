@@ -412,18 +412,29 @@ __global__ void __launch_bounds__(1024) k_batched(const BInst* __restrict__ inst
 // ---------------------------------------------------------------------------
 // k_boxes: a cluster solves a box
 // ---------------------------------------------------------------------------
-// The rows of one block's cells of a box.  A pass forms the operand, already
-// scaled by D^-1, on the block's cells and the plane before and after them, a
-// run of memory that the block loads once into a shared-memory tile; the rows
-// of A are then applied to the tile.  (The one-block kernel below read all
-// seven points of a row from L1 or L2, with a table look-up for each, and one
-// SM had to move a whole box: 64^3 boxes took 12 ms a step on it.)
+// The rows of one block's cells of a box.  A pass forms the operand on the
+// block's cells and the plane before and after them, a run of memory that the
+// block loads once into a shared-memory tile; the rows of Ahat = A D^-1 are then
+// applied to the tile: y = z + sum of (off-diagonal times invd of the neighbour)
+// times the neighbour's z, as the one-block kernel above forms it.  The six
+// factors depend on which faces the cell and its neighbours touch, that is on its
+// class: along each axis the first cell, the second, one inside, the last but one
+// or the last.  A table of the 125 classes holds them.  (A tile scaled by invd
+// needed only the cell's own mask, but gave back the cell's own value as C (invd z),
+// two roundings off; the table costs 13 shared-memory reads a row and none a
+// tile cell, where that took 9 and 2.  The one-block kernel read all seven points of a row
+// from L1 or L2, with a table look-up for each, and one SM had to move a whole
+// box: 64^3 boxes took 12 ms a step on it.)
+constexpr int kBoxCells = 125;   // classes of cells
+__device__ __forceinline__ int axis_class(int i, int n) {
+    return i == 0 ? 0 : i == n - 1 ? 4 : i == 1 ? 1 : i == n - 2 ? 3 : 2;
+}
 struct BoxOp {
     int sx, sy;
-    double off0, off1, off2;
-    const double *C, *invd;           // centre coefficient and its inverse by boundary mask
+    const double* factors;            // [class][6], W E S N B T; 0 where there is no neighbour
+    const unsigned char* mask;        // faces a class touches
     double* tile;
-    const unsigned char* faces;       // boundary mask of each tile cell
+    const unsigned char* cls;         // class of each of the block's cells
     int t0, tn, c0, m;                // first cell and cells of the tile, of the block
 
     // (two cells a thread at a time, their loads together: the L2 latency is
@@ -439,7 +450,7 @@ struct BoxOp {
                 if (e0 + q * nt < tn) z[q] = zf(t0 + e0 + q * nt);
 #pragma unroll
             for (int q = 0; q < G; q++)
-                if (e0 + q * nt < tn) tile[e0 + q * nt] = invd[faces[e0 + q * nt]] * z[q];
+                if (e0 + q * nt < tn) tile[e0 + q * nt] = z[q];
         }
         __syncthreads();
         for (int l0 = threadIdx.x; l0 < m; l0 += G * nt) {
@@ -450,17 +461,23 @@ struct BoxOp {
 #pragma unroll
             for (int q = 0; q < G; q++) {
                 if (l0 + q * nt >= m) break;
-                const int c = c0 + l0 + q * nt, e = c - t0;
-                const unsigned f = faces[e];
-                const double* t = tile + e;
+                const int c = c0 + l0 + q * nt;
+                const int k = cls[l0 + q * nt];
+                const unsigned f = mask[k];
+                const double2* a = reinterpret_cast<const double2*>(factors + 6 * k);
+                const double* t = tile + (c - t0);
                 const double w = f & 1u ? 0. : t[-sx], ea = f & 2u ? 0. : t[sx];
                 const double so = f & 4u ? 0. : t[-sy], no = f & 8u ? 0. : t[sy];
                 const double bo = f & 16u ? 0. : t[-1], to = f & 32u ? 0. : t[1];
-                const double z0 = C[f] * t[0];
-                double y = z0 + off0 * (w + ea);
-                y += off1 * (so + no);
-                y += off2 * (bo + to);
-                body(c, y, z0, p[q]);
+                const double2 ax = a[0], ay = a[1], az = a[2];
+                double y = t[0];
+                y += ax.x * w;
+                y += ax.y * ea;
+                y += ay.x * so;
+                y += ay.y * no;
+                y += az.x * bo;
+                y += az.y * to;
+                body(c, y, t[0], p[q]);
             }
         }
     }
@@ -473,16 +490,17 @@ struct BoxOp {
 
 __global__ void __launch_bounds__(1024, 1) k_boxes(const BInst* __restrict__ insts, const int* __restrict__ order,
                                                    int count, BVecs vs, BParams prm, BOut* __restrict__ out,
-                                                   unsigned* queue, int tile_cells) {
+                                                   unsigned* queue) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ TeamShared sh;
     __shared__ SolverState st_s;
-    __shared__ double sC[64], sinvd[64], tfold[6];
+    __shared__ double sinvd[64], tfold[6];
+    __shared__ __align__(16) double factors[kBoxCells * 6];
+    __shared__ unsigned char mask[kBoxCells];
     __shared__ int s_item;
     SolverState* st = &st_s;
     const int tid = threadIdx.x;
     double* tile = reinterpret_cast<double*>(smem_raw);
-    unsigned char* faces = smem_raw + (size_t)tile_cells * sizeof(double);
     ClusterTeam team = ClusterTeam::here(&sh);
     team.start();
     for (;;) {
@@ -502,20 +520,30 @@ __global__ void __launch_bounds__(1024, 1) k_boxes(const BInst* __restrict__ ins
         op.sy = n2;
         op.sx = n1 * n2;
         const int N = n0 * op.sx;
-        op.off0 = Ip->offd[0];
-        op.off1 = Ip->offd[1];
-        op.off2 = Ip->offd[2];
-        op.C = sC;
-        op.invd = sinvd;
+        op.factors = factors;
+        op.mask = mask;
         op.tile = tile;
-        op.faces = faces;
+        unsigned char* cls = smem_raw + (min(N, Ip->chunk + 2 * op.sx) + 1) / 2 * 16;
+        op.cls = cls;
         op.c0 = min(N, team.rank * Ip->chunk);
         op.m = min(Ip->chunk, N - op.c0);
         op.t0 = max(0, op.c0 - op.sx);
         op.tn = op.m > 0 ? min(N, op.c0 + op.m + op.sx) - op.t0 : 0;
-        if (tid < 64) {
-            sC[tid] = Ip->C[tid];
-            sinvd[tid] = Ip->invd[tid];
+        if (tid < 64) sinvd[tid] = Ip->invd[tid];
+        for (int k = tid; k < kBoxCells; k += blockDim.x) {
+            const int n[3] = {n0, n1, n2}, at[3] = {k / 25, k / 5 % 5, k % 5};
+            unsigned own = 0;
+            for (int d = 0; d < 3; d++) own |= (unsigned)(at[d] == 0) << 2 * d | (unsigned)(at[d] == 4) << (2 * d + 1);
+            mask[k] = (unsigned char)own;
+            for (int d = 0; d < 3; d++) {
+                // the neighbours' faces: across d only the ones they reach
+                const unsigned others = own & ~(3u << 2 * d);
+                const bool second = at[d] == 1, before_last = at[d] == 3 || (at[d] == 1 && n[d] == 3);
+                factors[6 * k + 2 * d] =
+                    at[d] == 0 ? 0. : Ip->offd[d] * Ip->invd[others | (unsigned)second << 2 * d];
+                factors[6 * k + 2 * d + 1] =
+                    at[d] == 4 ? 0. : Ip->offd[d] * Ip->invd[others | (unsigned)before_last << (2 * d + 1)];
+            }
         }
         if (tid < 6) tfold[tid] = Ip->tfold[tid];
         if (tid == 0) {
@@ -525,10 +553,9 @@ __global__ void __launch_bounds__(1024, 1) k_boxes(const BInst* __restrict__ ins
             z.tol_relative = prm.tol_relative;
             *st = z;
         }
-        for (int e = tid; e < op.tn; e += blockDim.x) {
-            const int g = op.t0 + e, i = g / op.sx, rem = g - i * op.sx, j = rem / n2, k = rem - j * n2;
-            faces[e] = (unsigned char)((i == 0) | (i == n0 - 1) << 1 | (j == 0) << 2 | (j == n1 - 1) << 3 |
-                                       (k == 0) << 4 | (k == n2 - 1) << 5);
+        for (int l = tid; l < op.m; l += blockDim.x) {
+            const int c = op.c0 + l, i = c / op.sx, rem = c - i * op.sx, j = rem / n2, k = rem - j * n2;
+            cls[l] = (unsigned char)(axis_class(i, n0) * 25 + axis_class(j, n1) * 5 + axis_class(k, n2));
         }
         __syncthreads();
         const int64_t off = Ip->off;
@@ -541,7 +568,7 @@ __global__ void __launch_bounds__(1024, 1) k_boxes(const BInst* __restrict__ ins
         double a2[2] = {0., 0.};
         op.pass([&](int e) { return V.x[e]; }, [&](int c) { return V.x[c]; },
                 [&](int c, double y, double, double xc) {
-                    const unsigned f = faces[c - op.t0];
+                    const unsigned f = mask[cls[c - op.c0]];
                     double bc = tt * xc;
 #pragma unroll
                     for (int q = 0; q < 6; q++)
@@ -551,7 +578,7 @@ __global__ void __launch_bounds__(1024, 1) k_boxes(const BInst* __restrict__ ins
                     V.r[c] = rr;
                     V.rh[c] = rr;
                     V.u[c] = 0.;
-                    a2[0] += rr * rr;
+                    a2[0] = fma(rr, rr, a2[0]);
                     a2[1] += bc * bc;
                 });
         team.sum<2>(a2, [&](const double* t) { finish_init(st, t); });
@@ -566,15 +593,20 @@ __global__ void __launch_bounds__(1024, 1) k_boxes(const BInst* __restrict__ ins
                 const double u5 = V.r[c] - beta5 * V.u[c];
                 xc = alpha1 * u5 + xc;
             }
-            V.x[c] = sinvd[faces[c - op.t0]] * xc;
+            V.x[c] = sinvd[mask[cls[c - op.c0]]] * xc;
         });
         if (st->status == ST_TAU0) {
             // BiCGStab2.inl:407-424: true residual; on failure M^-1 once more
             team.barrier();
             double a1[1] = {0.};
-            // (the tile holds x / C here: its rows are those of A x after the
-            // scaling is undone by the operand C x)
-            op.pass([&](int e) { return sC[faces[e - op.t0]] * V.x[e]; }, [&](int c) { return b[c]; },
+            // (the rows are those of A x for the operand C x)
+            op.pass([&](int e) {
+                        const int i = e / op.sx, rem = e - i * op.sx, j = rem / n2, k = rem - j * n2;
+                        const unsigned f = (i == 0) | (i == n0 - 1) << 1 | (j == 0) << 2 | (j == n1 - 1) << 3 |
+                                           (k == 0) << 4 | (k == n2 - 1) << 5;
+                        return Ip->C[f] * V.x[e];
+                    },
+                    [&](int c) { return b[c]; },
                     [&](int, double y, double, double bc) {
                         const double rr = bc - y;
                         a1[0] += rr * rr;
@@ -585,7 +617,7 @@ __global__ void __launch_bounds__(1024, 1) k_boxes(const BInst* __restrict__ ins
                 if (st->status == ST_CONVERGED) st->step = 0;
             });
             if (st->status == ST_BREAKDOWN)
-                op.each<1>([&](int c) { V.x[c] = sinvd[faces[c - op.t0]] * V.x[c]; });
+                op.each<1>([&](int c) { V.x[c] = sinvd[mask[cls[c - op.c0]]] * V.x[c]; });
         }
         if (team.rank == 0 && tid == 0) {
             BOut o{};
@@ -678,8 +710,11 @@ static int fill_instance(const dare_batch_instance& in, BInst& I) {
 // `blocks` blocks
 static int64_t box_chunk(int64_t cells, int blocks) { return ((cells + blocks - 1) / blocks + 31) / 32 * 32; }
 static int64_t box_tile(int64_t cells, int64_t plane, int64_t chunk) { return std::min(cells, chunk + 2 * plane); }
-constexpr size_t kBoxSmem = 220 * 1024;   // beside the kernel's static shared memory
-static size_t box_smem(int64_t tile) { return (size_t)(tile + 15) / 16 * 16 * (sizeof(double) + 1); }
+constexpr size_t kBoxSmem = 217 * 1024;   // beside the kernel's static shared memory (10 KB)
+// the tile, then a byte a cell of the block
+static size_t box_smem(int64_t tile, int64_t chunk) {
+    return (size_t)(tile + 1) / 2 * 2 * sizeof(double) + (size_t)(chunk + 15) / 16 * 16;
+}
 
 // The cluster size of every box: as few blocks as leave each at most 4096 x
 // vec cells (vec = 1, 2 or 4 by size class, tuned): fewer cells and the
@@ -733,7 +768,11 @@ static int upload_instances(dare_batch* bt) {
             I.vec = bt->vec_by_size[size_class(std::max(I.n0, std::max(I.n1, I.n2)))];
             int c = 0;
             while (c < nc - 1 && cells > ((int64_t)4096 * I.vec << c)) c++;
-            while (c < nc && box_smem(box_tile(cells, plane, box_chunk(cells, 1 << c))) > kBoxSmem) c++;
+            const auto smem = [&](int blocks) {
+                const int64_t chunk = box_chunk(cells, blocks);
+                return box_smem(box_tile(cells, plane, chunk), chunk);
+            };
+            while (c < nc && smem(1 << c) > kBoxSmem) c++;
             if (c < nc)
                 for (int k = 0; k < grow && c < nc - 1 && cells >= (int64_t)1024 << c; k++) c++;
             else
@@ -755,7 +794,8 @@ static int upload_instances(dare_batch* bt) {
                 const BInst& I = bt->host[id];
                 order.push_back(id);
                 if (c < kBoxClasses)
-                    smem = std::max(smem, box_smem(box_tile((int64_t)I.n0 * I.n1 * I.n2, (int64_t)I.n1 * I.n2, I.chunk)));
+                    smem = std::max(smem, box_smem(box_tile((int64_t)I.n0 * I.n1 * I.n2, (int64_t)I.n1 * I.n2, I.chunk),
+                                                   I.chunk));
             }
         if (c < kBoxClasses) bt->class_smem[c] = smem;
     }
@@ -792,7 +832,7 @@ static int launch_boxes(dare_batch* bt, int c, const BVecs& vs, const BParams& p
     if (clusters < 1) return set_error(ctx, DARE_ERR_UNSUPPORTED, "dare_batch: a cluster does not fit the device");
     cfg.gridDim = dim3((unsigned)std::min(clusters, count) << c);
     DARE_CUDA(ctx, cudaLaunchKernelEx(&cfg, kern, (const BInst*)bt->d_inst, (const int*)(bt->d_order + first), count,
-                                      vs, prm, bt->d_out, bt->d_queue + c, (int)(smem / (sizeof(double) + 1))));
+                                      vs, prm, bt->d_out, bt->d_queue + c));
     DARE_LAUNCHED(ctx);
     return DARE_OK;
 }

@@ -186,7 +186,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1) k_resident(ResidentArgs A
                     A.v.r[c] = rr;
                     A.v.rh[c] = rr;
                     A.v.u[c] = 0.;
-                    a2[0] += rr * rr;
+                    a2[0] = fma(rr, rr, a2[0]);
                     a2[1] += bc * bc;
                 });
         ok = team.template sum<2>(a2, [&](const double* t) { finish_init(st, t); }) && team_iterations(team, op, A.v, st);

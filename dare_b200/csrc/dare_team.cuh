@@ -323,7 +323,9 @@ __device__ bool team_iterations(Team& team, Op& op, const TeamVecs& V, SolverSta
                     [&](int c, double y, double z, double p) {
                         out[c] = y;
                         if (stage < 3) {
-                            dot[0] += y * p;
+                            // (fused as in the initial residual's sum: where Op is the
+                            // identity both add the same products, and alpha is 1)
+                            dot[0] = fma(y, p, dot[0]);
                         } else {
                             dot[0] += p * z;
                             dot[1] += z * z;
