@@ -858,15 +858,6 @@ static int launch_class(dare_batch* bt, int c, const BVecs& vs, const BParams& p
     return launch_boxes(bt, c, vs, prm, c >= 2 ? 1024 : block, sm);
 }
 
-// The context's stream for a class beside the first, and its events
-static int ensure_side(dare_ctx* ctx, int c) {
-    static_assert(sizeof(ctx->side) / sizeof(ctx->side[0]) == kBoxClasses, "a stream for every cluster size");
-    if (!ctx->fork) DARE_CUDA(ctx, cudaEventCreateWithFlags(&ctx->fork, cudaEventDisableTiming));
-    if (!ctx->join[c]) DARE_CUDA(ctx, cudaEventCreateWithFlags(&ctx->join[c], cudaEventDisableTiming));
-    if (!ctx->side[c]) DARE_CUDA(ctx, cudaStreamCreateWithFlags(&ctx->side[c], cudaStreamNonBlocking));
-    return DARE_OK;
-}
-
 // All classes at the same time: the largest clusters on the context's stream,
 // the others on its side streams between two events.
 static int launch_batch(dare_batch* bt, const dare_solver_params* p, int block) {
@@ -895,6 +886,7 @@ static int launch_batch(dare_batch* bt, const dare_solver_params* p, int block) 
         nused += used[c];
     }
     int rc;
+    static_assert(sizeof(ctx->side) / sizeof(ctx->side[0]) == kBoxClasses, "a stream for every cluster size");
     for (int c = 0; c < main_class; c++)
         if (used[c] && (rc = ensure_side(ctx, c))) return rc;
     if (nused > 1) DARE_CUDA(ctx, cudaEventRecord(ctx->fork, ctx->stream));

@@ -65,6 +65,13 @@ cudaError_t blocks_per_sm(const void* kernel, int threads, size_t smem, int* blo
     return cudaErrorMemoryAllocation;
 }
 
+int ensure_side(dare_ctx* ctx, int q) {
+    if (!ctx->fork) DARE_CUDA(ctx, cudaEventCreateWithFlags(&ctx->fork, cudaEventDisableTiming));
+    if (!ctx->join[q]) DARE_CUDA(ctx, cudaEventCreateWithFlags(&ctx->join[q], cudaEventDisableTiming));
+    if (!ctx->side[q]) DARE_CUDA(ctx, cudaStreamCreateWithFlags(&ctx->side[q], cudaStreamNonBlocking));
+    return DARE_OK;
+}
+
 // ---- kernels ---------------------------------------------------------------
 
 // Periodic face-ghost fill (HaloBuffer self-exchange on one rank; only ghosts

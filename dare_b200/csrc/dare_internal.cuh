@@ -76,13 +76,13 @@ struct dare_ctx {
     // the most blocks of a one-launch solve, in one cluster and over the device
     // (dare_ctx_set_team_blocks; negative: what the device holds)
     int team_cluster = -1, team_grid = -1;
-    // The cluster sizes of a batch run side by side on streams of the context,
-    // made when a solve first uses them (dare_batched.cu): a batch of one small
-    // box took 0.58 ms to make and destroy with five streams of its own, 0.36
-    // without.  The number of cluster sizes the device holds (-1: not asked yet).
+    // Streams beside `stream`, with their events, made when something first runs
+    // side by side (ensure_side): the cluster sizes of a batch, the lanes of a
+    // network's minibatch.  A batch of one small box took 0.58 ms to make and
+    // destroy with five streams of its own, 0.36 without.
     cudaStream_t side[5] = {nullptr};
     cudaEvent_t fork = nullptr, join[5] = {nullptr};
-    int box_classes = -1;
+    int box_classes = -1;   // cluster sizes the device holds (dare_batched.cu; -1: not asked yet)
     // per-kernel CUDA-event timing (dare_ctx_set_profiling)
     int profiling = 0;
     cudaEvent_t ev[16] = {nullptr};
@@ -204,6 +204,9 @@ inline void launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
 cudaError_t allow_smem(const void* kernel, size_t bytes);
 // The blocks of it that one SM holds (at least 1), with that limit raised
 cudaError_t blocks_per_sm(const void* kernel, int threads, size_t smem, int* blocks);
+
+// Side stream q of a context, its event and the one the side streams start from
+int ensure_side(dare_ctx* ctx, int q);
 
 inline int grid_blocks(const dare_ctx* ctx, int64_t work, int threads, int per_sm) {
     int64_t b = (work + threads - 1) / threads;

@@ -157,9 +157,9 @@ struct dare_unet {
     dare_gpu::unet::bf16* dP1 = nullptr;
     void* act_block = nullptr;            // one allocation for all of the above
     // Training: the pairs of a minibatch run side by side, each lane with its
-    // own activations, gradients and stream (the network's own are lane 0)
+    // own activations and gradients on a side stream of the context (the
+    // network's own, on the context's stream, are lane 0)
     struct dare_unet_lane* lane[4] = {nullptr, nullptr, nullptr, nullptr};
-    cudaEvent_t fork = nullptr;
     // ... as one graph from the second minibatch of the same size on, its
     // inputs copied into lg_in ([residuals][errors][norms] of lg_cap pairs)
     struct LossGraph {
@@ -173,6 +173,7 @@ struct dare_unet {
     float* z = nullptr;                   // forward output during training
     float* g = nullptr;                   // dL/dz
     float* part = nullptr;                // weight-gradient partial sums
+    size_t part_floats = 0;
     double* dscal = nullptr;              // [0] loss accumulator
     double* en = nullptr;                 // ||e||^2 of en_cap pairs of a public loss call, then as floats
     int en_cap = 0;

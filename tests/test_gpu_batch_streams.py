@@ -62,3 +62,39 @@ def test_batches_of_a_context_in_any_order():
     ctx.close()                  # the context before its batch
     del a
     gc.collect()
+
+
+def test_a_network_shares_them():
+    """A minibatch's lanes use the same streams: queued behind a batch that is still
+    being solved, replayed from its graph, and after the batch is gone."""
+    from tests.test_gpu_unet import _weights
+    from tests.test_gpu_unet_training import _pairs
+    solver = D.BiCGStab2({"Convergence Tolerance": 1e-11, "Maximum Iterations": 500, "tol_relative": 1})
+    rng = np.random.default_rng(4)
+    fields = [rng.random(int(np.prod(n))) for n in SIZES]
+    ctx = D.Context(0)
+    n, count = (16, 24, 32), 4
+    r, e = _pairs(n, count, 8)
+
+    def network(c):
+        net = D.LearnedPreconditioner(c, n, seed=1)
+        net.set_weights(_weights(2, net.num_params))
+        return net
+
+    grad = lambda net: net.loss_grad(r.data_ptr(), e.data_ptr(), count)[1]
+    want_grad = grad(network(D.Context(0)))
+    bt = D.Batch(ctx, [_instance(m, 9 + q) for q, m in enumerate(SIZES)])
+    net = network(ctx)
+    first = None
+    for turn in range(4):
+        for q, f in enumerate(fields):
+            bt.set_field(q, f)
+        bt.solve(solver, reports=False)
+        np.testing.assert_array_equal(grad(net), want_grad)
+        xs = [bt.get_field(q) for q in range(len(SIZES))]
+        first = first or xs
+        for x, w in zip(xs, first):
+            assert np.array_equal(x, w)
+    del bt
+    gc.collect()
+    np.testing.assert_array_equal(grad(net), want_grad)
