@@ -30,30 +30,18 @@ namespace {
 std::mutex g_limits;
 std::map<std::pair<const void*, int>, size_t> g_smem;                          // (kernel, device)
 std::map<std::tuple<const void*, int, int, size_t>, int> g_per_sm;             // (kernel, device, threads, bytes)
-
-cudaError_t allow_smem_locked(const void* kernel, int device, size_t bytes) {
-    size_t& most = g_smem.try_emplace({kernel, device}, (size_t)48 * 1024).first->second;   // what any kernel may use
-    if (bytes <= most) return cudaSuccess;
-    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    if (e == cudaSuccess) most = bytes;
-    return e;
-}
 }  // namespace
-
-cudaError_t allow_smem(const void* kernel, size_t bytes) try {
-    int device = 0;
-    if (const cudaError_t e = cudaGetDevice(&device)) return e;
-    std::lock_guard<std::mutex> lock(g_limits);
-    return allow_smem_locked(kernel, device, bytes);
-} catch (const std::bad_alloc&) {
-    return cudaErrorMemoryAllocation;
-}
 
 cudaError_t blocks_per_sm(const void* kernel, int threads, size_t smem, int* blocks) try {
     int device = 0;
     if (const cudaError_t e = cudaGetDevice(&device)) return e;
     std::lock_guard<std::mutex> lock(g_limits);
-    if (const cudaError_t e = allow_smem_locked(kernel, device, smem)) return e;
+    size_t& most = g_smem.try_emplace({kernel, device}, (size_t)48 * 1024).first->second;   // what any kernel may use
+    if (smem > most) {
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+        most = smem;
+    }
     int& n = g_per_sm[{kernel, device, threads, smem}];
     if (n < 1 && (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, threads, smem) != cudaSuccess || n < 1)) {
         cudaGetLastError();

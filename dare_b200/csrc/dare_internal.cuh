@@ -197,12 +197,10 @@ inline void launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
     cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);   // an error is picked up by DARE_LAUNCHED
 }
 
-// The most dynamic shared memory that a kernel may be launched with belongs to
-// the kernel on its device, for every context, system and thread alike: it is
-// only ever raised here (to what the current device's launches have asked for),
-// so that no launch is refused because another one needed less.
-cudaError_t allow_smem(const void* kernel, size_t bytes);
-// The blocks of it that one SM holds (at least 1), with that limit raised
+// The blocks of a kernel that an SM of the current device holds (at least 1), with
+// its limit of dynamic shared memory raised to `smem`.  The limit belongs to the
+// kernel on its device, for every context, system and thread alike, and is only
+// ever raised, so that no launch is refused because another one needed less.
 cudaError_t blocks_per_sm(const void* kernel, int threads, size_t smem, int* blocks);
 
 // Side stream q of a context, its event and the one the side streams start from
